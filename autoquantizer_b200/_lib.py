@@ -16,7 +16,7 @@ AQ_MAX_MATERIALS = 4
 
 AQ_FIXED, AQ_INT, AQ_FLOAT_EXP, AQ_SHARED_EXP, AQ_RAW_F32, AQ_RAW_F64 = range(6)
 AQ_MAT_FLUID, AQ_MAT_ELASTIC, AQ_MAT_COROTATED = range(3)
-AQ_ST_OUT_OF_DOMAIN, AQ_ST_NAN, AQ_ST_FALLBACK, AQ_ST_POOL_FULL = 0x1, 0x2, 0x4, 0x8
+AQ_ST_OUT_OF_DOMAIN, AQ_ST_NAN, AQ_ST_FALLBACK, AQ_ST_POOL_FULL, AQ_ST_STALLED = 0x1, 0x2, 0x4, 0x8, 0x10
 
 ERRORS = {0: "ok", -1: "bad argument", -2: "layout does not fit the simulator schema", -3: "CUDA error",
           -4: "device allocation failed", -5: "call not valid in the current state",

@@ -54,12 +54,12 @@ struct AdK {
   int bound_clip, friction;
   R clip_lo[3], clip_hi[3];
   // rotating SDF collider (3D; col_on = 0: none), the fields collider_at
-  // reads; col_c, col_s, col_yshift are this substep's angle and height
+  // reads; pose is this substep's angle and height
   int col_on, col_n, col_dims[3], col_off[3], col_lo[3], col_hi[3];
   const float* col_sdf;
   const float* col_nrm;
-  R col_omega, col_c, col_s;
-  int col_yshift;
+  R col_omega;
+  ColPose<R> pose;
 };
 
 template <int D>
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(256) k_ad_grid(const AdK<R> K, const R* __rest
 #pragma unroll
   for (int k = 0; k < D; ++k)
     if (ad_wall<R>(K, I, k, v[k])) v[k] = 0;
-  if (D == 3 && K.col_on) collide_node<R, true>(K, I[0], I[1], I[2], v);  // sdf_collision_no_arg
+  if (D == 3 && K.col_on) collide_node<R, true>(K, K.pose, I[0], I[1], I[2], v);  // sdf_collision_no_arg
 #pragma unroll
   for (int d = 0; d < 3; ++d) gv[4 * c + d] = d < D ? v[d] : (R)0;
   gv[4 * c + 3] = 0;
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(256) k_ad_grid_bwd(const AdK<R> K, const R* __
     // (relative to the collider), the forward removed the normal part of
     // the velocity, v' = v - ((v - cv).n) n, so vbar' = vbar - (vbar.n) n
     R nrm[3], cv[3];
-    if (collider_at<R, true>(K, I[0], I[1], I[2], nrm, cv)) {
+    if (collider_at<R, true>(K, K.pose, I[0], I[1], I[2], nrm, cv)) {
       R dn = 0, bn = 0;
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
@@ -782,9 +782,9 @@ struct AdImpl final : AdBase {
     K.col_omega = (R)a->col_omega;
     const double th = a->col_theta + a->col_omega * a->P.dt * t;
     const double h = a->col_height + a->col_rate * a->P.dt * t;
-    K.col_c = (R)cos(th);
-    K.col_s = (R)sin(th);
-    K.col_yshift = (int)(h / a->P.dx + 0.5);
+    K.pose.c = (R)cos(th);
+    K.pose.s = (R)sin(th);
+    K.pose.yshift = (int)(h / a->P.dx + 0.5);
   }
   int step(const void* in, void* out, int t, cudaStream_t st) override {
     set_substep(t);

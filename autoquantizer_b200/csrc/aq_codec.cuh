@@ -254,22 +254,24 @@ struct GRec {
 
 // Record r's W words into rec[0, W) / from rec: the pairs as 16-byte
 // vectors.  WC: the word count when it is a compile-time constant, else 0.
+// Loads go to L2: another CTA may have written the record earlier in the
+// same launch.
 template <int WC>
-__device__ __forceinline__ void load_grec(const uint64_t* __restrict__ words, int64_t r, int W, uint64_t* rec) {
+__device__ __forceinline__ void load_grec(const uint64_t* words, int64_t r, int W, uint64_t* rec) {
   const int Wn = WC ? WC : W, W2 = Wn & ~1;
   const uint64_t* g = words + (r >> 5) * 32 * (int64_t)Wn;
   const int l = (int)(r & 31);
 #pragma unroll
   for (int k = 0; k < W2; k += 2) {
-    const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(g + (k >> 1) * 64 + 2 * l));
+    const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2*>(g + (k >> 1) * 64 + 2 * l));
     rec[k] = v.x;
     rec[k + 1] = v.y;
   }
-  if (Wn & 1) rec[W2] = __ldg(g + W2 * 32 + l);
+  if (Wn & 1) rec[W2] = __ldcg(g + W2 * 32 + l);
 }
 
 template <int WC>
-__device__ __forceinline__ void store_grec(uint64_t* __restrict__ words, int64_t r, int W, const uint64_t* rec) {
+__device__ __forceinline__ void store_grec(uint64_t* words, int64_t r, int W, const uint64_t* rec) {
   const int Wn = WC ? WC : W, W2 = Wn & ~1;
   uint64_t* g = words + (r >> 5) * 32 * (int64_t)Wn;
   const int l = (int)(r & 31);

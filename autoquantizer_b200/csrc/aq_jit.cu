@@ -51,6 +51,8 @@ struct Driver {
   CUresult (*getfn)(CUfunction*, CUmodule, const char*) = nullptr;
   CUresult (*launch)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream,
                      void**, void**) = nullptr;
+  CUresult (*launch_coop)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream,
+                          void**) = nullptr;
   CUresult (*setattr)(CUfunction, CUfunction_attribute, int) = nullptr;
   CUresult (*occ)(int*, CUfunction, int, size_t) = nullptr;
   bool ok = false;
@@ -94,7 +96,7 @@ void init_once() {
               sym(g_nv.h, "nvrtcGetLoweredName", g_nv.lowered) && sym(g_nv.h, "nvrtcDestroyProgram", g_nv.destroy);
   }
   g_dr.ok = drv("cuModuleLoadData", g_dr.load) && drv("cuModuleGetFunction", g_dr.getfn) &&
-            drv("cuLaunchKernel", g_dr.launch) && drv("cuFuncSetAttribute", g_dr.setattr) &&
+            drv("cuLaunchKernel", g_dr.launch) && drv("cuLaunchCooperativeKernel", g_dr.launch_coop) && drv("cuFuncSetAttribute", g_dr.setattr) &&
             drv("cuOccupancyMaxActiveBlocksPerMultiprocessor", g_dr.occ);
 }
 
@@ -118,7 +120,7 @@ std::string jit_layout_source(const aq_layout& L) {
   snprintf(b, sizeof b,
            "struct JitLayout {\n  static constexpr bool kRegRecord = %s;\n  static constexpr int kWords = %d;\n"
            "  static constexpr int kMinBlocks = %d;\n",
-           jit_reg_record(L) ? "true" : "false", L.n_words, jit_reg_record(L) ? kJitRegRecordMinBlocks : kJitSlotMinBlocks);
+           jit_reg_record(L) ? "true" : "false", L.n_words, jit_min_blocks(L));
   s += b;
   s += "  static __device__ __forceinline__ aq_layout get(const aq_layout&) {\n    return aq_layout{";
   snprintf(b, sizeof b, "%d, %d, %d, %d, %d, %d, {0, 0}, {", L.n_slots, L.n_words, L.total_bits, L.compute_f64,
@@ -153,7 +155,8 @@ bool jit_available() {
   return g_nv.ok && g_dr.ok;
 }
 
-void* jit_k_step(int D, bool HF, bool HM, bool f64, bool col, bool sparse, const aq_layout& L, std::string* err) {
+void* jit_k_step(int D, bool HF, bool HM, bool f64, bool col, bool sparse, bool multi, const aq_layout& L,
+                 std::string* err) {
   std::lock_guard<std::mutex> g(g_mu);
   init_once();
   if (!g_nv.ok || !g_dr.ok) {
@@ -161,8 +164,8 @@ void* jit_k_step(int D, bool HF, bool HM, bool f64, bool col, bool sparse, const
     return nullptr;
   }
   char name[160];
-  snprintf(name, sizeof name, "aq::k_step<%d, %s, %s, %s, aq::JitLayout, %s, %s>", D, HF ? "true" : "false",
-           HM ? "true" : "false", f64 ? "double" : "float", col ? "true" : "false", sparse ? "true" : "false");
+  snprintf(name, sizeof name, "aq::k_step<%d, %s, %s, %s, aq::JitLayout, %s, %s, %s>", D, HF ? "true" : "false",
+           HM ? "true" : "false", f64 ? "double" : "float", col ? "true" : "false", sparse ? "true" : "false", multi ? "true" : "false");
   std::string src = "#include \"aq_kernels.cuh\"\nnamespace aq {\n";
   src += jit_layout_source(L);
   src += "}\n";
@@ -243,6 +246,12 @@ int jit_occupancy(void* fn, int block, size_t smem, int* out) {
 int jit_launch(void* fn, unsigned grid, unsigned block, size_t smem, cudaStream_t st, void** args) {
   return g_dr.launch((CUfunction)fn, grid, 1, 1, block, 1, 1, (unsigned)smem, (CUstream)st, args, nullptr) ==
                  CUDA_SUCCESS
+             ? AQ_OK
+             : AQ_E_CUDA;
+}
+
+int jit_launch_cooperative(void* fn, unsigned grid, unsigned block, size_t smem, cudaStream_t st, void** args) {
+  return g_dr.launch_coop((CUfunction)fn, grid, 1, 1, block, 1, 1, (unsigned)smem, (CUstream)st, args) == CUDA_SUCCESS
              ? AQ_OK
              : AQ_E_CUDA;
 }

@@ -66,12 +66,13 @@ namespace aq {
 constexpr int CH = AQ_CH;  // AQ_CH: aq_step_config.h
 constexpr int NWARP = CH / 32;
 // CTAs per SM the register allocation of k_step must allow: the layout's
-// choice (LA::kMinBlocks) for float, 512 / CH (128 registers) for double.
+// choice (LA::kMinBlocks) for float, 256 / CH (255 registers) for double
+// (3D FP64 state, 200,000 particles: 15 % faster than with 128 registers).
 // Short records kept in registers run best at 768 / CH CTAs (80 registers:
 // more resident warps beat the extra spills); records in shared-memory
 // slots at 512 / CH.
 #ifndef AQ_STEP_MIN_BLOCKS
-#define AQ_STEP_MIN_BLOCKS(R, LA) (sizeof(R) == 8 ? 512 / AQ_CH : LA::kMinBlocks)
+#define AQ_STEP_MIN_BLOCKS(R, LA) (sizeof(R) == 8 ? 256 / AQ_CH : LA::kMinBlocks)
 #endif
 
 template <int D>
@@ -107,6 +108,18 @@ struct R4T<double> {
   typedef double4 type;
 };
 
+// Where the collider is during one substep: cos and sin of its angle, its
+// height in cells, int(height / dx + 0.5).
+template <class R>
+struct ColPose {
+  R c, s;
+  int yshift;
+};
+
+// Passes one launch of k_step may make, at most: the default re-binning
+// interval's 16 substeps.
+constexpr int AQ_PASS_MAX = 17;
+
 template <class R>
 struct SimK {
   int res[3], nb[3];
@@ -123,9 +136,8 @@ struct SimK {
   const float* col_sdf;
   const float* col_nrm;
   R col_omega;
-  R col_c, col_s;  // cos and sin of the collider angle this launch
-  int col_yshift;  // collider height in cells this launch, int(height / dx + 0.5)
   int col_node_cv;  // 1: collider velocity omega x r from the node itself (sdf_collision_no_arg)
+  ColPose<R> pose[AQ_PASS_MAX];  // per pass of the launch
   // sparse grids (k_step's SP): grid block -> pool slot (-1: none), the
   // slots handed out so far, each slot's block, the pools' capacity
   int32_t* bptr;
@@ -134,23 +146,46 @@ struct SimK {
   int pool_cap;
 };
 
+// A chain of n_sub substeps is n_sub + 1 passes over the particles: pass 0
+// is P2G of the first substep, pass p in between G2P of substep p and P2G of
+// the next, pass n_sub the last G2P.  One launch makes the passes
+// [pass0, pass1), with a grid barrier between them (k_step's MULTI; all CTAs
+// resident), or the one pass pass0.  Pass p scatters into grid (rot + p) % 3,
+// gathers from (rot + p + 2) % 3 and, with `clear`, zeroes grid
+// (rot + p + 1) % 3 for the next pass; that one was last read by pass p - 1.
 struct StepArgs {
   uint64_t* words;
   const int32_t* pid;
   const int4* items;
   const int32_t* n_items;
-  int32_t* item_ctr;       // next unclaimed item of this launch (starts at zero)
-  int32_t* item_ctr_next;  // the next launch's counter, zeroed by this launch
-  const void* grid_in;  // G2P source (after grid_op)
-  void* grid_out;       // P2G target (zeroed)
+  int32_t* sync;           // MULTI: [0] barrier arrivals, [32] barrier releases, [64 + k] items claimed in pass
+                           // pass0 + k; zeroed before the launch
+  int32_t* ctr;            // one pass: items claimed, zero at the launch
+  int32_t* ctr_next;       // the next launch's, zeroed by this one
+  void* grid[3];
+  const void* gin;         // pass0's G2P source, P2G target and the grid it clears
+  void* gout;
+  void* gnext;
+  uint64_t sk;             // pass0's dithering key
   unsigned* status;
   unsigned long long* fallbacks;
   double* rmax;
   double* rmin;
-  uint64_t sk;          // dithering key of the G2P substep
-  int do_g2p, do_p2g, ranges;
-  int raw_in;           // grid_in holds P2G sums: apply grid_op while reading
+  uint64_t seed;           // of the dithering generator
+  int64_t step0;           // index of the chain's first substep
+  int64_t grid_nodes;      // nodes of a dense grid
+  int pass0, pass1, n_sub, rot, clear, ranges;
+  int do_g2p, do_p2g;      // pass0's halves
 };
+
+// Grid k of a pass: 0 its P2G target, 1 the next pass's, 2 its G2P source.
+__host__ __device__ __forceinline__ void* pass_grid(const StepArgs& A, int pass, int k) {
+  const int g = (A.rot + pass + k) % 3;
+  return g == 0 ? A.grid[0] : g == 1 ? A.grid[1] : A.grid[2];
+}
+
+// AQ_SYNC_WORDS: ints of StepArgs::sync
+constexpr int AQ_SYNC_WORDS = 64 + AQ_PASS_MAX;
 
 // Layout from the kernel parameter (nvcc build).
 struct RtLayout {
@@ -309,16 +344,17 @@ __device__ __forceinline__ bool col_node_cv_of(const SimK<R>& K) {
 }
 
 template <class R, bool NODE_CV = false, class KT>
-__device__ __forceinline__ bool collider_at(const KT& K, int I0, int I1, int I2, R (&nrm)[3], R (&cv)[3]) {
+__device__ __forceinline__ bool collider_at(const KT& K, const ColPose<R>& pose, int I0, int I1, int I2, R (&nrm)[3],
+                                            R (&cv)[3]) {
   const int n = K.col_n;
   const int i0 = I0 >= 2 * n ? I0 - 2 * n : I0, i2 = I2 >= 2 * n ? I2 - 2 * n : I2;
-  const R c = K.col_c, s = K.col_s;
+  const R c = pose.c, s = pose.s;
   const R o0 = (R)(i0 - n), o2 = (R)(i2 - n);
   // each operation rounded on its own (no FMA contraction), so that the
   // truncation to an index matches a plain CPU evaluation
   const R x = add_rn(add_rn(sub_rn(mul_rn(c, o0), mul_rn(s, o2)), (R)n), (R)0.5);
   const R z = add_rn(add_rn(add_rn(mul_rn(s, o0), mul_rn(c, o2)), (R)n), (R)0.5);
-  int r[3] = {(int)x, I1 - K.col_yshift, (int)z};
+  int r[3] = {(int)x, I1 - pose.yshift, (int)z};
 #pragma unroll
   for (int k = 0; k < 3; ++k) r[k] = max(min(r[k], K.col_hi[k]), K.col_lo[k]);
   const int a = r[0] - K.col_off[0], b = r[1] - K.col_off[1], e = r[2] - K.col_off[2];
@@ -338,9 +374,9 @@ __device__ __forceinline__ bool collider_at(const KT& K, int I0, int I1, int I2,
 }
 
 template <class R, bool NODE_CV = false, class KT>
-__device__ __forceinline__ void collide_node(const KT& K, int I0, int I1, int I2, R (&v)[3]) {
+__device__ __forceinline__ void collide_node(const KT& K, const ColPose<R>& pose, int I0, int I1, int I2, R (&v)[3]) {
   R nrm[3], cv[3];
-  if (!collider_at<R, NODE_CV>(K, I0, I1, I2, nrm, cv)) return;
+  if (!collider_at<R, NODE_CV>(K, pose, I0, I1, I2, nrm, cv)) return;
   R vr[3], dn = 0;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -353,7 +389,7 @@ __device__ __forceinline__ void collide_node(const KT& K, int I0, int I1, int I2
 }
 
 template <int D, class R, bool COL, class R4>
-__device__ __forceinline__ R4 grid_op_node(const SimK<R>& K, R4 g, int I0, int I1, int I2) {
+__device__ __forceinline__ R4 grid_op_node(const SimK<R>& K, const ColPose<R>& pose, R4 g, int I0, int I1, int I2) {
   const int I[3] = {I0, I1, I2};
   const R inv_m = (R)1 / (g.x + (R)1e-10);
   R v[3] = {inv_m * g.y, inv_m * g.z, D == 3 ? inv_m * g.w : (R)0};
@@ -368,7 +404,7 @@ __device__ __forceinline__ R4 grid_op_node(const SimK<R>& K, R4 g, int I0, int I
     if (I[k] < K.lb[k] && v[k] < (R)0) v[k] = 0;
     if (I[k] > K.ub[k] && v[k] > (R)0) v[k] = 0;
   }
-  if (COL && D == 3 && K.col_on) collide_node<R>(K, I0, I1, I2, v);
+  if (COL && D == 3 && K.col_on) collide_node<R>(K, pose, I0, I1, I2, v);
   g.y = v[0];
   g.z = v[1];
   g.w = v[2];
@@ -476,14 +512,149 @@ __device__ __forceinline__ void bspline(const R* x, const SimK<R>& K, int* base,
   }
 }
 
+// -------------------------------------------- particles outside the tile
+// A particle that left the tile its block's item stages is done by the whole
+// warp, lane k at node k of its stencil (3^D <= 27 lanes busy).
+
+// weights of offset o (0..2) from fx = x / dx - base
+template <class R>
+__device__ __forceinline__ R bspline_w(R fx, int o) {
+  const R a = (R)0.5 * ((R)1.5 - fx) * ((R)1.5 - fx);
+  const R b = (R)0.75 - (fx - (R)1) * (fx - (R)1);
+  const R c = (R)0.5 * (fx - (R)0.5) * (fx - (R)0.5);
+  return o == 0 ? a : (o == 1 ? b : c);
+}
+
+// G2P sums of lane src's particle (base, fx: each lane's own): part[d] = sum
+// w g_d, part[D + d D + e] = sum w g_d off_e, in every lane.
+template <int D, class R, bool COL, bool SP, class R4>
+__device__ __forceinline__ void gather_outside(const SimK<R>& K, const ColPose<R>& pose, const R4* gin, int src,
+                                               int lane, const int (&base)[3], const R (&fx)[3], R (&part)[D + D * D]) {
+  constexpr int NN = D == 3 ? 27 : 9;
+  const int off[3] = {D == 3 ? lane / 9 : lane / 3, D == 3 ? (lane / 3) % 3 : lane % 3, D == 3 ? lane % 3 : 0};
+  int n[3] = {0, 0, 0};
+  R weight = 1;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    n[d] = __shfl_sync(0xffffffffu, base[d], src) + off[d];
+    weight *= bspline_w<R>(__shfl_sync(0xffffffffu, fx[d], src), off[d]);
+  }
+  R4 g;
+  g.x = g.y = g.z = g.w = 0;
+  if (lane < NN) {
+    if (SP) {
+      const int sl = K.bptr[block_of<D>(K.nb, n[0], n[1], n[2])];
+      if (sl >= 0) g = gin[node_in_slot<D>(sl, n[0], n[1], n[2])];
+    } else {
+      g = gin[cell_index<D>(K.res, n[0], n[1], n[2])];
+    }
+    g = grid_op_node<D, R, COL>(K, pose, g, n[0], n[1], n[2]);
+  }
+  const R gv[3] = {g.y, g.z, g.w};
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const R wg = lane < NN ? weight * gv[d] : (R)0;
+    part[d] = wg;
+#pragma unroll
+    for (int e = 0; e < D; ++e) part[D + d * D + e] = (R)off[e] * wg;
+  }
+#pragma unroll
+  for (int k = 0; k < D + D * D; ++k)
+#pragma unroll
+    for (int m = 16; m; m >>= 1) part[k] += __shfl_xor_sync(0xffffffffu, part[k], m);
+}
+
+// P2G of lane src's particle into the global grid: node value w (m, q + Aff off)
+template <int D, class R, bool SP, class R4>
+__device__ __forceinline__ void scatter_outside(const SimK<R>& K, R4* gout, int src, int lane,
+                                             const int (&base)[3], const R (&fx)[3], const R (&q)[D],
+                                             const R (&Aff)[D * D], unsigned& fl) {
+  constexpr int BS = Geo<D>::BS, NN = D == 3 ? 27 : 9;
+  const int off[3] = {D == 3 ? lane / 9 : lane / 3, D == 3 ? (lane / 3) % 3 : lane % 3, D == 3 ? lane % 3 : 0};
+  int b[3] = {0, 0, 0}, n[3] = {0, 0, 0};
+  R weight = 1;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    b[d] = __shfl_sync(0xffffffffu, base[d], src);
+    n[d] = b[d] + off[d];
+    weight *= bspline_w<R>(__shfl_sync(0xffffffffu, fx[d], src), off[d]);
+  }
+  R mv[3] = {0, 0, 0};
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    R s = __shfl_sync(0xffffffffu, q[d], src);
+#pragma unroll
+    for (int e = 0; e < D; ++e) s += (R)off[e] * __shfl_sync(0xffffffffu, Aff[d * D + e], src);
+    mv[d] = weight * s;
+  }
+  if (SP) {
+    // slots of the (at most 2^D) blocks under the stencil, lane qb claims block qb's
+    const int f0 = b[0] / BS, f1 = b[1] / BS, f2 = D == 3 ? b[2] / BS : 0;
+    int sl = -1;
+    if (lane < (D == 3 ? 8 : 4)) {
+      const int c0 = f0 + (D == 3 ? lane >> 2 : lane >> 1), c1 = f1 + (D == 3 ? (lane >> 1) & 1 : lane & 1),
+                c2 = D == 3 ? f2 + (lane & 1) : 0;
+      if (c0 < K.nb[0] && c1 < K.nb[1] && (D == 2 || c2 < K.nb[2])) {
+        const int64_t bk = D == 3 ? ((int64_t)c0 * K.nb[1] + c1) * K.nb[2] + c2 : (int64_t)c0 * K.nb[1] + c1;
+        sl = claim_slot(K.bptr, K.n_alloc, K.pool_blk, K.pool_cap, bk);
+        if (sl < 0) fl |= AQ_ST_POOL_FULL;
+      }
+    }
+    const int qb = D == 3 ? ((n[0] / BS - f0) << 2) | ((n[1] / BS - f1) << 1) | (n[2] / BS - f2)
+                          : ((n[0] / BS - f0) << 1) | (n[1] / BS - f1);
+    sl = __shfl_sync(0xffffffffu, sl, qb & (D == 3 ? 7 : 3));
+    if (lane < NN && sl >= 0)
+      red_add_node(gout + node_in_slot<D>(sl, n[0], n[1], n[2]), weight * K.p_mass, mv[0], mv[1], mv[2]);
+  } else if (lane < NN) {
+    red_add_node(gout + cell_index<D>(K.res, n[0], n[1], n[2]), weight * K.p_mass, mv[0], mv[1], mv[2]);
+  }
+}
+
+// Barrier of all CTAs of the launch (all of them resident: a cooperative
+// launch), the k-th of the launch (k >= 1).  sync[0] counts arrivals, the
+// last one of a round stores the round's number to sync[32], which the others
+// poll (in another cache line than the arrivals).  The fences order the
+// CTA's grid and record writes before it and its reads after it.  False when
+// the wait ran out of time (2^34 cycles, some 9 s), which no launch whose
+// CTAs are resident comes near.
+__device__ __forceinline__ bool grid_barrier(int32_t* sync, unsigned k) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int ok = 1;
+    __threadfence();
+    if ((unsigned)atomicAdd(sync, 1) + 1u == k * gridDim.x) {
+      __threadfence();
+      atomicExch(sync + 32, (int)k);
+    } else {
+      const long long t0 = clock64();
+      unsigned seen;
+      for (;;) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(sync + 32) : "memory");
+        if (seen >= k) break;
+        if (clock64() - t0 > (1ll << 34)) {
+          ok = 0;
+          break;
+        }
+        __nanosleep(32);
+      }
+    }
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
 // ------------------------------------------------------------ the step
 
 // COL: compiled with the SDF collider (the library's own build always is;
 // the layout-specialized build only when a collider is set).  SP: sparse
 // grids (grid_in / grid_out are node pools reached through K.bptr).
-template <int D, bool HF, bool HM, class R, class LA, bool COL = true, bool SP = false>
-__global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __grid_constant__ aq_layout Lp, const SimK<R> K,
-                                                const StepArgs A) {
+template <int D, bool HF, bool HM, class R, class LA, bool COL = true, bool SP = false, bool MULTI = false>
+__global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __grid_constant__ aq_layout Lp,
+                                                const __grid_constant__ SimK<R> K,
+                                                const __grid_constant__ StepArgs A) {
   typedef Sch<D, HF, HM> S;
   typedef Geo<D> G;
   typedef typename R4T<R>::type R4;
@@ -499,6 +670,11 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
   R4* ptile = gtile + TNP;                                     // NWARP x TNP (m, m v): P2G, per warp
   uint64_t* srec = reinterpret_cast<uint64_t*>(ptile + NWARP * TNP);  // CH x WS: each thread's record (RtLayout)
   __shared__ int sbox[6];  // tile-coordinate box of the item's P2G base cells (min[3], max[3])
+  // MULTI: this pass's G2P source, P2G target and dithering key (in shared
+  // memory: held in registers over the whole unit loop they spill)
+  __shared__ const void* s_gin;
+  __shared__ void* s_gout;
+  __shared__ uint64_t s_sk;
   __shared__ int s_next;   // the CTA's next work item, claimed from A.item_ctr
   __shared__ int sslot[SP ? 27 : 1];  // sparse grids: pool slots of the 3^D blocks around the item's block
   // range detection: the CTA's running max / min per slot (ord_key order)
@@ -506,12 +682,10 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nitems = *A.n_items;
-  if (A.ranges && A.do_g2p && tid < NS) {
+  if (A.ranges && tid < NS) {
     s_rmax[tid] = 0ull;   // below every key
     s_rmin[tid] = ~0ull;  // above every key
   }
-  const R4* gin = reinterpret_cast<const R4*>(A.grid_in);
-  R4* gout = reinterpret_cast<R4*>(A.grid_out);
   unsigned fl = 0, nfall = 0;
   // the thread's record words: registers when the layout (and so the word
   // count and every bit offset) is a compile-time constant and the record
@@ -520,18 +694,35 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
   uint64_t* const myrec = LA::kRegRecord ? rrec : srec + tid * WS;
   R4 zero4;
   zero4.x = zero4.y = zero4.z = zero4.w = 0;
-  if (A.do_p2g)  // private tiles start at zero; the flush of every item re-zeroes them
-    for (int j = tid; j < NWARP * TNP; j += CH) ptile[j] = zero4;
+  for (int j = tid; j < NWARP * TNP; j += CH) ptile[j] = zero4;  // the flush of every item re-zeroes them
 
-  // Work items are whole cell blocks, claimed one at a time from a counter
+  for (int pass = A.pass0; pass < (MULTI ? A.pass1 : A.pass0 + 1); ++pass) {
+  const bool do_g2p = MULTI ? pass > 0 : A.do_g2p, do_p2g = MULTI ? pass < A.n_sub : A.do_p2g;
+  if (tid == 0) {
+    s_next = blockIdx.x;
+    if (MULTI) {
+      s_gout = pass_grid(A, pass, 0);
+      s_gin = pass_grid(A, pass, 2);
+      s_sk = step_key(A.seed, A.step0 + pass - 1);
+    } else if (blockIdx.x == 0) {
+      *A.ctr_next = 0;
+    }
+  }
+  const ColPose<R>& pose = K.pose[MULTI ? pass - A.pass0 : 0];
+  if (A.clear && do_p2g) {  // the next pass's P2G target
+    const int64_t nn = SP ? (int64_t)min(*(volatile int32_t*)K.n_alloc, K.pool_cap) * 64 : A.grid_nodes;
+    R4* const gnext = reinterpret_cast<R4*>(MULTI ? pass_grid(A, pass, 1) : A.gnext);
+    for (int64_t j = (int64_t)blockIdx.x * CH + tid; j < nn; j += (int64_t)gridDim.x * CH) gnext[j] = zero4;
+  }
+#define AQ_GIN reinterpret_cast<const R4*>(MULTI ? s_gin : A.gin)
+#define AQ_GOUT reinterpret_cast<R4*>(MULTI ? s_gout : A.gout)
+
+  // Work items are cell blocks or parts of them: a CTA's first is the one of
+  // its own number, the others are claimed one at a time from a counter
   // (largest imbalance: one item).  Inside an item the warps take the
   // block's records 32 at a time (units u = warp, warp + NWARP, ...), with
   // no CTA barrier between units: the grid tile is staged once per item and
   // the warp tiles are flushed once per item.
-  if (tid == 0) {
-    if (blockIdx.x == 0) *A.item_ctr_next = 0;
-    s_next = atomicAdd(A.item_ctr, 1);
-  }
   __syncthreads();
   for (int it = s_next; it < nitems; it = s_next) {
     const int4 item = A.items[it];
@@ -564,7 +755,7 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
       }
       __syncthreads();
     }
-    if (A.do_g2p) {  // stage the grid tile (m, v after grid_op)
+    if (do_g2p) {  // stage the grid tile (m, v after grid_op)
       for (int j = tid; j < TNP; j += CH) {
         int l0, l1, l2 = 0;
         if (D == 3) {
@@ -583,11 +774,11 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
         if (ok) {
           if (SP) {
             const int sl = tile_slot<D>(sslot, ob0, ob1, ob2, g0, g1, g2);
-            if (sl >= 0) g = gin[node_in_slot<D>(sl, g0, g1, g2)];
+            if (sl >= 0) g = AQ_GIN[node_in_slot<D>(sl, g0, g1, g2)];
           } else {
-            g = gin[cell_index<D>(K.res, g0, g1, g2)];
+            g = AQ_GIN[cell_index<D>(K.res, g0, g1, g2)];
           }
-          if (A.raw_in) g = grid_op_node<D, R, COL>(K, g, g0, g1, g2);
+          g = grid_op_node<D, R, COL>(K, pose, g, g0, g1, g2);
         }
         gtile[j] = g;
       }
@@ -604,7 +795,7 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
       }
       R vals[NS];
       if (active) {
-        if (A.do_g2p) {  // G2P reads x, F|J and the material id; v and C are rewritten
+        if (do_g2p) {  // G2P reads x, F|J and the material id; v and C are rewritten
           constexpr unsigned XFM = ((1u << D) - 1u) | (((1u << S::NFJ) - 1u) << S::FJ) | (HM ? 1u << S::MAT : 0u);
           decode_record<NS, R, XFM>(L, myrec, vals);
 #pragma unroll
@@ -615,22 +806,24 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
       }
 
       // ---------------------------------------------------------------- G2P
-      if (A.do_g2p && active) {
+      if (do_g2p) {
         int base[3] = {0, 0, 0};
-        R fx[3] = {0, 0, 0}, w[3][3];
-        bspline<D, R>(vals + S::X, K, base, fx, w, fl);
-        bool in_tile = true;
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          const int l = base[d] - o[d];
-          in_tile = in_tile && l >= 0 && l <= T - 3;
-        }
+        R fx[3] = {0, 0, 0};
         R nv[D], Sm[D][D];
 #pragma unroll
         for (int d = 0; d < D; ++d) {
           nv[d] = 0;
 #pragma unroll
           for (int e = 0; e < D; ++e) Sm[d][e] = 0;
+        }
+        bool in_tile = true;
+        if (active) {
+        R w[3][3];
+        bspline<D, R>(vals + S::X, K, base, fx, w, fl);
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          const int l = base[d] - o[d];
+          in_tile = in_tile && l >= 0 && l <= T - 3;
         }
         const int lb = in_tile ? (D == 3 ? (base[0] - o[0]) * G::XS + (base[1] - o[1]) * T + (base[2] - o[2])
                                          : (base[0] - o[0]) * T + (base[1] - o[1]))
@@ -681,38 +874,29 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
                 }
               }
             }
-        } else {
-          // outside the tile (rare): the global grid, one node per iteration
-          // (a rolled loop keeps this cold path out of the instruction cache)
-          ++nfall;
-#pragma unroll 1
-          for (int k = 0; k < (D == 3 ? 27 : 9); ++k) {
-            const int a = D == 3 ? k / 9 : k / 3, b = D == 3 ? (k / 3) % 3 : k % 3, c = D == 3 ? k % 3 : 0;
-            const R wa = a == 0 ? w[0][0] : (a == 1 ? w[1][0] : w[2][0]);
-            const R wb = b == 0 ? w[0][1] : (b == 1 ? w[1][1] : w[2][1]);
-            const R wc = c == 0 ? w[0][2] : (c == 1 ? w[1][2] : w[2][2]);
-            const R wab = wa * wb;
-            const R weight = D == 3 ? wab * wc : wab;
-            const int n0 = base[0] + a, n1 = base[1] + b, n2 = D == 3 ? base[2] + c : 0;
-            R4 g;
-            if (SP) {
-              const int sl = K.bptr[block_of<D>(K.nb, n0, n1, n2)];
-              g = sl >= 0 ? gin[node_in_slot<D>(sl, n0, n1, n2)] : zero4;
-            } else {
-              g = gin[cell_index<D>(K.res, n0, n1, n2)];
-            }
-            if (A.raw_in) g = grid_op_node<D, R, COL>(K, g, n0, n1, n2);
-            const R gv[3] = {g.y, g.z, g.w};
-            const R offr[3] = {(R)a, (R)b, (R)c};
+        }
+        }
+        // Lanes outside the tile (drifted since the binning): the warp takes
+        // them one after another, a lane per node of the stencil, from the
+        // global grid, and sums over the lanes.  (One lane alone walks its
+        // nodes while the other 31 wait: with 2 % of the particles outside,
+        // half the units had such a lane.)
+        #pragma unroll 1
+        for (unsigned om = __ballot_sync(0xffffffffu, active && !in_tile); om; om &= om - 1) {
+          const int src = __ffs(om) - 1;
+          R part[D + D * D];
+          gather_outside<D, R, COL, SP>(K, pose, AQ_GIN, src, lane, base, fx, part);
+          if (lane == src) {
+            ++nfall;
 #pragma unroll
             for (int d = 0; d < D; ++d) {
-              const R wg = weight * gv[d];
-              nv[d] += wg;
+              nv[d] = part[d];
 #pragma unroll
-              for (int e = 0; e < D; ++e) Sm[d][e] += offr[e] * wg;
+              for (int e = 0; e < D; ++e) Sm[d][e] = part[D + d * D + e];
             }
           }
         }
+        if (active) {
         // new_C = 4 inv_dx sum w g_v (off - fx)^T;  new_x = x + dt new_v
         R nC[D * D];
 #pragma unroll
@@ -759,12 +943,13 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
         for (int k = 0; k < D * D; ++k) vals[S::C + k] = nC[k];
         // bit_pack_assign of the new state; vals become the values a later
         // read of the record returns (input of the next P2G)
-        encode_record<NS, R>(L, vals, myrec, particle_key(A.sk, pid), (const float*)0, (const double*)0);
+        encode_record<NS, R>(L, vals, myrec, particle_key(MULTI ? s_sk : A.sk, pid), (const float*)0, (const double*)0);
         store_grec<LA::kWords>(A.words, rec, W, myrec);
+        }
       }
 
       // -------------------------------------------- range detection (opt)
-      if (A.ranges && A.do_g2p) {
+      if (A.ranges && do_g2p) {
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
           double mx = active ? (double)vals[s] : -(double)AQ_POS_INF;
@@ -782,10 +967,10 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
       }
 
       // ---------------------------------------------------------------- P2G
-      if (A.do_p2g) {
+      if (do_p2g) {
         int base[3] = {0, 0, 0};
         R fx[3] = {0, 0, 0}, w[3][3];
-        R Aff[D * D], q[D];
+        R Aff[D * D] = {}, q[D] = {};
         bool in_tile = false;
         int lb = 0;
         if (active) {
@@ -888,60 +1073,18 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
                   __syncwarp(tm);
                 }
               }
-          } else if (mine) {  // outside the tile: straight to the global grid
-            // sparse grids: slots of the (at most 2^D) blocks under the stencil
-            int fsl[D == 3 ? 8 : 4];
-            const int fb0 = base[0] / G::BS, fb1 = base[1] / G::BS, fb2 = D == 3 ? base[2] / G::BS : 0;
-            if (SP) {
-#pragma unroll 1
-              for (int qb = 0; qb < (D == 3 ? 8 : 4); ++qb) {
-                const int c0 = fb0 + (D == 3 ? qb >> 2 : qb >> 1), c1 = fb1 + (D == 3 ? (qb >> 1) & 1 : qb & 1),
-                          c2 = D == 3 ? fb2 + (qb & 1) : 0;
-                int sl = -1;
-                if (c0 < K.nb[0] && c1 < K.nb[1] && (D == 2 || c2 < K.nb[2])) {
-                  const int64_t bk = D == 3 ? ((int64_t)c0 * K.nb[1] + c1) * K.nb[2] + c2 : (int64_t)c0 * K.nb[1] + c1;
-                  sl = claim_slot(K.bptr, K.n_alloc, K.pool_blk, K.pool_cap, bk);
-                  if (sl < 0) fl |= AQ_ST_POOL_FULL;
-                }
-                fsl[qb] = sl;
-              }
-            }
-            // one node per iteration: a rolled loop keeps this cold path
-            // out of the instruction cache
-#pragma unroll 1
-            for (int k = 0; k < (D == 3 ? 27 : 9); ++k) {
-              const int a = D == 3 ? k / 9 : k / 3, b = D == 3 ? (k / 3) % 3 : k % 3, c = D == 3 ? k % 3 : 0;
-              const R wa = a == 0 ? w[0][0] : (a == 1 ? w[1][0] : w[2][0]);
-              const R wb = b == 0 ? w[0][1] : (b == 1 ? w[1][1] : w[2][1]);
-              const R wc = c == 0 ? w[0][2] : (c == 1 ? w[1][2] : w[2][2]);
-              const R weight = D == 3 ? wa * wb * wc : wa * wb;
-              R mv[3] = {0, 0, 0};
-#pragma unroll
-              for (int d = 0; d < D; ++d) {
-                R s = q[d];
-                s += (R)a * Aff[d * D + 0];
-                s += (R)b * Aff[d * D + 1];
-                if (D == 3) s += (R)c * Aff[d * D + 2];
-                mv[d] = weight * s;
-              }
-              const int n0 = base[0] + a, n1 = base[1] + b, n2 = D == 3 ? base[2] + c : 0;
-              if (SP) {
-                const int qb = D == 3 ? ((n0 / G::BS - fb0) << 2) | ((n1 / G::BS - fb1) << 1) | (n2 / G::BS - fb2)
-                                      : ((n0 / G::BS - fb0) << 1) | (n1 / G::BS - fb1);
-                const int sl = fsl[qb];
-                if (sl >= 0)
-                  red_add_node(gout + node_in_slot<D>(sl, n0, n1, n2), weight * K.p_mass, mv[0], mv[1], mv[2]);
-              } else {
-                red_add_node(gout + cell_index<D>(K.res, n0, n1, n2), weight * K.p_mass, mv[0], mv[1], mv[2]);
-              }
-            }
           }
           __syncwarp();
         }
+        // lanes outside the tile: straight to the global grid, a lane per node
+#pragma unroll 1
+        for (unsigned om = __ballot_sync(0xffffffffu, active && !in_tile); om; om &= om - 1)
+          scatter_outside<D, R, SP>(K, AQ_GOUT, __ffs(om) - 1, lane, base, fx, q, Aff, fl);
+        __syncwarp();
       }
     }  // units
     __syncthreads();
-    if (A.do_p2g) {
+    if (do_p2g) {
       // sum the warp tiles, re-zero them, flush: one vector reduction per
       // node of the box the item's particles touched (base box + 2); the
       // tiles are zero outside it
@@ -972,20 +1115,27 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
           int sl = tile_slot<D>(sslot, ob0, ob1, ob2, g0, g1, g2);
           if (sl < 0) sl = claim_slot(K.bptr, K.n_alloc, K.pool_blk, K.pool_cap, block_of<D>(K.nb, g0, g1, g2));
           if (sl >= 0)
-            red_add_node(gout + node_in_slot<D>(sl, g0, g1, g2), sum.x, sum.y, sum.z, sum.w);
+            red_add_node(AQ_GOUT + node_in_slot<D>(sl, g0, g1, g2), sum.x, sum.y, sum.z, sum.w);
           else
             fl |= AQ_ST_POOL_FULL;
         } else {
-          red_add_node(gout + cell_index<D>(K.res, g0, g1, g2), sum.x, sum.y, sum.z, sum.w);
+          red_add_node(AQ_GOUT + cell_index<D>(K.res, g0, g1, g2), sum.x, sum.y, sum.z, sum.w);
         }
       }
     }
-    if (tid == 0) s_next = atomicAdd(A.item_ctr, 1);
+    if (tid == 0) s_next = (int)gridDim.x + atomicAdd(MULTI ? A.sync + 64 + (pass - A.pass0) : A.ctr, 1);
     __syncthreads();
   }
+#undef AQ_GIN
+#undef AQ_GOUT
+  if (MULTI && pass + 1 < A.pass1 && !grid_barrier(A.sync, (unsigned)(pass + 1 - A.pass0))) {
+    fl |= AQ_ST_STALLED;
+    break;
+  }
+  }  // passes
   if (fl) atomicOr(A.status, fl);
   if (nfall) atomicAdd(A.fallbacks, (unsigned long long)nfall);
-  if (A.ranges && A.do_g2p && tid < NS) {  // one merge per CTA and slot
+  if (A.ranges && tid < NS) {  // one merge per CTA and slot
     if (s_rmax[tid] != 0ull) atomic_max_d(A.rmax + tid, ord_val(s_rmax[tid]));
     if (s_rmin[tid] != ~0ull) atomic_min_d(A.rmin + tid, ord_val(s_rmin[tid]));
   }

@@ -2,10 +2,11 @@
 // of the substep (include/aq.h).  The fused substep kernel k_step lives in
 // aq_kernels.cuh (see there for the data layout and the algorithm).
 //
-// Per substep: one k_step launch (grid_op of the accumulated grid as each
-// tile is staged, G2P of substep k, P2G of substep k+1 into the other grid,
-// which a memset clears first).  Every sort_interval substeps the records
-// are re-binned: k_bin (cell key and rank), an exclusive scan of the
+// Per substep: one pass of k_step (grid_op of the accumulated grid as each
+// tile is staged, G2P of substep k, P2G of substep k+1 into the next of three
+// grids, the third being cleared for the substep after).  The passes between
+// two re-binnings are one cooperative launch with a grid barrier between
+// passes.  Every sort_interval substeps the records are re-binned: k_bin (cell key and rank), an exclusive scan of the
 // per-cell counts, k_scatter (records and ids into block-wide slot-major
 // order), k_items_count + k_items (one work item per occupied block, the
 // fullest blocks first).
@@ -137,24 +138,36 @@ __global__ void __launch_bounds__(SCATTER_T) k_scatter(const uint64_t* __restric
   pout[dst] = p;
 }
 
-// One work item per occupied cell block: (block, first record, count),
-// ordered by decreasing count in buckets of 16 records (largest first, so
-// that the persistent CTAs that claim items end on small ones).
+// Work items: (block, first record, count), one per occupied cell block or,
+// where a block holds more than item_max records, that block's records in
+// equal parts of whole 32-record units.  Ordered by decreasing count in
+// buckets of 16 records (largest first, so that the persistent CTAs that
+// claim items end on small ones).
 // item_info: [0] item count, [1, 1 + IB) bucket sizes, [1 + IB, 1 + 2 IB)
 // bucket fill cursors; zeroed before k_items_count.
 constexpr int IB = 64;
 
 __device__ __forceinline__ int item_bucket(int c) { return IB - 1 - min(IB - 1, (c - 1) >> 4); }
 
-__global__ void k_items_count(const int32_t* __restrict__ start, int nblk, int32_t* __restrict__ item_info) {
+// parts of a block of c records, and the records per part (the last has the rest)
+__device__ __forceinline__ int item_part(int c, int item_max) {
+  const int parts = (c + item_max - 1) / item_max;
+  return ((c + parts - 1) / parts + 31) & ~31;
+}
+
+__global__ void k_items_count(const int32_t* __restrict__ start, int nblk, int item_max,
+                              int32_t* __restrict__ item_info) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nblk) return;
   const int c = start[(int64_t)(b + 1) * 64] - start[(int64_t)b * 64];
-  if (c > 0) atomicAdd(item_info + 1 + item_bucket(c), 1);
+  if (c <= 0) return;
+  const int per = item_part(c, item_max), full = c / per, rest = c - full * per;
+  if (full) atomicAdd(item_info + 1 + item_bucket(per), full);
+  if (rest) atomicAdd(item_info + 1 + item_bucket(rest), 1);
 }
 
 // blk_of (sparse grids): the grid block of each compact block index, else null
-__global__ void k_items(const int32_t* __restrict__ start, int nblk, int4* __restrict__ items,
+__global__ void k_items(const int32_t* __restrict__ start, int nblk, int item_max, int4* __restrict__ items,
                         int32_t* __restrict__ item_info, const int32_t* __restrict__ blk_of) {
   __shared__ int off[IB];
   if (threadIdx.x == 0) {
@@ -170,8 +183,17 @@ __global__ void k_items(const int32_t* __restrict__ start, int nblk, int4* __res
   if (b >= nblk) return;
   const int s = start[(int64_t)b * 64], c = start[(int64_t)(b + 1) * 64] - s;
   if (c <= 0) return;
-  const int k = item_bucket(c);
-  items[off[k] + atomicAdd(item_info + 1 + IB + k, 1)] = make_int4(blk_of ? blk_of[b] : b, s, c, 0);
+  const int blk = blk_of ? blk_of[b] : b;
+  const int per = item_part(c, item_max), full = c / per, rest = c - full * per;
+  if (full) {
+    const int k = item_bucket(per);
+    const int at = off[k] + atomicAdd(item_info + 1 + IB + k, full);
+    for (int q = 0; q < full; ++q) items[at + q] = make_int4(blk, s + q * per, per, 0);
+  }
+  if (rest) {
+    const int k = item_bucket(rest);
+    items[off[k] + atomicAdd(item_info + 1 + IB + k, 1)] = make_int4(blk, s + full * per, rest, 0);
+  }
 }
 
 // ------------------------------------------------- sparse-grid binning
@@ -253,10 +275,11 @@ __global__ void k_cstart(const int32_t* __restrict__ ccount, const int32_t* __re
 }
 
 // Empty the pools for a new set of active blocks: zero the slots handed out
-// so far in both pools, and their table entries
+// so far in the pools, and their table entries
 template <class R4>
 __global__ void k_pool_reset(int32_t* __restrict__ bptr, int32_t* __restrict__ pool_blk,
-                             const int32_t* __restrict__ n_alloc, int cap, R4* __restrict__ p0, R4* __restrict__ p1) {
+                             const int32_t* __restrict__ n_alloc, int cap, R4* __restrict__ p0, R4* __restrict__ p1,
+                             R4* __restrict__ p2) {
   const int used = min(*n_alloc, cap);
   R4 z;
   z.x = z.y = z.z = z.w = 0;
@@ -264,6 +287,7 @@ __global__ void k_pool_reset(int32_t* __restrict__ bptr, int32_t* __restrict__ p
        i += (int64_t)gridDim.x * blockDim.x) {
     p0[i] = z;
     p1[i] = z;
+    if (p2) p2[i] = z;
     if ((i & 63) == 0) {
       const int64_t s = i >> 6;
       if (pool_blk[s] >= 0) bptr[pool_blk[s]] = -1;
@@ -587,14 +611,15 @@ struct aq_sim {
   uint64_t* words[2] = {nullptr, nullptr};
   int32_t* pid[2] = {nullptr, nullptr};
   int cur = 0;
-  void* grid[2] = {nullptr, nullptr};
+  void* grid[3] = {nullptr, nullptr, nullptr};  // [2]: null in a simulator that keeps two (THIRD_GRID_MAX)
+  int rot = 0;  // three grids: grid[rot] is zero and takes the next chain's first P2G
   int64_t ncell = 0, nkeys = 0;
   int nblk = 0;
   int32_t *keys = nullptr, *ranks = nullptr, *cell_count = nullptr, *cell_start = nullptr, *scan_sums = nullptr;
   int4* items = nullptr;
   int32_t* n_items = nullptr;  // [0] item count, then k_items' bucket sizes and cursors
-  int32_t* item_ctr = nullptr;  // [2] k_step's item claim counters
-  int64_t step_launches = 0;
+  int32_t* sync = nullptr;  // k_step's grid barrier and claim counters (StepArgs::sync), then ctr's two
+  int64_t step_launches = 0;  // launches without MULTI
   int64_t max_items = 0;
   unsigned* status = nullptr;
   unsigned long long* fallbacks = nullptr;
@@ -661,12 +686,20 @@ struct aq_sim {
   int prof_on = 0;
   cudaEvent_t* prof_ev[2] = {nullptr, nullptr};  // [PROF_CAP * 2]
   int prof_n[2] = {0, 0};
+  int64_t prof_passes = 0;  // passes of the timed k_step launches
+  bool multi = false;  // jit_fn makes several passes in a cooperative launch (k_step's MULTI)
 };
 
 namespace aq {
 
 template <int D, bool HF, bool HM, class R>
 static int setup_step_kernel(aq_sim* s, size_t smem_jit, size_t smem_aot, bool col);
+
+// Largest grid that is kept three times (SimImpl::launch_chain): k_step then
+// clears its next target itself and needs no memset, nor a launch of its own,
+// per substep.  In a larger one the clear is small beside the memory a third
+// copy takes.
+constexpr size_t THIRD_GRID_MAX = size_t(1) << 28;
 
 template <int D, bool HF, bool HM, class R>
 struct SimImpl final : SimBase {
@@ -729,6 +762,14 @@ struct SimImpl final : SimBase {
     return b + (reg_record ? 0 : sizeof(uint64_t) * (size_t)CH * s->WS);
   }
 
+  // Records per work item, at most.
+  int item_max() const {
+    return (int)std::max<int64_t>(64, (s->n / s->step_grid + 63) / 64 * 64);
+  }
+
+  // Work items there can be, at most: a launch needs no more CTAs.
+  int64_t items_bound() const { return std::min<int64_t>(s->nblk, s->n) + s->n / item_max() + 1; }
+
   int sort(cudaStream_t st) override {
     if (s->P.sparse) return sort_sparse(st);
     aq_sim* S_ = s;
@@ -744,8 +785,9 @@ struct SimImpl final : SimBase {
     const int nxt = 1 - S_->cur;
     k_scatter<<<grid_for(n, SCATTER_T), SCATTER_T, 0, st>>>(S_->words[S_->cur], S_->pid[S_->cur], S_->words[nxt], S_->pid[nxt],
                                                 S_->keys, S_->ranks, S_->cell_start, n, S_->W);
-    k_items_count<<<grid_for(S_->nblk, 256), 256, 0, st>>>(S_->cell_start, S_->nblk, S_->n_items);
-    k_items<<<grid_for(S_->nblk, 256), 256, 0, st>>>(S_->cell_start, S_->nblk, S_->items, S_->n_items, nullptr);
+    const int im = item_max();
+    k_items_count<<<grid_for(S_->nblk, 256), 256, 0, st>>>(S_->cell_start, S_->nblk, im, S_->n_items);
+    k_items<<<grid_for(S_->nblk, 256), 256, 0, st>>>(S_->cell_start, S_->nblk, im, S_->items, S_->n_items, nullptr);
     AQ_CUDA_TRY(cudaGetLastError());
     S_->cur = nxt;
     S_->launches += 7;
@@ -809,15 +851,16 @@ struct SimImpl final : SimBase {
     k_scatter<<<grid_for(n, SCATTER_T), SCATTER_T, 0, st>>>(
         S_->words[S_->cur], S_->pid[S_->cur], S_->words[nxt], S_->pid[nxt], S_->keys, S_->ranks, S_->cstart, n, S_->W);
     AQ_CUDA_TRY(cudaMemsetAsync(S_->n_items, 0, sizeof(int32_t) * (1 + 2 * IB), st));
-    k_items_count<<<grid_for(n_occ, 256), 256, 0, st>>>(S_->cstart, n_occ, S_->n_items);
-    k_items<<<grid_for(n_occ, 256), 256, 0, st>>>(S_->cstart, n_occ, S_->items, S_->n_items, S_->occ_blk);
+    const int im = item_max();
+    k_items_count<<<grid_for(n_occ, 256), 256, 0, st>>>(S_->cstart, n_occ, im, S_->n_items);
+    k_items<<<grid_for(n_occ, 256), 256, 0, st>>>(S_->cstart, n_occ, im, S_->items, S_->n_items, S_->occ_blk);
     // the active blocks: empty the pools, then the 3^D blocks around every
     // occupied block; pools grow (dropping their contents, which the next
     // launch rebuilds from the records) when the new set may not fit
     typedef typename R4T<R>::type R4;
     const int nn = D == 3 ? 27 : 9;
     k_pool_reset<R4><<<num_sms() * 4, 256, 0, st>>>(S_->bptr, S_->pool_blk, S_->n_alloc, S_->pool_cap,
-                                                    (R4*)S_->grid[0], (R4*)S_->grid[1]);
+                                                    (R4*)S_->grid[0], (R4*)S_->grid[1], (R4*)S_->grid[2]);
     AQ_CUDA_TRY(cudaMemsetAsync(S_->n_alloc, 0, sizeof(int32_t), st));
     const int64_t need = std::min<int64_t>((int64_t)nn * n_occ, S_->nblk);  // activated blocks, at most
     if (need > S_->pool_cap) {
@@ -826,7 +869,7 @@ struct SimImpl final : SimBase {
       // interval (claim_slot) must not starve the blocks that need one
       const int64_t want =
           std::min<int64_t>(std::min<int64_t>(need + need / 4 + 256, (int64_t)S_->nblk + 256), 0x7fffffffLL);
-      for (int k = 0; k < 2; ++k) {
+      for (int k = 0; k < 3; ++k) {
         if (S_->grid[k]) cudaFree(S_->grid[k]);
         S_->grid[k] = nullptr;
       }
@@ -840,6 +883,16 @@ struct SimImpl final : SimBase {
           return AQ_E_NOMEM;
         }
         AQ_CUDA_TRY(cudaMemsetAsync(S_->grid[k], 0, sizeof(R4) * 64 * (size_t)want, st));
+      }
+      S_->rot = 0;
+      const size_t bytes = sizeof(R4) * 64 * (size_t)want;
+      if (bytes <= THIRD_GRID_MAX) {
+        if (cudaMalloc(&S_->grid[2], bytes) == cudaSuccess) {
+          AQ_CUDA_TRY(cudaMemsetAsync(S_->grid[2], 0, bytes, st));
+        } else {
+          cudaGetLastError();
+          S_->grid[2] = nullptr;
+        }
       }
       AQ_CUDA_TRY(cudaMalloc((void**)&S_->pool_blk, sizeof(int32_t) * (size_t)want));
       AQ_CUDA_TRY(cudaMemsetAsync(S_->pool_blk, 0xff, sizeof(int32_t) * (size_t)want, st));
@@ -857,57 +910,102 @@ struct SimImpl final : SimBase {
     return AQ_OK;
   }
 
-  // clear = false: gout already holds this pass's sums of earlier chunks
-  // (streamed mode clears it once per pass)
+  // One pass of its own grids: P2G only, G2P + P2G or G2P only.  clear =
+  // false: gout already holds this pass's sums of earlier chunks (streamed
+  // mode clears it once per pass)
   int launch_step(int do_g2p, int do_p2g, void* gin, void* gout, cudaStream_t st, bool clear = true) {
     // the P2G target starts at zero (profiled as the grid pass)
     if (do_p2g && clear && (rc_ = clear_grid(gout, st))) return rc_;
-    aq_sim* S_ = s;
     StepArgs a;
     memset(&a, 0, sizeof(a));
+    a.pass0 = do_g2p ? 1 : 0;
+    a.pass1 = a.pass0 + 1;
+    a.n_sub = do_p2g ? 2 : 1;
+    a.grid[0] = do_g2p ? gin : gout;  // pass p scatters into grid p % 3 and gathers from the one before
+    a.grid[1] = gout;
+    return launch(a, st);
+  }
+
+  // Passes [pass0, pass1) of a chain of n_sub substeps on the three grids.
+  int launch_chain(int pass0, int pass1, int n_sub, cudaStream_t st) {
+    StepArgs a;
+    memset(&a, 0, sizeof(a));
+    a.pass0 = pass0;
+    a.pass1 = pass1;
+    a.n_sub = n_sub;
+    a.rot = s->rot;
+    a.clear = 1;
+    for (int k = 0; k < 3; ++k) a.grid[k] = s->grid[k];
+    return launch(a, st);
+  }
+
+  // The arguments every launch has; the launch itself.  a's chain starts at
+  // the simulator's current substep.
+  int launch(StepArgs& a, cudaStream_t st) {
+    aq_sim* S_ = s;
     a.words = S_->words[S_->cur];
     a.pid = S_->pid[S_->cur];
     a.items = S_->items;
     a.n_items = S_->n_items;
-    // two claim counters alternate between launches; each launch zeroes the
-    // one the next launch uses (both start at zero)
-    a.item_ctr = S_->item_ctr + (S_->step_launches & 1);
-    a.item_ctr_next = S_->item_ctr + ((S_->step_launches + 1) & 1);
-    ++S_->step_launches;
-    a.grid_in = gin;
-    a.grid_out = gout;
+    a.sync = S_->sync;
     a.status = S_->status;
     a.fallbacks = S_->fallbacks;
     a.rmax = S_->rmax;
     a.rmin = S_->rmin;
-    a.sk = step_key(S_->P.seed, S_->step);
-    a.do_g2p = do_g2p;
-    a.do_p2g = do_p2g;
+    a.seed = S_->P.seed;
+    a.step0 = S_->step;
+    a.grid_nodes = S_->ncell;
     a.ranges = S_->ranges_on;
-    a.raw_in = do_g2p;  // grid_in holds the previous P2G sums; grid_op runs as the tile is staged
     K.bptr = S_->bptr;
     K.n_alloc = S_->n_alloc;
     K.pool_blk = S_->pool_blk;
     K.pool_cap = S_->pool_cap;
-    K.col_c = (R)cos(S_->col_theta);
-    K.col_s = (R)sin(S_->col_theta);
-    K.col_yshift = (int)(S_->col_height / S_->P.dx + 0.5);
+    if (K.col_on) {  // step_collider (mpm_solver.py:1542-1547) after every substep
+      double theta = S_->col_theta, height = S_->col_height;
+      for (int p = 0; p < a.pass1; ++p) {
+        if (p > 1) {
+          theta += S_->col_omega * S_->P.dt;
+          height += S_->col_rate * S_->P.dt;
+        }
+        if (p < a.pass0) continue;
+        K.pose[p - a.pass0].c = (R)cos(theta);
+        K.pose[p - a.pass0].s = (R)sin(theta);
+        K.pose[p - a.pass0].yshift = (int)(height / S_->P.dx + 0.5);
+      }
+    }
+    const int passes = a.pass1 - a.pass0;
+    a.gin = pass_grid(a, a.pass0, 2);
+    a.gout = pass_grid(a, a.pass0, 0);
+    a.gnext = pass_grid(a, a.pass0, 1);
+    a.sk = step_key(a.seed, a.step0 + a.pass0 - 1);
+    a.do_g2p = a.pass0 > 0;
+    a.do_p2g = a.pass0 < a.n_sub;
+    const int ctas = (int)std::min<int64_t>(S_->step_grid, items_bound());
+    if (S_->multi) AQ_CUDA_TRY(cudaMemsetAsync(S_->sync, 0, sizeof(int32_t) * AQ_SYNC_WORDS, st));
+    // two claim counters alternate between launches without MULTI; each launch
+    // zeroes the one the next launch uses (both start at zero)
+    a.ctr = S_->sync + AQ_SYNC_WORDS + (S_->step_launches & 1);
+    a.ctr_next = S_->sync + AQ_SYNC_WORDS + ((S_->step_launches + 1) & 1);
+    if (!S_->multi) ++S_->step_launches;
     const bool prof = S_->prof_on && S_->prof_n[0] < aq_sim::PROF_CAP;
     if (prof) AQ_CUDA_TRY(cudaEventRecord(S_->prof_ev[0][2 * S_->prof_n[0]], st));
+    void* args[] = {(void*)&S_->L, (void*)&K, (void*)&a};
     if (S_->jit_fn) {
-      void* args[] = {(void*)&S_->L, (void*)&K, (void*)&a};
-      if (jit_launch(S_->jit_fn, S_->step_grid, CH, S_->step_smem, st, args) != AQ_OK) {
+      const int rc = passes > 1 ? jit_launch_cooperative(S_->jit_fn, ctas, CH, S_->step_smem, st, args)
+                                : jit_launch(S_->jit_fn, ctas, CH, S_->step_smem, st, args);
+      if (rc != AQ_OK) {
         set_last_cuda_error(cudaErrorLaunchFailure, "cuLaunchKernel(k_step)");
         return AQ_E_CUDA;
       }
-    } else if (S_->P.sparse) {
-      k_step<D, HF, HM, R, RtLayout, true, true><<<S_->step_grid, CH, S_->step_smem, st>>>(S_->L, K, a);
-      AQ_CUDA_TRY(cudaGetLastError());
     } else {
-      k_step<D, HF, HM, R, RtLayout><<<S_->step_grid, CH, S_->step_smem, st>>>(S_->L, K, a);
-      AQ_CUDA_TRY(cudaGetLastError());
+      const void* f = S_->P.sparse ? (const void*)k_step<D, HF, HM, R, RtLayout, true, true>
+                                   : (const void*)k_step<D, HF, HM, R, RtLayout>;
+      AQ_CUDA_TRY(cudaLaunchKernel(f, dim3(ctas), dim3(CH), args, S_->step_smem, st));
     }
-    if (prof) AQ_CUDA_TRY(cudaEventRecord(S_->prof_ev[0][2 * S_->prof_n[0]++ + 1], st));
+    if (prof) {
+      AQ_CUDA_TRY(cudaEventRecord(S_->prof_ev[0][2 * S_->prof_n[0]++ + 1], st));
+      S_->prof_passes += passes;
+    }
     S_->launches += 1;
     return AQ_OK;
   }
@@ -1026,11 +1124,16 @@ struct SimImpl final : SimBase {
         if ((rc = stream_pass(1, 0, S_->grid[a], nullptr, st, true, true))) return rc;
         S_->last_grid = a;
       }
-      ++S_->step;
-      S_->col_theta += S_->col_omega * S_->P.dt;
-      S_->col_height += S_->col_rate * S_->P.dt;
+      advance();
     }
     return AQ_OK;
+  }
+
+  // one substep further; step_collider (mpm_solver.py:1542-1547) after each
+  void advance() {
+    ++s->step;
+    s->col_theta += s->col_omega * s->P.dt;
+    s->col_height += s->col_rate * s->P.dt;
   }
 
   int substeps(int n, cudaStream_t st) override {
@@ -1044,24 +1147,29 @@ struct SimImpl final : SimBase {
       }
       int m = interval - S_->since_sort;
       if (m > n) m = n;
-      // P2G of the first substep, then per substep one fused launch: grid_op
-      // applied while staging the tile, G2P, P2G of the next substep into
-      // the other (cleared) grid
-      int a = 0;
-      if ((rc = launch_step(0, 1, nullptr, S_->grid[a], st))) return rc;
-      for (int k = 0; k < m; ++k) {
-        const int b = 1 - a;
-        if (k + 1 < m) {
-          if ((rc = launch_step(1, 1, S_->grid[a], S_->grid[b], st))) return rc;
-          a = b;
-        } else {
-          if ((rc = launch_step(1, 0, S_->grid[a], nullptr, st))) return rc;
-          S_->last_grid = a;
+      // m + 1 passes: P2G of the first substep, G2P of each fused with P2G
+      // of the next, G2P of the last (grid_op applied as tiles are staged)
+      if (S_->grid[2]) {
+        const int per = S_->multi ? AQ_PASS_MAX : 1;
+        for (int p = 0; p <= m; p += per)
+          if ((rc = launch_chain(p, std::min(p + per, m + 1), m, st))) return rc;
+        S_->last_grid = (S_->rot + m + 2) % 3;
+        S_->rot = (S_->rot + m) % 3;
+        for (int k = 0; k < m; ++k) advance();
+      } else {
+        int a = 0;
+        if ((rc = launch_step(0, 1, nullptr, S_->grid[a], st))) return rc;
+        for (int k = 0; k < m; ++k) {
+          const int b = 1 - a;
+          if (k + 1 < m) {
+            if ((rc = launch_step(1, 1, S_->grid[a], S_->grid[b], st))) return rc;
+            a = b;
+          } else {
+            if ((rc = launch_step(1, 0, S_->grid[a], nullptr, st))) return rc;
+            S_->last_grid = a;
+          }
+          advance();
         }
-        ++S_->step;
-        // step_collider (mpm_solver.py:1542-1547) after every substep
-        S_->col_theta += S_->col_omega * S_->P.dt;
-        S_->col_height += S_->col_rate * S_->P.dt;
       }
       S_->since_sort += m;
       n -= m;
@@ -1092,11 +1200,19 @@ struct SimImpl final : SimBase {
 // select the library's own k_step, and size its persistent grid.
 template <int D, bool HF, bool HM, class R>
 static int setup_step_kernel(aq_sim* s, size_t smem_jit, size_t smem_aot, bool col) {
-  int occ = 0;
+  int occ = 0, dev = 0, coop = 0;
   s->jit_fn = nullptr;
+  AQ_CUDA_TRY(cudaGetDevice(&dev));
+  AQ_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
   if (s->P.jit) {
     const size_t smem = smem_jit;
-    s->jit_fn = jit_k_step(D, HF, HM, sizeof(R) == 8, col, s->P.sparse != 0, s->L, &s->jit_error);
+    // Several passes a launch where a CTA's share of the records is one
+    // 64-record item or less: there the launches and their gaps weigh (2D,
+    // 8,192 particles: 13 % of a substep; 65,536: 11 %; 3D, 60,000: 8 %),
+    // while with more units per warp the pass loop's registers cost what it
+    // saves (262,144: +-3 %, 2,097,152: 3 % slower).
+    s->multi = coop && s->cap <= (int64_t)64 * kJitShortRecordMinBlocks * num_sms();
+    s->jit_fn = jit_k_step(D, HF, HM, sizeof(R) == 8, col, s->P.sparse != 0, s->multi, s->L, &s->jit_error);
     if (s->jit_fn && (jit_set_smem(s->jit_fn, (int)smem) != AQ_OK || jit_occupancy(s->jit_fn, CH, smem, &occ) != AQ_OK)) {
       s->jit_fn = nullptr;
       s->jit_error = "cuFuncSetAttribute/occupancy failed";
@@ -1104,6 +1220,7 @@ static int setup_step_kernel(aq_sim* s, size_t smem_jit, size_t smem_aot, bool c
     s->step_smem = smem;
   }
   if (!s->jit_fn) {
+    s->multi = false;
     const size_t smem = smem_aot;
     s->step_smem = smem;
     if (s->P.sparse) {
@@ -1151,7 +1268,7 @@ static void free_sim(aq_sim* s) {
     }
   }
   if (s->P.sparse) {
-    for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < 3; ++k)
       if (s->grid[k]) cudaFree(s->grid[k]);
     if (s->pool_blk) cudaFree(s->pool_blk);
     if (s->ccount) cudaFree(s->ccount);
@@ -1224,7 +1341,9 @@ int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
   }
   s->nblk = (int)nblk64;
   s->nkeys = P->sparse ? 0 : (int64_t)s->nblk * 64;
-  s->max_items = P->sparse ? std::min<int64_t>(s->nblk, P->n_particles) + 1 : (int64_t)s->nblk + 1;
+  // one item per occupied block and, where blocks are split (item_part),
+  // less than one more per 32 records
+  s->max_items = std::min<int64_t>(s->nblk, P->n_particles) + P->n_particles / 32 + 1;
   const size_t rsz = P->precision ? sizeof(double) : sizeof(float);
   const int64_t n = s->n;
   const int nt = (int)((s->nkeys + SCAN_TILE - 1) / SCAN_TILE);
@@ -1273,7 +1392,7 @@ int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
   }
   alloc((void**)&s->items, sizeof(int4) * s->max_items);
   alloc((void**)&s->n_items, sizeof(int32_t) * (1 + 2 * IB));
-  alloc((void**)&s->item_ctr, 2 * sizeof(int32_t));
+  alloc((void**)&s->sync, sizeof(int32_t) * (AQ_SYNC_WORDS + 2));
   alloc((void**)&s->status, sizeof(unsigned));
   alloc((void**)&s->fallbacks, sizeof(unsigned long long));
   alloc((void**)&s->rmax, sizeof(double) * AQ_MAX_SLOTS);
@@ -1284,7 +1403,16 @@ int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
     free_sim(s);
     return AQ_E_LIMIT;
   }
+  const size_t gbytes = rsz * 4 * s->ncell, before = total;
+  const bool third = !P->sparse && gbytes <= THIRD_GRID_MAX;
+  if (third) total += (gbytes + 255) & ~(size_t)255;  // the third grid, behind the others
   e = cudaMalloc(&s->slab, total);
+  if (e == cudaSuccess && third) {
+    s->grid[2] = static_cast<char*>(s->slab) + before;
+  } else if (e != cudaSuccess && third) {  // without it
+    cudaGetLastError();
+    e = cudaMalloc(&s->slab, before);
+  }
   if (e == cudaSuccess)
     for (int k = 0; k < nparts; ++k) *parts[k].p = static_cast<char*>(s->slab) + parts[k].off;
   if (e != cudaSuccess) {
@@ -1311,11 +1439,12 @@ int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
   } else {
     e = cudaMemset(s->grid[0], 0, rsz * 4 * s->ncell);
     if (e == cudaSuccess) e = cudaMemset(s->grid[1], 0, rsz * 4 * s->ncell);
+    if (e == cudaSuccess && s->grid[2]) e = cudaMemset(s->grid[2], 0, rsz * 4 * s->ncell);
   }
   if (e == cudaSuccess) e = cudaMemset(s->words[0], 0, sizeof(uint64_t) * (grouped_words(n, s->W) + 2));
   if (e == cudaSuccess) e = cudaMemset(s->status, 0, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(s->fallbacks, 0, sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMemset(s->item_ctr, 0, 2 * sizeof(int32_t));
+  if (e == cudaSuccess) e = cudaMemset(s->sync, 0, sizeof(int32_t) * (AQ_SYNC_WORDS + 2));
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "cudaMemset");
     free_sim(s);
@@ -1739,6 +1868,7 @@ int aq_sim_profile_enable(aq_sim* s, int32_t on) {
       }
       s->prof_n[k] = 0;
     }
+    s->prof_passes = 0;
   }
   s->prof_on = on ? 1 : 0;
   return AQ_OK;
@@ -1756,7 +1886,8 @@ int aq_sim_profile_get(aq_sim* s, int32_t which, double* h_total_ms, int64_t* h_
   }
   s->prof_n[which] = 0;
   *h_total_ms = tot;
-  *h_launches = n;
+  *h_launches = which == 0 ? s->prof_passes : n;
+  if (which == 0) s->prof_passes = 0;
   return AQ_OK;
 }
 

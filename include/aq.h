@@ -52,6 +52,7 @@ extern "C" {
 #define AQ_ST_NAN 0x2u            /* a NaN position was met; base clamped */
 #define AQ_ST_FALLBACK 0x4u       /* a particle left its shared-memory tile (informational) */
 #define AQ_ST_POOL_FULL 0x8u      /* sparse grid: no free node block; contributions to it were dropped */
+#define AQ_ST_STALLED 0x10u       /* a substep launch gave up waiting for its own blocks: the state is not valid */
 
 /* scalar kinds: quantized types of the reference
  *   AQ_FIXED      ti.quant.fixed(frac=bits, signed, range, offset)
@@ -329,8 +330,9 @@ int aq_sim_launches(const aq_sim* sim, int64_t* h_out);
  * substep kernel (k_step) and of the grid kernel (k_grid) on the stream they
  * run on.  No reference counterpart (the reference profiles through CUPTI,
  * taichi_submission/taichi/program/kernel_profiler.h:46).  which: 0 = k_step,
- * 1 = the grid clear before each P2G.  profile_get synchronizes and resets
- * the accumulators. */
+ * counted in passes over the particles (one launch may make several), 1 = the
+ * grid clears that are launches of their own.  profile_get synchronizes and
+ * resets the accumulators. */
 int aq_sim_profile_enable(aq_sim* sim, int32_t on);
 int aq_sim_profile_get(aq_sim* sim, int32_t which, double* h_total_ms, int64_t* h_launches);
 
