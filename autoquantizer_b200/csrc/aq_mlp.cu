@@ -281,7 +281,7 @@ int aq_mlp_forward(int32_t in, int32_t h, int32_t out, const float* d_params, co
     z2 = a1 + (size_t)B * h;
     a2 = z2 + (size_t)B * h;
   } else {
-    AQ_CUDA_TRY(cudaMallocAsync((void**)&tmp, sizeof(float) * 2 * (size_t)B * h, st));
+    AQ_CUDA_TRY(pool_alloc((void**)&tmp, sizeof(float) * 2 * (size_t)B * h, st));
     a1 = tmp;
     a2 = tmp + (size_t)B * h;
   }
@@ -292,7 +292,7 @@ int aq_mlp_forward(int32_t in, int32_t h, int32_t out, const float* d_params, co
   k_gemm_bf16<float, __nv_bfloat16, EPI_FWD><<<gemm_grid(B, out), GTHREADS, 0, st>>>(
       a2, h, 1, wb + o.w3, h, 1, B, out, h, d_params + o.b3, nullptr, nullptr, d_y, 0);
   AQ_CUDA_TRY(cudaGetLastError());
-  if (tmp) AQ_CUDA_TRY(cudaFreeAsync(tmp, st));
+  pool_free(tmp, st);
   return AQ_OK;
 }
 
@@ -307,7 +307,7 @@ int aq_mlp_backward(int32_t in, int32_t h, int32_t out, const uint16_t* d_params
   const float* z2 = a1 + (size_t)B * h;
   const float* a2 = z2 + (size_t)B * h;
   float* dz = nullptr;
-  AQ_CUDA_TRY(cudaMallocAsync((void**)&dz, sizeof(float) * 2 * (size_t)B * h, st));
+  AQ_CUDA_TRY(pool_alloc((void**)&dz, sizeof(float) * 2 * (size_t)B * h, st));
   float* dz2 = dz;
   float* dz1 = dz + (size_t)B * h;
   // layer 3: dW3 = dy^T a2, db3, dz2 = (dy W3) * gelu'(z2)
@@ -327,7 +327,7 @@ int aq_mlp_backward(int32_t in, int32_t h, int32_t out, const uint16_t* d_params
       dz1, h, 0, d_x, in, 0, h, in, B, nullptr, nullptr, nullptr, d_grad + o.w1, 0);
   k_colsum<<<grid_for(h, 128), 128, 0, st>>>(dz1, B, h, d_grad + o.b1);
   AQ_CUDA_TRY(cudaGetLastError());
-  AQ_CUDA_TRY(cudaFreeAsync(dz, st));
+  pool_free(dz, st);
   return AQ_OK;
 }
 

@@ -798,14 +798,14 @@ struct SimImpl final : SimBase {
 
   // Grow a device buffer (contents dropped) to at least `need` elements.
   template <class T>
-  static int grow(T*& p, int64_t& cap_elems, int64_t need) {
+  static int grow(T*& p, int64_t& cap_elems, int64_t need, cudaStream_t st) {
     if (need <= cap_elems && p) return AQ_OK;
-    if (p) cudaFree(p);
+    pool_free(p, st);
     p = nullptr;
     cap_elems = 0;
-    const cudaError_t e = cudaMalloc((void**)&p, sizeof(T) * (size_t)need);
+    const cudaError_t e = pool_alloc((void**)&p, sizeof(T) * (size_t)need, st);
     if (e != cudaSuccess) {
-      set_last_cuda_error(e, "cudaMalloc (sparse grid)");
+      set_last_cuda_error(e, "cudaMallocFromPoolAsync (sparse grid)");
       return AQ_E_NOMEM;
     }
     cap_elems = need;
@@ -838,8 +838,8 @@ struct SimImpl final : SimBase {
     if (n_occ > S_->occ_cap) {
       const int64_t want = (int64_t)n_occ + n_occ / 4 + 64;
       cc = cs = 0;
-      if ((rc = grow(S_->ccount, cc, want * 64))) return rc;
-      if ((rc = grow(S_->cstart, cs, want * 64 + 1))) return rc;
+      if ((rc = grow(S_->ccount, cc, want * 64, st))) return rc;
+      if ((rc = grow(S_->cstart, cs, want * 64 + 1, st))) return rc;
       S_->occ_cap = want;
     }
     AQ_CUDA_TRY(cudaMemsetAsync(S_->ccount, 0, sizeof(int32_t) * 64 * (size_t)n_occ, st));
@@ -870,16 +870,16 @@ struct SimImpl final : SimBase {
       const int64_t want =
           std::min<int64_t>(std::min<int64_t>(need + need / 4 + 256, (int64_t)S_->nblk + 256), 0x7fffffffLL);
       for (int k = 0; k < 3; ++k) {
-        if (S_->grid[k]) cudaFree(S_->grid[k]);
+        pool_free(S_->grid[k], st);
         S_->grid[k] = nullptr;
       }
-      if (S_->pool_blk) cudaFree(S_->pool_blk);
+      pool_free(S_->pool_blk, st);
       S_->pool_blk = nullptr;
       S_->pool_cap = 0;
       for (int k = 0; k < 2; ++k) {
-        const cudaError_t e = cudaMalloc(&S_->grid[k], sizeof(R4) * 64 * (size_t)want);
+        const cudaError_t e = pool_alloc(&S_->grid[k], sizeof(R4) * 64 * (size_t)want, st);
         if (e != cudaSuccess) {
-          set_last_cuda_error(e, "cudaMalloc (sparse grid pool)");
+          set_last_cuda_error(e, "cudaMallocFromPoolAsync (sparse grid pool)");
           return AQ_E_NOMEM;
         }
         AQ_CUDA_TRY(cudaMemsetAsync(S_->grid[k], 0, sizeof(R4) * 64 * (size_t)want, st));
@@ -887,14 +887,14 @@ struct SimImpl final : SimBase {
       S_->rot = 0;
       const size_t bytes = sizeof(R4) * 64 * (size_t)want;
       if (bytes <= THIRD_GRID_MAX) {
-        if (cudaMalloc(&S_->grid[2], bytes) == cudaSuccess) {
+        if (pool_alloc(&S_->grid[2], bytes, st) == cudaSuccess) {
           AQ_CUDA_TRY(cudaMemsetAsync(S_->grid[2], 0, bytes, st));
         } else {
           cudaGetLastError();
           S_->grid[2] = nullptr;
         }
       }
-      AQ_CUDA_TRY(cudaMalloc((void**)&S_->pool_blk, sizeof(int32_t) * (size_t)want));
+      AQ_CUDA_TRY(pool_alloc((void**)&S_->pool_blk, sizeof(int32_t) * (size_t)want, st));
       AQ_CUDA_TRY(cudaMemsetAsync(S_->pool_blk, 0xff, sizeof(int32_t) * (size_t)want, st));
       S_->pool_cap = (int)want;
     }
@@ -1268,14 +1268,13 @@ static void free_sim(aq_sim* s) {
     }
   }
   if (s->P.sparse) {
-    for (int k = 0; k < 3; ++k)
-      if (s->grid[k]) cudaFree(s->grid[k]);
-    if (s->pool_blk) cudaFree(s->pool_blk);
-    if (s->ccount) cudaFree(s->ccount);
-    if (s->cstart) cudaFree(s->cstart);
-    if (s->cub_tmp) cudaFree(s->cub_tmp);
+    for (int k = 0; k < 3; ++k) pool_free(s->grid[k], 0);
+    pool_free(s->pool_blk, 0);
+    pool_free(s->ccount, 0);
+    pool_free(s->cstart, 0);
+    pool_free(s->cub_tmp, 0);
   }
-  if (s->slab) cudaFree(s->slab);
+  pool_free(s->slab, 0);
   if (s->h_words) cudaFreeHost(s->h_words);
   if (s->words_dl) cudaFree(s->words_dl);
   if (s->words_up[1]) cudaFree(s->words_up[1]);
@@ -1349,7 +1348,7 @@ int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
   const int nt = (int)((s->nkeys + SCAN_TILE - 1) / SCAN_TILE);
   cudaError_t e = cudaSuccess;
   // every buffer is carved from one device allocation (one cudaMalloc per
-  // simulator, one cudaFree at destroy), each on a 256-byte boundary
+  // simulator, given back at destroy), each on a 256-byte boundary
   struct Part {
     void** p;
     size_t off;
@@ -1406,18 +1405,18 @@ int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
   const size_t gbytes = rsz * 4 * s->ncell, before = total;
   const bool third = !P->sparse && gbytes <= THIRD_GRID_MAX;
   if (third) total += (gbytes + 255) & ~(size_t)255;  // the third grid, behind the others
-  e = cudaMalloc(&s->slab, total);
+  e = pool_alloc(&s->slab, total, 0);
   if (e == cudaSuccess && third) {
     s->grid[2] = static_cast<char*>(s->slab) + before;
   } else if (e != cudaSuccess && third) {  // without it
     cudaGetLastError();
-    e = cudaMalloc(&s->slab, before);
+    e = pool_alloc(&s->slab, before, 0);
   }
   if (e == cudaSuccess)
     for (int k = 0; k < nparts; ++k) *parts[k].p = static_cast<char*>(s->slab) + parts[k].off;
   if (e != cudaSuccess) {
     s->slab = nullptr;
-    set_last_cuda_error(e, "cudaMalloc");
+    set_last_cuda_error(e, "cudaMallocFromPoolAsync");
     free_sim(s);
     return AQ_E_NOMEM;
   }
@@ -1435,7 +1434,7 @@ int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
                                              s->occ_len, s->n_alloc + 1, (int)n);
     if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, b3, s->occ_len, s->occ_first, (int)n);
     s->cub_bytes = std::max(std::max(b1, b2), std::max(b3, (size_t)256));
-    if (e == cudaSuccess) e = cudaMalloc(&s->cub_tmp, s->cub_bytes);
+    if (e == cudaSuccess) e = pool_alloc(&s->cub_tmp, s->cub_bytes, 0);
   } else {
     e = cudaMemset(s->grid[0], 0, rsz * 4 * s->ncell);
     if (e == cudaSuccess) e = cudaMemset(s->grid[1], 0, rsz * 4 * s->ncell);
