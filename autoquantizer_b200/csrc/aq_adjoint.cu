@@ -49,10 +49,8 @@ namespace aq {
 template <class R>
 struct AdK {
   int res[3], D, NS, HF, mat;
-  R inv_dx, dx, dt, p_mass, kst, four_inv_dx2, grav, mu, lam;
-  double lb[3], ub[3];
-  int bound_clip, friction;
-  R clip_lo[3], clip_hi[3];
+  R inv_dx, dx, dt, p_mass, kst, four_inv_dx, four_inv_dx2, grav, mu, lam;
+  int wlo[3], whi[3];  // walls: node indices below wlo / above whi
   // rotating SDF collider (3D; col_on = 0: none), the fields collider_at
   // reads; pose is this substep's angle and height
   int col_on, col_n, col_dims[3], col_off[3], col_lo[3], col_hi[3];
@@ -68,8 +66,7 @@ __device__ __forceinline__ int64_t ad_cell(const int (&res)[3], const int* I) {
 }
 
 template <int D, class R>
-__device__ __forceinline__ void ad_weights(const R* x, const AdK<R>& K, int* base, R* fx, R (&w)[3][3],
-                                           R (&dw)[3][3]) {
+__device__ __forceinline__ void ad_weights(const R* x, const AdK<R>& K, int (&base)[3], R (&fx)[3], R (&w)[3][3]) {
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     R t = x[d] * K.inv_dx - (R)0.5;
@@ -80,7 +77,14 @@ __device__ __forceinline__ void ad_weights(const R* x, const AdK<R>& K, int* bas
     w[0][d] = (R)0.5 * ((R)1.5 - fx[d]) * ((R)1.5 - fx[d]);
     w[1][d] = (R)0.75 - (fx[d] - (R)1) * (fx[d] - (R)1);
     w[2][d] = (R)0.5 * (fx[d] - (R)0.5) * (fx[d] - (R)0.5);
-    // dN/dx (per unit x: chain with inv_dx)
+  }
+}
+
+// dN/dx per unit x
+template <int D, class R>
+__device__ __forceinline__ void ad_dweights(const AdK<R>& K, const R (&fx)[3], R (&dw)[3][3]) {
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
     dw[0][d] = -((R)1.5 - fx[d]) * K.inv_dx;
     dw[1][d] = (R)-2 * (fx[d] - (R)1) * K.inv_dx;
     dw[2][d] = (fx[d] - (R)0.5) * K.inv_dx;
@@ -224,491 +228,762 @@ __device__ __forceinline__ void ad_sigma_bwd(const AdK<R>& K, const R* s, const 
   }
 }
 
-template <int D>
-__device__ __forceinline__ void offs(int o, int* off) {
-  off[0] = D == 3 ? o / 9 : o / 3;
-  off[1] = D == 3 ? (o / 3) % 3 : o % 3;
-  off[2] = D == 3 ? o % 3 : 0;
+// ------------------------------------------------------------- layout
+//
+// States and their adjoints inside the library: the particles in the order
+// of ad_sort_key, in groups of 32 that hold slot s of all 32 side by side, so
+// that a warp's loads and stores of a slot are one coalesced access.
+
+__host__ __device__ __forceinline__ int64_t ad_padded(int64_t n) { return (n + 31) & ~int64_t(31); }
+
+template <int NS>
+__device__ __forceinline__ int64_t ad_at(int64_t p, int s) {
+  return ((p >> 5) * NS + s) * 32 + (p & 31);
 }
 
-// ------------------------------------------------------------- forward
+template <int NS, int LO, int HI, class R>
+__device__ __forceinline__ void ad_load(const R* __restrict__ st, int64_t p, R (&s)[NS]) {
+#pragma unroll
+  for (int k = LO; k < HI; ++k) s[k] = st[ad_at<NS>(p, k)];
+}
 
-// Runs of equal keys over consecutive lanes of a warp.  The state is sorted
-// by base cell, so a run holds the warp's particles of one cell, which add
-// into the same 3^D nodes: run_sum adds a value over the lane's run in
-// log2(longest run) shuffle steps, and the run's first lane makes the one
-// global atomic for the whole run instead of one per particle.
-struct WarpRuns {
-  int lane, end, steps;  // end: last lane of this lane's run
-  bool head;             // this lane starts its run
+// ------------------------------------------------------------- warp tiles
+//
+// Every kernel works warp by warp: 32 particles, neighbours on the grid, and
+// the box of nodes their stencils reach.  Where the box fits AdTile nodes the
+// warp gathers from a copy of it in shared memory (the node's own operation
+// - grid_op or its transpose - applied once per node as it is copied) and
+// scatters into a zeroed copy that goes to the grid with one vector reduction
+// per node; otherwise (particles that have drifted far apart) straight from
+// and to the grid.  No two warps share a tile, so there is no CTA barrier.
+// Particle by particle with scalar global atomics, from rows of 96 bytes and
+// with the grid's operation in kernels of its own, a substep of the 3D
+// falling block (262,144 particles, FP32) took 127 us forward (now 52) and
+// 287 us backward, recomputed sums and squares included (now 141).
+//
+// Half a block's cells (4 x 2 x 4, and 4 x 8 in 2D) reach 6 x 4 x 6 = 144
+// nodes (6 x 10 = 60); AdTile leaves room for a cell of drift on every side,
+// and for the warps whose particles lie in two blocks.
+template <int D>
+struct AdTile {
+  static constexpr int N = D == 3 ? 384 : 192;
 };
 
-__device__ __forceinline__ WarpRuns warp_runs(long long key) {
-  WarpRuns r;
-  r.lane = threadIdx.x & 31;
-  const long long prev = __shfl_up_sync(0xffffffffu, key, 1);
-  r.head = r.lane == 0 || prev != key;
-  const unsigned starts = __ballot_sync(0xffffffffu, r.head);
-  const unsigned later = r.lane == 31 ? 0u : (starts & (0xffffffffu << (r.lane + 1)));
-  r.end = later ? __ffs(later) - 2 : 31;
-  const int len = r.head ? r.end - r.lane + 1 : 1;
-  const int maxlen = (int)__reduce_max_sync(0xffffffffu, (unsigned)len);
-  int steps = 0;
-  while ((1 << steps) < maxlen) ++steps;
-  r.steps = steps;
-  return r;
-}
+struct AdBox {
+  int o[3], e1, e2, n;  // origin, extents of axes 1 and 2, nodes
+  bool fits;
+};
 
-// After the call the run's first lane holds the sum of v over the run.
-template <class R>
-__device__ __forceinline__ R run_sum(R v, const WarpRuns& r) {
-  for (int k = 0; k < r.steps; ++k) {
-    const int d = 1 << k;
-    const R o = __shfl_down_sync(0xffffffffu, v, d);
-    if (r.lane + d <= r.end) v += o;
+// the box of the lanes with `on` (none: an empty box)
+template <int D>
+__device__ __forceinline__ AdBox ad_box(bool on, const int (&base)[3]) {
+  AdBox b;
+  int e[3] = {1, 1, 1};
+  const bool any = __any_sync(0xffffffffu, on);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    b.o[d] = 0;
+    if (d < D) {
+      const int lo = __reduce_min_sync(0xffffffffu, on ? base[d] : 0x7fffffff);
+      const int hi = __reduce_max_sync(0xffffffffu, on ? base[d] : -1);
+      b.o[d] = any ? lo : 0;
+      e[d] = any ? hi - lo + 3 : 3;
+    }
   }
-  return v;
+  b.e1 = e[1];
+  b.e2 = D == 3 ? e[2] : 1;
+  b.fits = any;
+#pragma unroll
+  for (int d = 0; d < D; ++d) b.fits = b.fits && e[d] <= AdTile<D>::N;
+  b.n = b.fits ? e[0] * e[1] * e[2] : 0;  // each extent <= 384: no overflow
+  b.fits = b.fits && b.n <= AdTile<D>::N;
+  return b;
 }
 
-template <int D, bool HF, class R>
-__global__ void __launch_bounds__(128) k_ad_p2g(const AdK<R> K, const R* __restrict__ st, int64_t n,
-                                                R* __restrict__ grid) {
-  typedef Sch<D, HF, false> S;
-  const int64_t p0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = p0 < n;
-  if (__all_sync(0xffffffffu, !active)) return;
-  const int64_t p = active ? p0 : n - 1;  // lanes past the end take part in the shuffles only
-  const R* s = st + p * K.NS;
-  int base[3];
-  R fx[3], w[3][3], dw[3][3];
-  ad_weights<D, R>(s + S::X, K, base, fx, w, dw);
-  R sig[9], A[9];
-  ad_sigma<D, HF, R>(K, s, sig);
-#pragma unroll
-  for (int k = 0; k < D * D; ++k) A[k] = K.kst * sig[k] + K.p_mass * s[S::C + k];
-  const WarpRuns runs = warp_runs(active ? (long long)ad_cell<D>(K.res, base) : -1 - (long long)(threadIdx.x & 31));
-  const R on = active ? (R)1 : (R)0;
-  for (int o = 0; o < (D == 3 ? 27 : 9); ++o) {
-    int off[3], I[3];
-    offs<D>(o, off);
-    R wt = on, dpos[3];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      wt *= w[off[d]][d];
-      dpos[d] = ((R)off[d] - fx[d]) * K.dx;
-      I[d] = base[d] + off[d];
-    }
-    R val[4];
-    val[0] = run_sum(wt * K.p_mass, runs);
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      R a = K.p_mass * s[S::V + d];
-#pragma unroll
-      for (int e = 0; e < D; ++e) a += A[d * D + e] * dpos[e];
-      val[1 + d] = run_sum(wt * a, runs);
-    }
-    if (active && runs.head) {
-      R* g = grid + 4 * ad_cell<D>(K.res, I);
-#pragma unroll
-      for (int k = 0; k < 1 + D; ++k) atomicAdd(g + k, val[k]);
-    }
+// node j of a box: its index in axis order (exact float floors: j < 2^10)
+template <int D>
+__device__ __forceinline__ void ad_node(const AdBox& b, int j, int (&I)[3]) {
+  if (D == 3) {
+    const int q = (int)(((float)j + 0.5f) / (float)b.e2);
+    const int i0 = (int)(((float)q + 0.5f) / (float)b.e1);
+    I[0] = b.o[0] + i0;
+    I[1] = b.o[1] + (q - i0 * b.e1);
+    I[2] = b.o[2] + (j - q * b.e2);
+  } else {
+    const int i0 = (int)(((float)j + 0.5f) / (float)b.e1);
+    I[0] = b.o[0] + i0;
+    I[1] = b.o[1] + (j - i0 * b.e1);
+    I[2] = 0;
   }
 }
 
 // wall mask of component k at node I given the velocity sign (grid_op)
 template <class R>
-__device__ __forceinline__ bool ad_wall(const AdK<R>& K, const int* I, int k, R vk) {
-  return (I[k] < K.lb[k] && vk < (R)0) || (I[k] > K.ub[k] && vk > (R)0);
+__device__ __forceinline__ bool ad_wall(const AdK<R>& K, const int (&I)[3], int k, R vk) {
+  return (I[k] < K.wlo[k] && vk < (R)0) || (I[k] > K.whi[k] && vk > (R)0);
 }
 
+// Grid velocity of a node from its sums (m, P): (0, v).
 template <int D, class R>
-__global__ void __launch_bounds__(256) k_ad_grid(const AdK<R> K, const R* __restrict__ grid, R* __restrict__ gv,
-                                                 int64_t ncell) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncell) return;
-  int I[3] = {0, 0, 0};
-  if (D == 3) {
-    I[2] = (int)(c % K.res[2]);
-    I[1] = (int)((c / K.res[2]) % K.res[1]);
-    I[0] = (int)(c / ((int64_t)K.res[2] * K.res[1]));
-  } else {
-    I[1] = (int)(c % K.res[1]);
-    I[0] = (int)(c / K.res[1]);
+struct AdGridOp {
+  typedef typename R4T<R>::type R4;
+  const AdK<R>& K;
+  const R4* grid;
+  __device__ __forceinline__ R4 operator()(const int (&I)[3]) const {
+    R4 g = grid[ad_cell<D>(K.res, I)];
+    const R inv_m = (R)1 / (g.x + (R)1e-10);
+    R v[3] = {inv_m * g.y, inv_m * g.z, D == 3 ? inv_m * g.w : (R)0};
+    v[1] -= K.dt * K.grav;
+#pragma unroll
+    for (int k = 0; k < D; ++k)
+      if (ad_wall<R>(K, I, k, v[k])) v[k] = 0;
+    if (D == 3 && K.col_on) collide_node<R, true>(K, K.pose, I[0], I[1], I[2], v);  // sdf_collision_no_arg
+    g.x = 0;
+    g.y = v[0];
+    g.z = v[1];
+    g.w = v[2];
+    return g;
   }
-  const R* g = grid + 4 * c;
-  const R inv_m = (R)1 / (g[0] + (R)1e-10);
-  R v[3] = {0, 0, 0};
+};
+
+// Adjoint of a node's sums, (mbar, Pbar), from the sums and the adjoint of
+// its velocity (grid^T).
+template <int D, class R>
+struct AdGridOpT {
+  typedef typename R4T<R>::type R4;
+  const AdK<R>& K;
+  const R4* grid;
+  const R4* gvb;
+  __device__ __forceinline__ R4 operator()(const int (&I)[3]) const {
+    const int64_t c = ad_cell<D>(K.res, I);
+    const R4 g = grid[c], b = gvb[c];
+    const R P[3] = {g.y, g.z, g.w};
+    const R inv_m = (R)1 / (g.x + (R)1e-10);
+    R v[3] = {inv_m * P[0], inv_m * P[1], D == 3 ? inv_m * P[2] : (R)0};
+    v[1] -= K.dt * K.grav;
+    R vb[3] = {b.y, b.z, D == 3 ? b.w : (R)0};
+    if (D == 3 && K.col_on) {
+      // collider^T: where the node is inside and moving into the surface
+      // (relative to the collider), the forward removed the normal part of
+      // the velocity, v' = v - ((v - cv).n) n, so vbar' = vbar - (vbar.n) n
+      R nrm[3], cv[3];
+      if (collider_at<R, true>(K, K.pose, I[0], I[1], I[2], nrm, cv)) {
+        R dn = 0, bn = 0;
 #pragma unroll
-  for (int d = 0; d < D; ++d) v[d] = inv_m * g[1 + d];
-  v[1] -= K.dt * K.grav;
+        for (int k = 0; k < 3; ++k) {
+          const R vw = ad_wall<R>(K, I, k, v[k]) ? (R)0 : v[k];  // the collider's input
+          dn += (vw - cv[k]) * nrm[k];
+          bn += vb[k] * nrm[k];
+        }
+        if (dn < (R)0)
 #pragma unroll
-  for (int k = 0; k < D; ++k)
-    if (ad_wall<R>(K, I, k, v[k])) v[k] = 0;
-  if (D == 3 && K.col_on) collide_node<R, true>(K, K.pose, I[0], I[1], I[2], v);  // sdf_collision_no_arg
+          for (int k = 0; k < 3; ++k) vb[k] -= bn * nrm[k];
+      }
+    }
+    R4 r;
+    R mb = 0, Pb[3] = {0, 0, 0};
 #pragma unroll
-  for (int d = 0; d < 3; ++d) gv[4 * c + d] = d < D ? v[d] : (R)0;
-  gv[4 * c + 3] = 0;
+    for (int d = 0; d < D; ++d) {
+      const R bd = ad_wall<R>(K, I, d, v[d]) ? (R)0 : vb[d];
+      Pb[d] = bd * inv_m;
+      mb -= bd * P[d] * inv_m * inv_m;
+    }
+    r.x = mb;
+    r.y = Pb[0];
+    r.z = Pb[1];
+    r.w = Pb[2];
+    return r;
+  }
+};
+
+// copy a box into a tile through the node's operation
+template <int D, class R4, class F>
+__device__ __forceinline__ void ad_stage(const AdBox& b, R4* tile, const F& node) {
+  for (int j = threadIdx.x & 31; j < b.n; j += 32) {
+    int I[3];
+    ad_node<D>(b, j, I);
+    tile[j] = node(I);
+  }
+  __syncwarp();
 }
 
-template <int D, bool HF, class R>
-__global__ void __launch_bounds__(128) k_ad_g2p(const AdK<R> K, const R* __restrict__ st, const R* __restrict__ gv,
-                                                R* __restrict__ out, int64_t n) {
-  typedef Sch<D, HF, false> S;
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const R* s = st + p * K.NS;
-  R* so = out + p * K.NS;
-  int base[3];
-  R fx[3], w[3][3], dw[3][3];
-  ad_weights<D, R>(s + S::X, K, base, fx, w, dw);
-  R nv[3] = {0, 0, 0}, nC[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int o = 0; o < (D == 3 ? 27 : 9); ++o) {
-    int off[3], I[3];
-    offs<D>(o, off);
-    R wt = 1, dpos[3];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      wt *= w[off[d]][d];
-      dpos[d] = ((R)off[d] - fx[d]) * K.dx;
-      I[d] = base[d] + off[d];
-    }
-    const R* g = gv + 4 * ad_cell<D>(K.res, I);
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      nv[d] += wt * g[d];
-#pragma unroll
-      for (int e = 0; e < D; ++e) nC[d * D + e] += K.four_inv_dx2 * wt * g[d] * dpos[e];
-    }
+template <class R4>
+__device__ __forceinline__ void ad_zero(const AdBox& b, R4* tile) {
+  R4 z;
+  z.x = z.y = z.z = z.w = 0;
+  for (int j = threadIdx.x & 31; j < b.n; j += 32) tile[j] = z;
+  __syncwarp();
+}
+
+template <int D, class R, class R4>
+__device__ __forceinline__ void ad_flush(const AdK<R>& K, const AdBox& b, const R4* tile, R4* grid) {
+  __syncwarp();
+  for (int j = threadIdx.x & 31; j < b.n; j += 32) {
+    const R4 v = tile[j];
+    if (v.x == (R)0 && v.y == (R)0 && v.z == (R)0 && v.w == (R)0) continue;
+    int I[3];
+    ad_node<D>(b, j, I);
+    red_add_node(grid + ad_cell<D>(K.res, I), v.x, v.y, v.z, v.w);
   }
+}
+
+template <int D>
+__device__ __forceinline__ int ad_local(const AdBox& b, const int (&base)[3]) {
+  return D == 3 ? ((base[0] - b.o[0]) * b.e1 + (base[1] - b.o[1])) * b.e2 + (base[2] - b.o[2])
+                : (base[0] - b.o[0]) * b.e1 + (base[1] - b.o[1]);
+}
+
+// The particle's view of its 3^D nodes, in the tile (TILE) or on the grid
+// through the node's operation.
+template <int D, class R, bool TILE, class F>
+struct AdSrc {
+  typedef typename R4T<R>::type R4;
+  const R4* t;  // the base node in the tile
+  int sa, sb;   // tile strides of axes 0 and 1
+  const F& node;
+  const int (&base)[3];
+  __device__ __forceinline__ R4 operator()(int a, int b, int c) const {
+    if (TILE) return t[a * sa + b * sb + c];
+    const int I[3] = {base[0] + a, base[1] + b, D == 3 ? base[2] + c : 0};
+    return node(I);
+  }
+};
+
+// nv = sum w g, Sm = sum w g off^T over the nodes' (y, z, w)
+template <int D, class R, bool TILE, class S>
+__device__ __forceinline__ void ad_gather(const S& src, const R (&w)[3][3], R (&nv)[3], R (&Sm)[3][3]) {
+#pragma unroll
+  for (int d = 0; d < 3; ++d) nv[d] = Sm[d][0] = Sm[d][1] = Sm[d][2] = 0;
+#pragma unroll(TILE ? 3 : 1)
+  for (int a = 0; a < 3; ++a)
+#pragma unroll(TILE ? 3 : 1)
+    for (int b = 0; b < 3; ++b) {
+      const R wab = w[a][0] * w[b][1];
+      R P[3] = {0, 0, 0}, Q[3] = {0, 0, 0};
+#pragma unroll(TILE ? 3 : 1)
+      for (int c = 0; c < (D == 3 ? 3 : 1); ++c) {
+        const auto g = src(a, b, c);
+        const R wc = D == 3 ? w[c][2] : (R)1;
+        const R gv[3] = {g.y, g.z, g.w};
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          P[d] += wc * gv[d];
+          if (D == 3 && c) Q[d] += (R)c * wc * gv[d];
+        }
+      }
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        const R wp = wab * P[d];
+        nv[d] += wp;
+        Sm[d][0] += (R)a * wp;
+        Sm[d][1] += (R)b * wp;
+        if (D == 3) Sm[d][2] += wab * Q[d];
+      }
+    }
+}
+
+// xb += sum_i h_i grad w_i with h_i = c0 g.x + (g.y, g.z, g.w) . (q + Aff off)
+template <int D, class R, bool TILE, class S>
+__device__ __forceinline__ void ad_grad_w(const S& src, const R (&w)[3][3], const R (&dw)[3][3], R c0, const R (&q)[3],
+                                          const R (&Aff)[9], R (&xb)[3]) {
+#pragma unroll(TILE ? 3 : 1)
+  for (int a = 0; a < 3; ++a)
+#pragma unroll(TILE ? 3 : 1)
+    for (int b = 0; b < 3; ++b) {
+      R qab[3], H = 0, Hd = 0;
+#pragma unroll
+      for (int d = 0; d < D; ++d) qab[d] = q[d] + (R)a * Aff[d * D] + (R)b * Aff[d * D + 1];
+#pragma unroll(TILE ? 3 : 1)
+      for (int c = 0; c < (D == 3 ? 3 : 1); ++c) {
+        const auto g = src(a, b, c);
+        const R gv[3] = {g.y, g.z, g.w};
+        R h = c0 * g.x;
+#pragma unroll
+        for (int d = 0; d < D; ++d) h += gv[d] * (D == 3 ? qab[d] + (R)c * Aff[d * D + 2] : qab[d]);
+        if (D == 3) {
+          H += w[c][2] * h;
+          Hd += dw[c][2] * h;
+        } else {
+          H = h;
+        }
+      }
+      xb[0] += dw[a][0] * w[b][1] * H;
+      xb[1] += w[a][0] * dw[b][1] * H;
+      if (D == 3) xb[2] += w[a][0] * w[b][1] * Hd;
+    }
+}
+
+// Add w (m0, q + Aff off) into the particle's nodes: in the tile with plain
+// read-add-writes (lanes of the same base cell take turns, and an offset's
+// updates are visible to the warp before the next one's: lanes of
+// neighbouring cells reach a node at different offsets), else with global
+// reductions.  All lanes call it.
+template <int D, class R, bool TILE, class R4>
+__device__ __forceinline__ void ad_scatter(const AdK<R>& K, bool on, const int (&base)[3], R4* tile, const AdBox& box,
+                                           R4* grid, const R (&w)[3][3], R m0, const R (&q)[3], const R (&Aff)[9]) {
+  const int lane = threadIdx.x & 31;
+  const int lb = TILE ? ad_local<D>(box, base) : 0;
+  int rank = 0, rounds = 1;
+  if (TILE) {
+    const unsigned peers = __match_any_sync(0xffffffffu, on ? lb : -1 - lane);
+    rank = __popc(peers & ((1u << lane) - 1u));
+    rounds = (int)__reduce_max_sync(0xffffffffu, (unsigned)__popc(peers));
+  }
+  const int sb = D == 3 ? box.e2 : 1, sa = D == 3 ? box.e1 * box.e2 : box.e1;
+  for (int r = 0; r < rounds; ++r) {
+    const bool mine = on && rank == r;
+    const unsigned tm = __ballot_sync(0xffffffffu, mine);
+    if (mine) {
+#pragma unroll(TILE ? 3 : 1)
+      for (int a = 0; a < 3; ++a)
+#pragma unroll(TILE ? 3 : 1)
+        for (int b = 0; b < 3; ++b) {
+          const R wab = w[a][0] * w[b][1];
+          R qab[3] = {0, 0, 0};
+#pragma unroll
+          for (int d = 0; d < D; ++d) qab[d] = q[d] + (R)a * Aff[d * D] + (R)b * Aff[d * D + 1];
+#pragma unroll(TILE ? 3 : 1)
+          for (int c = 0; c < (D == 3 ? 3 : 1); ++c) {
+            const R wt = D == 3 ? wab * w[c][2] : wab;
+            R val[3] = {0, 0, 0};
+#pragma unroll
+            for (int d = 0; d < D; ++d) val[d] = wt * (D == 3 ? qab[d] + (R)c * Aff[d * D + 2] : qab[d]);
+            if (TILE) {
+              R4& t = tile[lb + a * sa + b * sb + c];
+              R4 v = t;
+              v.x += wt * m0;
+              v.y += val[0];
+              v.z += val[1];
+              if (D == 3) v.w += val[2];
+              t = v;
+              __syncwarp(tm);
+            } else {
+              const int I[3] = {base[0] + a, base[1] + b, D == 3 ? base[2] + c : 0};
+              red_add_node(grid + ad_cell<D>(K.res, I), wt * m0, val[0], val[1], val[2]);
+            }
+          }
+        }
+    }
+    __syncwarp();
+  }
+}
+
+// zero a grid for a later scatter (grid-stride over its nodes)
+template <class R4>
+__device__ __forceinline__ void ad_clear(R4* g, int64_t nodes) {
+  if (!g) return;
+  R4 z;
+  z.x = z.y = z.z = z.w = 0;
+  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nodes; j += (int64_t)gridDim.x * blockDim.x)
+    g[j] = z;
+}
+
+// P2G terms of a particle: Aff = A dx, q = m v - Aff fx
+template <int D, bool HF, class R>
+__device__ __forceinline__ void ad_p2g_terms(const AdK<R>& K, const R* s, const R (&fx)[3], R (&q)[3], R (&Aff)[9]) {
+  typedef Sch<D, HF, false> S;
+  R sig[9];
+  ad_sigma<D, HF, R>(K, s, sig);
+#pragma unroll
+  for (int k = 0; k < D * D; ++k) Aff[k] = (K.kst * sig[k] + K.p_mass * s[S::C + k]) * K.dx;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    so[S::X + d] = s[S::X + d] + K.dt * nv[d];
-    so[S::V + d] = nv[d];
+    q[d] = K.p_mass * s[S::V + d];
+#pragma unroll
+    for (int e = 0; e < D; ++e) q[d] -= Aff[d * D + e] * fx[e];
   }
+}
+
+// Threads per CTA.  A CTA is no unit of work here; two warps keep the
+// granularity of shared memory fine.
+constexpr int AD_T = 64;
+
+// ------------------------------------------------------------- forward
+
+// A pass of the forward chain: G2P of one substep (state in -> out, from the
+// sums in gin) and / or P2G of the next (of the new state, or of `in`) into
+// gout, which is zero; gclr (may be null) is zeroed for the pass after.
+template <int D, bool HF, class R, bool G2P, bool P2G>
+__global__ void __launch_bounds__(AD_T) k_ad_pass(const __grid_constant__ AdK<R> K, const R* __restrict__ in,
+                                                  R* __restrict__ out, int64_t n,
+                                                  const typename R4T<R>::type* __restrict__ gin,
+                                                  typename R4T<R>::type* gout, typename R4T<R>::type* gclr,
+                                                  int64_t nodes) {
+  typedef Sch<D, HF, false> S;
+  typedef typename R4T<R>::type R4;
+  constexpr int NS = S::NS;
+  __shared__ __align__(16) R4 tiles[AD_T / 32][AdTile<D>::N];
+  R4* const tile = tiles[threadIdx.x >> 5];
+  ad_clear(gclr, nodes);
+  const int64_t p = (int64_t)blockIdx.x * AD_T + threadIdx.x;
+  const bool on = p < n;
+  R s[NS];
+  int base[3] = {0, 0, 0};
+  R fx[3] = {0, 0, 0}, w[3][3];
+  if (on) ad_load<NS, 0, NS>(in, p, s);
+  if (G2P) {
+    if (on) ad_weights<D, R>(s + S::X, K, base, fx, w);
+    const AdBox box = ad_box<D>(on, base);
+    const AdGridOp<D, R> node{K, gin};
+    R nv[3], Sm[3][3];
+    if (box.fits) {
+      ad_stage<D>(box, tile, node);
+      const AdSrc<D, R, true, AdGridOp<D, R>> src{tile + (on ? ad_local<D>(box, base) : 0),
+                                                  D == 3 ? box.e1 * box.e2 : box.e1, D == 3 ? box.e2 : 1, node, base};
+      if (on) ad_gather<D, R, true>(src, w, nv, Sm);
+      __syncwarp();
+    } else if (on) {
+      const AdSrc<D, R, false, AdGridOp<D, R>> src{nullptr, 0, 0, node, base};
+      ad_gather<D, R, false>(src, w, nv, Sm);
+    }
+    if (on) {
+      R nC[9];
 #pragma unroll
-  for (int k = 0; k < D * D; ++k) so[S::C + k] = nC[k];
-  if (HF) {
+      for (int d = 0; d < D; ++d)
 #pragma unroll
-    for (int i = 0; i < D; ++i)
+        for (int e = 0; e < D; ++e) nC[d * D + e] = K.four_inv_dx * (Sm[d][e] - nv[d] * fx[e]);
 #pragma unroll
-      for (int j = 0; j < D; ++j) {
-        R a = 0;
-#pragma unroll
-        for (int k = 0; k < D; ++k) a += ((i == k ? (R)1 : (R)0) + K.dt * nC[i * D + k]) * s[S::FJ + k * D + j];
-        so[S::FJ + i * D + j] = a;
+      for (int d = 0; d < D; ++d) {
+        s[S::X + d] += K.dt * nv[d];
+        s[S::V + d] = nv[d];
       }
-  } else {
-    R tr = 0;
 #pragma unroll
-    for (int d = 0; d < D; ++d) tr += nC[d * D + d];
-    so[S::FJ] = ((R)1 + K.dt * tr) * s[S::FJ];
+      for (int k = 0; k < D * D; ++k) s[S::C + k] = nC[k];
+      if (HF) {
+        R nF[9];
+#pragma unroll
+        for (int i = 0; i < D; ++i)
+#pragma unroll
+          for (int j = 0; j < D; ++j) {
+            R a = 0;
+#pragma unroll
+            for (int k = 0; k < D; ++k) a += ((i == k ? (R)1 : (R)0) + K.dt * nC[i * D + k]) * s[S::FJ + k * D + j];
+            nF[i * D + j] = a;
+          }
+#pragma unroll
+        for (int k = 0; k < D * D; ++k) s[S::FJ + k] = nF[k];
+      } else {
+        R tr = 0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) tr += nC[d * D + d];
+        s[S::FJ] = ((R)1 + K.dt * tr) * s[S::FJ];
+      }
+#pragma unroll
+      for (int k = 0; k < NS; ++k) out[ad_at<NS>(p, k)] = s[k];
+    }
+  }
+  if (P2G) {
+    R q[3], Aff[9];
+    if (on) {
+      ad_weights<D, R>(s + S::X, K, base, fx, w);
+      ad_p2g_terms<D, HF, R>(K, s, fx, q, Aff);
+    }
+    const AdBox box = ad_box<D>(on, base);
+    if (box.fits) {
+      ad_zero(box, tile);
+      ad_scatter<D, R, true>(K, on, base, tile, box, gout, w, K.p_mass, q, Aff);
+      ad_flush<D, R>(K, box, tile, gout);
+    } else {
+      ad_scatter<D, R, false>(K, on, base, tile, box, gout, w, K.p_mass, q, Aff);
+    }
   }
 }
 
 // ------------------------------------------------------------- reverse
 
-// G2P^T: from the adjoint of the new state (ab_out) to the adjoint of the
-// old state's x and F|J (ab_in, overwritten) and the grid velocity adjoint
-// (gvb, accumulated).
+// G2P^T: from the adjoint of the new state (ab_out) to the x and F|J parts
+// of the old state's adjoint (ab_in) and the grid velocity's adjoint (added
+// to gvb, zero before).  With q = v'bar - 4/dx C'bar fx and Aff = 4/dx C'bar:
+// vbar_i += w (q + Aff off), wbar_i = v_i . (q + Aff off), and through dpos
+// xbar -= 4/dx^2 C'bar^T sum w v.
 template <int D, bool HF, class R>
-__global__ void __launch_bounds__(128) k_ad_g2p_bwd(const AdK<R> K, const R* __restrict__ st,
-                                                    const R* __restrict__ gv, const R* __restrict__ ab_out,
-                                                    R* __restrict__ ab_in, R* __restrict__ gvb, int64_t n) {
+__global__ void __launch_bounds__(AD_T) k_ad_g2p_bwd(const __grid_constant__ AdK<R> K, const R* __restrict__ st,
+                                                     const R* __restrict__ ab_out, R* __restrict__ ab_in, int64_t n,
+                                                     const typename R4T<R>::type* __restrict__ grid,
+                                                     typename R4T<R>::type* gvb, typename R4T<R>::type* gclr,
+                                                     int64_t nodes) {
   typedef Sch<D, HF, false> S;
-  const int64_t p0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = p0 < n;
-  if (__all_sync(0xffffffffu, !active)) return;
-  const int64_t p = active ? p0 : n - 1;  // lanes past the end take part in the shuffles only
-  const R* s = st + p * K.NS;
-  const R* bo = ab_out + p * K.NS;
-  R* bi = ab_in + p * K.NS;
-  int base[3];
-  R fx[3], w[3][3], dw[3][3];
-  ad_weights<D, R>(s + S::X, K, base, fx, w, dw);
-  const WarpRuns runs = warp_runs(active ? (long long)ad_cell<D>(K.res, base) : -1 - (long long)(threadIdx.x & 31));
-  // recompute new C (needed for F' = (I + dt C') F)
-  R nC[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int o = 0; o < (D == 3 ? 27 : 9); ++o) {
-    int off[3], I[3];
-    offs<D>(o, off);
-    R wt = 1, dpos[3];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      wt *= w[off[d]][d];
-      dpos[d] = ((R)off[d] - fx[d]) * K.dx;
-      I[d] = base[d] + off[d];
-    }
-    const R* g = gv + 4 * ad_cell<D>(K.res, I);
+  typedef typename R4T<R>::type R4;
+  constexpr int NS = S::NS;
+  extern __shared__ __align__(16) unsigned char ad_smem[];
+  R4* const tile = reinterpret_cast<R4*>(ad_smem) + (threadIdx.x >> 5) * 2 * AdTile<D>::N;
+  R4* const stile = tile + AdTile<D>::N;
+  ad_clear(gclr, nodes);
+  const int64_t p = (int64_t)blockIdx.x * AD_T + threadIdx.x;
+  const bool on = p < n;
+  R s[NS], bo[NS];
+  int base[3] = {0, 0, 0};
+  R fx[3] = {0, 0, 0}, w[3][3];
+  if (on) {
+    ad_load<NS, S::X, S::X + D>(st, p, s);
+    ad_load<NS, S::FJ, NS>(st, p, s);
+    ad_load<NS, 0, NS>(ab_out, p, bo);
+    ad_weights<D, R>(s + S::X, K, base, fx, w);
+  }
+  const AdBox box = ad_box<D>(on, base);
+  const AdGridOp<D, R> node{K, grid};
+  R nv[3], Sm[3][3];
+  const AdSrc<D, R, true, AdGridOp<D, R>> src{tile + (on && box.fits ? ad_local<D>(box, base) : 0),
+                                              D == 3 ? box.e1 * box.e2 : box.e1, D == 3 ? box.e2 : 1, node, base};
+  const AdSrc<D, R, false, AdGridOp<D, R>> gsrc{nullptr, 0, 0, node, base};
+  if (box.fits) {
+    ad_stage<D>(box, tile, node);
+    ad_zero(box, stile);
+    if (on) ad_gather<D, R, true>(src, w, nv, Sm);
+  } else if (on) {
+    ad_gather<D, R, false>(gsrc, w, nv, Sm);
+  }
+  R q[3], Aff[9], xb[3] = {0, 0, 0};
+  if (on) {
+    R nC[9];
 #pragma unroll
     for (int d = 0; d < D; ++d)
 #pragma unroll
-      for (int e = 0; e < D; ++e) nC[d * D + e] += K.four_inv_dx2 * wt * g[d] * dpos[e];
-  }
-  R xb[3] = {0, 0, 0}, vpb[3] = {0, 0, 0}, Cpb[9];
+      for (int e = 0; e < D; ++e) nC[d * D + e] = K.four_inv_dx * (Sm[d][e] - nv[d] * fx[e]);
+    R Cpb[9];
 #pragma unroll
-  for (int k = 0; k < D * D; ++k) Cpb[k] = bo[S::C + k];
-  R FJb[9];
-  if (HF) {
-    // F' = (I + dt C') F
+    for (int k = 0; k < D * D; ++k) Cpb[k] = bo[S::C + k];
+    if (HF) {
+      // F' = (I + dt C') F
 #pragma unroll
-    for (int i = 0; i < D; ++i)
+      for (int i = 0; i < D; ++i)
 #pragma unroll
-      for (int j = 0; j < D; ++j) {
-        R a = 0, c = 0;
+        for (int j = 0; j < D; ++j) {
+          R a = 0, c = 0;
 #pragma unroll
-        for (int k = 0; k < D; ++k) {
-          a += ((k == i ? (R)1 : (R)0) + K.dt * nC[k * D + i]) * bo[S::FJ + k * D + j];  // (I+dtC')^T F'bar
-          c += bo[S::FJ + i * D + k] * s[S::FJ + j * D + k];                            // F'bar F^T
+          for (int k = 0; k < D; ++k) {
+            a += ((k == i ? (R)1 : (R)0) + K.dt * nC[k * D + i]) * bo[S::FJ + k * D + j];  // (I+dtC')^T F'bar
+            c += bo[S::FJ + i * D + k] * s[S::FJ + j * D + k];                            // F'bar F^T
+          }
+          ab_in[ad_at<NS>(p, S::FJ + i * D + j)] = a;
+          Cpb[i * D + j] += K.dt * c;
         }
-        FJb[i * D + j] = a;
-        Cpb[i * D + j] += K.dt * c;
-      }
-  } else {
-    R tr = 0;
+    } else {
+      R tr = 0;
 #pragma unroll
-    for (int d = 0; d < D; ++d) tr += nC[d * D + d];
-    FJb[0] = ((R)1 + K.dt * tr) * bo[S::FJ];
-    const R trb = K.dt * s[S::FJ] * bo[S::FJ];
+      for (int d = 0; d < D; ++d) tr += nC[d * D + d];
+      ab_in[ad_at<NS>(p, S::FJ)] = ((R)1 + K.dt * tr) * bo[S::FJ];
+      const R trb = K.dt * s[S::FJ] * bo[S::FJ];
 #pragma unroll
-    for (int d = 0; d < D; ++d) Cpb[d * D + d] += trb;
-  }
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    xb[d] = bo[S::X + d];
-    vpb[d] = bo[S::V + d] + K.dt * bo[S::X + d];
-  }
-  for (int o = 0; o < (D == 3 ? 27 : 9); ++o) {
-    int off[3], I[3];
-    offs<D>(o, off);
-    R wt = 1, dpos[3];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      wt *= w[off[d]][d];
-      dpos[d] = ((R)off[d] - fx[d]) * K.dx;
-      I[d] = base[d] + off[d];
+      for (int d = 0; d < D; ++d) Cpb[d * D + d] += trb;
     }
-    const int64_t cell = ad_cell<D>(K.res, I);
-    const R* g = gv + 4 * cell;
-    R wb = 0;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      R cd = 0;  // (C'bar dpos)_d
-#pragma unroll
-      for (int e = 0; e < D; ++e) cd += Cpb[d * D + e] * dpos[e];
-      const R vb = run_sum(active ? wt * (vpb[d] + K.four_inv_dx2 * cd) : (R)0, runs);
-      if (active && runs.head) atomicAdd(gvb + 4 * cell + d, vb);
-      wb += g[d] * (vpb[d] + K.four_inv_dx2 * cd);
-    }
-    // through dpos = x_i - x_p: xbar -= 4/dx^2 w C'bar^T v_i
 #pragma unroll
     for (int e = 0; e < D; ++e) {
-      R a = 0;
+      xb[e] = bo[S::X + e];
 #pragma unroll
-      for (int d = 0; d < D; ++d) a += Cpb[d * D + e] * g[d];
-      xb[e] -= K.four_inv_dx2 * wt * a;
+      for (int d = 0; d < D; ++d) xb[e] -= K.four_inv_dx2 * Cpb[d * D + e] * nv[d];
     }
-    // through w
+#pragma unroll
+    for (int k = 0; k < D * D; ++k) Aff[k] = K.four_inv_dx * Cpb[k];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      R gw = dw[off[d]][d];
+      q[d] = bo[S::V + d] + K.dt * bo[S::X + d];
 #pragma unroll
-      for (int e = 0; e < D; ++e)
-        if (e != d) gw *= w[off[e]][e];
-      xb[d] += wb * gw;
+      for (int e = 0; e < D; ++e) q[d] -= Aff[d * D + e] * fx[e];
     }
+    R dw[3][3];
+    ad_dweights<D, R>(K, fx, dw);
+    if (box.fits)
+      ad_grad_w<D, R, true>(src, w, dw, (R)0, q, Aff, xb);
+    else
+      ad_grad_w<D, R, false>(gsrc, w, dw, (R)0, q, Aff, xb);
+#pragma unroll
+    for (int d = 0; d < D; ++d) ab_in[ad_at<NS>(p, S::X + d)] = xb[d];
   }
-  if (!active) return;
-  for (int k = 0; k < K.NS; ++k) bi[k] = 0;
-#pragma unroll
-  for (int d = 0; d < D; ++d) bi[S::X + d] = xb[d];
-  if (HF) {
-#pragma unroll
-    for (int k = 0; k < D * D; ++k) bi[S::FJ + k] = FJb[k];
+  if (box.fits) {
+    ad_scatter<D, R, true>(K, on, base, stile, box, gvb, w, (R)0, q, Aff);
+    ad_flush<D, R>(K, box, stile, gvb);
   } else {
-    bi[S::FJ] = FJb[0];
+    ad_scatter<D, R, false>(K, on, base, stile, box, gvb, w, (R)0, q, Aff);
   }
 }
 
-// grid^T: from the velocity adjoint to the (m, P) adjoint, in place in gvb
-template <int D, class R>
-__global__ void __launch_bounds__(256) k_ad_grid_bwd(const AdK<R> K, const R* __restrict__ grid,
-                                                     R* __restrict__ gvb, int64_t ncell) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncell) return;
-  int I[3] = {0, 0, 0};
-  if (D == 3) {
-    I[2] = (int)(c % K.res[2]);
-    I[1] = (int)((c / K.res[2]) % K.res[1]);
-    I[0] = (int)(c / ((int64_t)K.res[2] * K.res[1]));
-  } else {
-    I[1] = (int)(c % K.res[1]);
-    I[0] = (int)(c / K.res[1]);
-  }
-  const R* g = grid + 4 * c;
-  const R me = g[0] + (R)1e-10;
-  const R inv_m = (R)1 / me;
-  R v[3] = {0, 0, 0};
+// Sums over the warp of NS values per lane, in 31 exchanges: in each step the
+// two halves of a lane group keep half of the values each.  Lane l returns
+// the sum of value l.
+template <int NS>
+__device__ __forceinline__ double ad_warp_sums(const double (&v)[NS]) {
+  double a[32];
 #pragma unroll
-  for (int d = 0; d < D; ++d) v[d] = inv_m * g[1 + d];
-  v[1] -= K.dt * K.grav;
-  R vb[3] = {0, 0, 0};
+  for (int k = 0; k < 32; ++k) a[k] = k < NS ? v[k] : 0.0;
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int d = 0; d < D; ++d) vb[d] = gvb[4 * c + d];
-  if (D == 3 && K.col_on) {
-    // collider^T: where the node is inside and moving into the surface
-    // (relative to the collider), the forward removed the normal part of
-    // the velocity, v' = v - ((v - cv).n) n, so vbar' = vbar - (vbar.n) n
-    R nrm[3], cv[3];
-    if (collider_at<R, true>(K, K.pose, I[0], I[1], I[2], nrm, cv)) {
-      R dn = 0, bn = 0;
+  for (int h = 16; h; h >>= 1) {
+    const bool up = lane & h;
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const R vw = ad_wall<R>(K, I, k, v[k]) ? (R)0 : v[k];  // the collider's input
-        dn += (vw - cv[k]) * nrm[k];
-        bn += vb[k] * nrm[k];
-      }
-      if (dn < (R)0)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) vb[k] -= bn * nrm[k];
+    for (int k = 0; k < h; ++k) {
+      const double keep = up ? a[k + h] : a[k], give = up ? a[k] : a[k + h];
+      a[k] = keep + __shfl_xor_sync(0xffffffffu, give, h);
     }
   }
-  R mb = 0, Pb[3] = {0, 0, 0};
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    R b = vb[d];
-    if (ad_wall<R>(K, I, d, v[d])) b = 0;
-    Pb[d] = b * inv_m;
-    mb -= b * g[1 + d] * inv_m * inv_m;
-  }
-  gvb[4 * c + 0] = mb;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) gvb[4 * c + 1 + d] = d < D ? Pb[d] : (R)0;
+  return a[0];
 }
 
-// P2G^T: adds the old-state adjoint through P2G into ab_in
+constexpr int AD_SENS_COPIES = 32;  // copies of the sensitivity sums, so that CTAs' additions do not queue on one
+
+// P2G^T: the old state's adjoint, completed (ab_in holds G2P^T's part on
+// entry); with sens, its squares are added to the sensitivity sums in FP64.
 template <int D, bool HF, class R>
-__global__ void __launch_bounds__(128) k_ad_p2g_bwd(const AdK<R> K, const R* __restrict__ st,
-                                                    const R* __restrict__ gb, R* __restrict__ ab_in, int64_t n) {
+__global__ void __launch_bounds__(AD_T) k_ad_p2g_bwd(const __grid_constant__ AdK<R> K, const R* __restrict__ st,
+                                                     R* ab_in, int64_t n,
+                                                     const typename R4T<R>::type* __restrict__ grid,
+                                                     const typename R4T<R>::type* __restrict__ gvb,
+                                                     double* __restrict__ sens) {
   typedef Sch<D, HF, false> S;
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const R* s = st + p * K.NS;
-  R* bi = ab_in + p * K.NS;
-  int base[3];
-  R fx[3], w[3][3], dw[3][3];
-  ad_weights<D, R>(s + S::X, K, base, fx, w, dw);
-  R sig[9], A[9];
-  ad_sigma<D, HF, R>(K, s, sig);
-#pragma unroll
-  for (int k = 0; k < D * D; ++k) A[k] = K.kst * sig[k] + K.p_mass * s[S::C + k];
-  R xb[3] = {0, 0, 0}, vb[3] = {0, 0, 0}, Ab[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int o = 0; o < (D == 3 ? 27 : 9); ++o) {
-    int off[3], I[3];
-    offs<D>(o, off);
-    R wt = 1, dpos[3];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      wt *= w[off[d]][d];
-      dpos[d] = ((R)off[d] - fx[d]) * K.dx;
-      I[d] = base[d] + off[d];
+  typedef typename R4T<R>::type R4;
+  constexpr int NS = S::NS;
+  __shared__ __align__(16) R4 tiles[AD_T / 32][AdTile<D>::N];
+  R4* const tile = tiles[threadIdx.x >> 5];
+  const int64_t p = (int64_t)blockIdx.x * AD_T + threadIdx.x;
+  const bool on = p < n;
+  R s[NS], bi[NS];
+  int base[3] = {0, 0, 0};
+  R fx[3] = {0, 0, 0}, w[3][3];
+  if (on) {
+    ad_load<NS, 0, NS>(st, p, s);
+    ad_load<NS, S::X, S::X + D>(ab_in, p, bi);
+    ad_load<NS, S::FJ, NS>(ab_in, p, bi);
+    ad_weights<D, R>(s + S::X, K, base, fx, w);
+  }
+  const AdBox box = ad_box<D>(on, base);
+  const AdGridOpT<D, R> node{K, grid, gvb};
+  R nv[3], Sm[3][3], q[3], Aff[9], dw[3][3], xb[3] = {0, 0, 0};
+  if (on) {
+    ad_p2g_terms<D, HF, R>(K, s, fx, q, Aff);
+    ad_dweights<D, R>(K, fx, dw);
+  }
+  if (box.fits) {
+    ad_stage<D>(box, tile, node);
+    const AdSrc<D, R, true, AdGridOpT<D, R>> src{tile + (on ? ad_local<D>(box, base) : 0),
+                                                 D == 3 ? box.e1 * box.e2 : box.e1, D == 3 ? box.e2 : 1, node, base};
+    if (on) {
+      ad_gather<D, R, true>(src, w, nv, Sm);
+      ad_grad_w<D, R, true>(src, w, dw, K.p_mass, q, Aff, xb);
     }
-    const R* g = gb + 4 * ad_cell<D>(K.res, I);
-    const R mb = g[0];
-    R wb = K.p_mass * mb;
+  } else if (on) {
+    const AdSrc<D, R, false, AdGridOpT<D, R>> src{nullptr, 0, 0, node, base};
+    ad_gather<D, R, false>(src, w, nv, Sm);
+    ad_grad_w<D, R, false>(src, w, dw, K.p_mass, q, Aff, xb);
+  }
+  if (on) {
+    R sb[9];
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      const R Pb = g[1 + d];
-      R a = K.p_mass * s[S::V + d];
-#pragma unroll
-      for (int e = 0; e < D; ++e) a += A[d * D + e] * dpos[e];
-      wb += Pb * a;
-      vb[d] += wt * K.p_mass * Pb;
+    for (int d = 0; d < D; ++d)
 #pragma unroll
       for (int e = 0; e < D; ++e) {
-        Ab[d * D + e] += wt * Pb * dpos[e];
-        xb[e] -= wt * A[d * D + e] * Pb;  // through dpos = x_i - x_p
+        const R Ab = K.dx * (Sm[d][e] - nv[d] * fx[e]);
+        bi[S::C + d * D + e] = K.p_mass * Ab;
+        sb[d * D + e] = K.kst * Ab;
+        xb[e] -= Aff[d * D + e] * K.inv_dx * nv[d];  // through dpos = x_i - x_p
       }
-    }
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      R gw = dw[off[d]][d];
+      bi[S::X + d] += xb[d];
+      bi[S::V + d] = K.p_mass * nv[d];
+    }
+    ad_sigma_bwd<D, HF, R>(K, s, sb, bi);
 #pragma unroll
-      for (int e = 0; e < D; ++e)
-        if (e != d) gw *= w[off[e]][e];
-      xb[d] += wb * gw;
+    for (int k = 0; k < NS; ++k) ab_in[ad_at<NS>(p, k)] = bi[k];
+  }
+  if (sens) {
+    double sq[NS];
+#pragma unroll
+    for (int k = 0; k < NS; ++k) sq[k] = on ? (double)bi[k] * (double)bi[k] : 0.0;
+    const double t = ad_warp_sums<NS>(sq);
+    __shared__ double part[AD_T / 32][32];
+    part[threadIdx.x >> 5][threadIdx.x & 31] = t;
+    __syncthreads();
+    if (threadIdx.x < NS) {
+      double a = 0;
+#pragma unroll
+      for (int k = 0; k < AD_T / 32; ++k) a += part[k][threadIdx.x];
+      atomicAdd(sens + (blockIdx.x % AD_SENS_COPIES) * NS + threadIdx.x, a);
     }
   }
-  R sb[9];
-#pragma unroll
-  for (int k = 0; k < D * D; ++k) {
-    bi[S::C + k] += K.p_mass * Ab[k];
-    sb[k] = K.kst * Ab[k];
-  }
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    bi[S::X + d] += xb[d];
-    bi[S::V + d] += vb[d];
-  }
-  ad_sigma_bwd<D, HF, R>(K, s, sb, bi);
 }
 
-template <class R>
-__global__ void k_ad_accum(const R* __restrict__ ab, int64_t n, int ns, double* __restrict__ sens) {
-  extern __shared__ double shs[];
-  for (int s = threadIdx.x; s < ns; s += blockDim.x) shs[s] = 0;
-  __syncthreads();
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * ns; i += (int64_t)gridDim.x * blockDim.x) {
-    const double v = (double)ab[i];
-    atomicAdd(&shs[i % ns], v * v);
-  }
-  __syncthreads();
-  for (int s = threadIdx.x; s < ns; s += blockDim.x) atomicAdd(&sens[s], shs[s]);
-}
+// ------------------------------------------------------------- order
+//
+// Order of the particles inside the library, from their base cells at the
+// start (they move little over an adjoint horizon): by cell block (4^3 or
+// 8^2) along a serpentine, so that blocks that follow each other are
+// neighbours; inside a block the first particle of every cell, then the
+// second of every cell, and so on, so that a warp's lanes scatter from
+// different cells.
+constexpr int AD_RANK_BITS = 10;  // ranks beyond 2^10 - 1 share the last place
 
-// Particle order for locality: the key of a particle is its base cell
-// (row-major), clamped to the grid; sorting the state by it once per forward
-// pass puts the particles a warp scatters from and gathers into next to
-// each other on the grid (they move little over an adjoint horizon).
 template <class R>
 __global__ void k_ad_keys(const R* __restrict__ st, int64_t n, int ns, int D, int r0, int r1, int r2, R inv_dx,
-                          int32_t* __restrict__ keys, int32_t* __restrict__ idx) {
+                          int32_t* __restrict__ count, uint64_t* __restrict__ keys, int32_t* __restrict__ idx) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int res[3] = {r0, r1, r2};
-  int64_t key = 0;
+  const int bs = D == 3 ? 2 : 3;  // log2 of the block's edge
+  int64_t cell = 0;
+  int b[3] = {0, 0, 0};
   for (int d = 0; d < D; ++d) {
     const R t = st[i * ns + d] * inv_dx - (R)0.5;
-    int b = t == t ? (int)floor(t) : 0;
-    b = min(max(b, 0), res[d] - 1);
-    key = key * res[d] + b;
+    const int f = t == t ? (int)floor(t) : 0;
+    b[d] = min(max(f, 0), res[d] - 1);
+    cell = cell * res[d] + b[d];
   }
-  keys[i] = (int32_t)key;
+  const int rank = min(atomicAdd(count + cell, 1), (1 << AD_RANK_BITS) - 1);
+  uint64_t blk = 0;
+  int turn = 0;  // whether this axis runs backwards
+  for (int d = 0; d < D; ++d) {
+    const int nb = (res[d] + (1 << bs) - 1) >> bs, q = b[d] >> bs;
+    const int at = turn ? nb - 1 - q : q;
+    blk = blk * nb + at;
+    turn ^= at & 1;
+  }
+  const int m = (1 << bs) - 1;
+  // cells z fastest, then x, then y, as the simulator's binning
+  const int c = D == 3 ? (((b[1] & m) << 2 | (b[0] & m)) << 2) | (b[2] & m) : ((b[0] & m) << 3) | (b[1] & m);
+  keys[i] = ((blk << AD_RANK_BITS) | (uint64_t)rank) << 6 | (uint64_t)c;
   idx[i] = (int32_t)i;
 }
 
-// rows of a state: out[i] = in[perm[i]] (gather) or out[perm[i]] = in[i]
-template <class R>
-__global__ void k_ad_permute(const R* __restrict__ in, R* __restrict__ out, const int32_t* __restrict__ perm, int64_t n,
-                             int ns, int gather) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n * ns) return;
-  const int64_t i = k / ns, s = k - i * ns;
-  const int64_t j = perm[i];
-  if (gather)
-    out[i * ns + s] = in[j * ns + s];
-  else
-    out[j * ns + s] = in[i * ns + s];
+// Between the caller's rows (n x ns, the caller's order) and the library's
+// groups: a warp moves a group through shared memory, so that both sides are
+// read and written in contiguous runs.  TO: rows -> groups.
+template <class R, bool TO>
+__global__ void __launch_bounds__(128) k_ad_permute(const R* __restrict__ in, R* __restrict__ out,
+                                                    const int32_t* __restrict__ perm, int64_t n, int ns) {
+  __shared__ R sh[4][32][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t g = (int64_t)blockIdx.x * 4 + warp;
+  if (g * 32 >= n) return;
+  const int cnt = (int)min((int64_t)32, n - g * 32);
+  const int64_t row = lane < cnt ? (int64_t)perm[g * 32 + lane] * ns : 0;
+  if (TO) {
+    for (int r = 0; r < cnt; ++r) {
+      const int64_t at = __shfl_sync(0xffffffffu, row, r);
+      if (lane < ns) sh[warp][r][lane] = in[at + lane];
+    }
+    __syncwarp();
+    for (int s = 0; s < ns; ++s)
+      if (lane < cnt) out[(g * ns + s) * 32 + lane] = sh[warp][lane][s];
+  } else {
+    for (int s = 0; s < ns; ++s)
+      if (lane < cnt) sh[warp][lane][s] = in[(g * ns + s) * 32 + lane];
+    __syncwarp();
+    for (int r = 0; r < cnt; ++r) {
+      const int64_t at = __shfl_sync(0xffffffffu, row, r);
+      if (lane < ns) out[at + lane] = sh[warp][r][lane];
+    }
+  }
 }
 
 // --------------------------------------------------------------- host
 
 struct AdBase {
   virtual ~AdBase() {}
+  virtual int setup() = 0;
   // t: index of the substep (the collider's angle and height depend on it)
-  virtual int step(const void* in, void* out, int t, cudaStream_t st) = 0;
-  virtual int step_bwd(const void* s_in, const void* ab_out, void* ab_in, int t, cudaStream_t st) = 0;
-  virtual int accum(const void* ab, double* sens, cudaStream_t st) = 0;
-  virtual int sort_keys(const void* s0, int32_t* keys, int32_t* idx, cudaStream_t st) = 0;
+  virtual int p2g(const void* in, cudaStream_t st) = 0;
+  virtual int g2p(const void* in, void* out, int t, bool then_p2g, cudaStream_t st) = 0;
+  virtual int step_bwd(const void* s_in, const void* ab_out, void* ab_in, int t, bool accumulate, cudaStream_t st) = 0;
+  virtual int sort_keys(const void* s0, int32_t* count, uint64_t* keys, int32_t* idx, cudaStream_t st) = 0;
   virtual int permute(const void* in, void* out, bool gather, cudaStream_t st) = 0;
 };
 
@@ -719,16 +994,19 @@ struct aq_adjoint {
   int D = 0, NS = 0;
   int64_t n = 0, ncell = 0;
   size_t rsz = 4;
-  void* grid = nullptr;  // (m, P) per node
-  void* gv = nullptr;    // grid velocity per node
-  void* gvb = nullptr;   // velocity adjoint, then (m, P) adjoint
+  // three node grids in rotation: g[rot] takes (or holds) the current
+  // state's sums (m, P); every kernel that fills one of the others clears
+  // the one after, so that g[rot] is zero whenever a chain starts
+  void* g[3] = {nullptr, nullptr, nullptr};
+  int rot = 0;
   std::vector<void*> ckpt;  // states at multiples of the checkpoint interval (every > 0), or the initial state
-  std::vector<void*> seg;   // states of one segment (recomputed); two ping-pong states (every == 0)
+  std::vector<void*> seg;   // states between two checkpoints; two ping-pong states (every == 0)
   std::vector<void*> stash;  // bisection checkpointing: one state per recursion level, plus a scratch state
   int T = 0, every = 0;
+  int seg_of = -1;           // the segment whose states seg holds
   int32_t* perm = nullptr;  // sorted position -> caller's particle index (length n)
   int64_t recomputed = 0;   // forward substeps run again by the last backward pass
-  double* dsens = nullptr;
+  double* dsens = nullptr;  // AD_SENS_COPIES x NS
   aq::AdBase* impl = nullptr;
   // SDF collider (aq_adjoint_set_collider): caller-owned volumes; at
   // substep t the angle is theta + omega dt t and the height
@@ -737,21 +1015,29 @@ struct aq_adjoint {
   const float* col_sdf = nullptr;
   const float* col_nrm = nullptr;
   double col_theta = 0, col_height = 0, col_omega = 0, col_rate = 0;
+
+  size_t state_bytes() const { return rsz * NS * (size_t)aq::ad_padded(n); }
 };
 
 namespace aq {
 
+// I < lb and I > ub of a node index against a wall in doubles, as integers
+static int wall_lo(double lb) { return !(lb > -1e9) ? -1000000000 : lb > 1e9 ? 1000000000 : (int)ceil(lb); }
+static int wall_hi(double ub) { return !(ub < 1e9) ? 1000000000 : ub < -1e9 ? -1000000000 : (int)floor(ub); }
+
 template <int D, bool HF, class R>
 struct AdImpl final : AdBase {
+  typedef typename R4T<R>::type R4;
   aq_adjoint* a;
   AdK<R> K;
+  static constexpr int G2P_BWD_SMEM = (AD_T / 32) * 2 * AdTile<D>::N * (int)sizeof(R4);
   explicit AdImpl(aq_adjoint* adj) : a(adj) {
     const aq_params& P = adj->P;
     memset(&K, 0, sizeof(K));
     for (int d = 0; d < 3; ++d) {
       K.res[d] = d < D ? P.res[d] : 1;
-      K.lb[d] = P.lb[d];
-      K.ub[d] = P.ub[d];
+      K.wlo[d] = wall_lo(P.lb[d]);
+      K.whi[d] = wall_hi(P.ub[d]);
     }
     K.D = D;
     K.NS = adj->NS;
@@ -762,10 +1048,15 @@ struct AdImpl final : AdBase {
     K.dt = (R)P.dt;
     K.p_mass = (R)P.p_mass;
     K.kst = (R)(-(P.dt * P.p_vol * 4.0 * (1.0 / P.dx) * (1.0 / P.dx)));
+    K.four_inv_dx = (R)(4.0 / P.dx);
     K.four_inv_dx2 = (R)(4.0 / (P.dx * P.dx));
     K.grav = (R)P.gravity;
     K.mu = (R)P.mat[0].mu;
     K.lam = (R)P.mat[0].lam;
+  }
+  int setup() override {
+    AQ_CUDA_TRY(cudaFuncSetAttribute(k_ad_g2p_bwd<D, HF, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2P_BWD_SMEM));
+    return AQ_OK;
   }
   void set_substep(int t) {
     K.col_on = a->col_on;
@@ -786,91 +1077,103 @@ struct AdImpl final : AdBase {
     K.pose.s = (R)sin(th);
     K.pose.yshift = (int)(h / a->P.dx + 0.5);
   }
-  int step(const void* in, void* out, int t, cudaStream_t st) override {
+  R4* g(int k) const { return (R4*)a->g[(a->rot + k) % 3]; }
+  unsigned blocks() const { return grid_for(a->n, AD_T); }
+
+  // the sums of state `in` into g[rot]
+  int p2g(const void* in, cudaStream_t st) override {
+    k_ad_pass<D, HF, R, false, true><<<blocks(), AD_T, 0, st>>>(K, (const R*)in, nullptr, a->n, nullptr, g(0), g(1),
+                                                                a->ncell);
+    AQ_CUDA_TRY(cudaGetLastError());
+    return AQ_OK;
+  }
+  // substep t from the state whose sums are in g[rot], and the new state's
+  // sums, which g[rot] then names
+  int g2p(const void* in, void* out, int t, bool then_p2g, cudaStream_t st) override {
     set_substep(t);
-    const size_t gbytes = sizeof(R) * 4 * a->ncell;
-    AQ_CUDA_TRY(cudaMemsetAsync(a->grid, 0, gbytes, st));
-    k_ad_p2g<D, HF, R><<<grid_for(a->n, 128), 128, 0, st>>>(K, (const R*)in, a->n, (R*)a->grid);
-    k_ad_grid<D, R><<<grid_for(a->ncell, 256), 256, 0, st>>>(K, (const R*)a->grid, (R*)a->gv, a->ncell);
-    k_ad_g2p<D, HF, R><<<grid_for(a->n, 128), 128, 0, st>>>(K, (const R*)in, (const R*)a->gv, (R*)out, a->n);
+    if (then_p2g)
+      k_ad_pass<D, HF, R, true, true><<<blocks(), AD_T, 0, st>>>(K, (const R*)in, (R*)out, a->n, g(0), g(1), g(2),
+                                                                 a->ncell);
+    else
+      k_ad_pass<D, HF, R, true, false><<<blocks(), AD_T, 0, st>>>(K, (const R*)in, (R*)out, a->n, g(0), nullptr,
+                                                                  nullptr, 0);
     AQ_CUDA_TRY(cudaGetLastError());
+    a->rot = (a->rot + 1) % 3;
     return AQ_OK;
   }
-  int step_bwd(const void* s_in, const void* ab_out, void* ab_in, int t, cudaStream_t st) override {
+  // reverse of substep t, whose old state's sums are in g[rot]
+  int step_bwd(const void* s_in, const void* ab_out, void* ab_in, int t, bool accumulate, cudaStream_t st) override {
     set_substep(t);
-    const size_t gbytes = sizeof(R) * 4 * a->ncell;
-    // recompute the grid of this substep
-    AQ_CUDA_TRY(cudaMemsetAsync(a->grid, 0, gbytes, st));
-    k_ad_p2g<D, HF, R><<<grid_for(a->n, 128), 128, 0, st>>>(K, (const R*)s_in, a->n, (R*)a->grid);
-    k_ad_grid<D, R><<<grid_for(a->ncell, 256), 256, 0, st>>>(K, (const R*)a->grid, (R*)a->gv, a->ncell);
-    AQ_CUDA_TRY(cudaMemsetAsync(a->gvb, 0, gbytes, st));
-    k_ad_g2p_bwd<D, HF, R><<<grid_for(a->n, 128), 128, 0, st>>>(K, (const R*)s_in, (const R*)a->gv,
-                                                                 (const R*)ab_out, (R*)ab_in, (R*)a->gvb, a->n);
-    k_ad_grid_bwd<D, R><<<grid_for(a->ncell, 256), 256, 0, st>>>(K, (const R*)a->grid, (R*)a->gvb, a->ncell);
-    k_ad_p2g_bwd<D, HF, R><<<grid_for(a->n, 128), 128, 0, st>>>(K, (const R*)s_in, (const R*)a->gvb, (R*)ab_in,
-                                                                 a->n);
+    k_ad_g2p_bwd<D, HF, R><<<blocks(), AD_T, G2P_BWD_SMEM, st>>>(K, (const R*)s_in, (const R*)ab_out, (R*)ab_in, a->n,
+                                                                 g(0), g(1), g(2), a->ncell);
+    k_ad_p2g_bwd<D, HF, R><<<blocks(), AD_T, 0, st>>>(K, (const R*)s_in, (R*)ab_in, a->n, g(0), g(1),
+                                                      accumulate ? a->dsens : nullptr);
     AQ_CUDA_TRY(cudaGetLastError());
+    a->rot = (a->rot + 2) % 3;
     return AQ_OK;
   }
-  int accum(const void* ab, double* sens, cudaStream_t st) override {
-    k_ad_accum<R><<<num_sms() * 2, 256, sizeof(double) * a->NS, st>>>((const R*)ab, a->n, a->NS, sens);
-    AQ_CUDA_TRY(cudaGetLastError());
-    return AQ_OK;
-  }
-  int sort_keys(const void* s0, int32_t* keys, int32_t* idx, cudaStream_t st) override {
+  int sort_keys(const void* s0, int32_t* count, uint64_t* keys, int32_t* idx, cudaStream_t st) override {
     k_ad_keys<R><<<grid_for(a->n, 256), 256, 0, st>>>((const R*)s0, a->n, a->NS, D, K.res[0], K.res[1], K.res[2],
-                                                      K.inv_dx, keys, idx);
+                                                      K.inv_dx, count, keys, idx);
     AQ_CUDA_TRY(cudaGetLastError());
     return AQ_OK;
   }
   int permute(const void* in, void* out, bool gather, cudaStream_t st) override {
-    k_ad_permute<R><<<grid_for(a->n * a->NS, 256), 256, 0, st>>>((const R*)in, (R*)out, a->perm, a->n, a->NS,
-                                                                 gather ? 1 : 0);
+    const unsigned nb = grid_for(a->n, 128);
+    if (gather)
+      k_ad_permute<R, true><<<nb, 128, 0, st>>>((const R*)in, (R*)out, a->perm, a->n, a->NS);
+    else
+      k_ad_permute<R, false><<<nb, 128, 0, st>>>((const R*)in, (R*)out, a->perm, a->n, a->NS);
     AQ_CUDA_TRY(cudaGetLastError());
     return AQ_OK;
   }
 };
 
-// Sort the particles by base cell: a->perm[sorted position] = caller's index.
+// Sort the particles (ad_sort order): a->perm[sorted position] = caller's index.
 static int ad_make_perm(aq_adjoint* a, const void* d_s0, cudaStream_t st) {
-  if (!a->perm) AQ_CUDA_TRY(cudaMalloc((void**)&a->perm, sizeof(int32_t) * a->n));
-  int32_t* tmp = nullptr;  // keys in, keys out, idx in
-  AQ_CUDA_TRY(cudaMallocAsync((void**)&tmp, sizeof(int32_t) * 3 * a->n, st));
-  int32_t *kin = tmp, *kout = tmp + a->n, *iin = tmp + 2 * a->n;
-  int rc = a->impl->sort_keys(d_s0, kin, iin, st);
-  int bits = 1;
-  while (bits < 31 && (int64_t(1) << bits) < a->ncell) ++bits;
+  const int bs = a->D == 3 ? 4 : 8;
+  int64_t nblk = 1;
+  for (int d = 0; d < a->D; ++d) nblk *= (a->P.res[d] + bs - 1) / bs;
+  int bits = AD_RANK_BITS + 6 + 1;
+  while (bits < 64 && (int64_t(1) << (bits - AD_RANK_BITS - 6)) < nblk) ++bits;
   size_t tb = 0;
-  // keys are non-negative: sorted as unsigned over their low `bits` bits
-  uint32_t *uk = reinterpret_cast<uint32_t*>(kin), *uo = reinterpret_cast<uint32_t*>(kout);
+  uint64_t* nk = nullptr;
+  AQ_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, nk, nk, (int32_t*)nullptr, a->perm, (int)a->n, 0, bits, st));
+  const size_t n8 = (sizeof(uint64_t) * (size_t)a->n + 255) & ~(size_t)255;
+  char* tmp = nullptr;  // keys in, keys out, idx in, the sort's own
+  if (pool_alloc((void**)&tmp, 3 * n8 + tb, st) != cudaSuccess) return AQ_E_NOMEM;
+  uint64_t *kin = (uint64_t*)tmp, *kout = (uint64_t*)(tmp + n8);
+  int32_t* iin = (int32_t*)(tmp + 2 * n8);
+  // per-cell counts in a grid that is not in use; cleared again behind them
+  void* count = a->g[a->rot];
+  cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int32_t) * a->ncell, st);
+  int rc = e == cudaSuccess ? a->impl->sort_keys(d_s0, (int32_t*)count, kin, iin, st) : AQ_E_CUDA;
   if (rc == AQ_OK &&
-      cub::DeviceRadixSort::SortPairs(nullptr, tb, uk, uo, iin, a->perm, (int)a->n, 0, bits, st) != cudaSuccess)
+      cub::DeviceRadixSort::SortPairs(tmp + 3 * n8, tb, kin, kout, iin, a->perm, (int)a->n, 0, bits, st) != cudaSuccess)
     rc = AQ_E_CUDA;
-  void* temp = nullptr;
-  if (rc == AQ_OK && cudaMallocAsync(&temp, tb ? tb : 1, st) != cudaSuccess) rc = AQ_E_NOMEM;
-  if (rc == AQ_OK &&
-      cub::DeviceRadixSort::SortPairs(temp, tb, uk, uo, iin, a->perm, (int)a->n, 0, bits, st) != cudaSuccess)
-    rc = AQ_E_CUDA;
-  if (temp) cudaFreeAsync(temp, st);
-  cudaFreeAsync(tmp, st);
+  if (cudaMemsetAsync(count, 0, sizeof(int32_t) * a->ncell, st) != cudaSuccess && rc == AQ_OK) rc = AQ_E_CUDA;
+  pool_free(tmp, st);
+  return rc;
+}
+
+// Run substeps t0 .. t0 + k - 1 from the state in `in` (k >= 1), landing the
+// state t0 + j in buf(j); with keep_sums, g[rot] then holds the last state's
+// sums.
+template <class F>
+static int ad_chain(aq_adjoint* a, const void* in, int t0, int k, const F& buf, bool keep_sums, cudaStream_t st) {
+  int rc = a->impl->p2g(in, st);
+  for (int j = 1; j <= k && rc == AQ_OK; ++j) {
+    rc = a->impl->g2p(in, buf(j), t0 + j - 1, j < k || keep_sums, st);
+    in = buf(j);
+  }
   return rc;
 }
 
 // Run substeps t0 .. t0 + k - 1 from the state in `in` (k >= 1), landing the
 // state t0 + k in `dst` and using `tmp` as the other buffer; `in` is kept.
 static int ad_run(aq_adjoint* a, const void* in, int t0, int k, void* dst, void* tmp, cudaStream_t st) {
-  void* bufs[2] = {dst, tmp};
-  int j = (k % 2 == 1) ? 0 : 1;  // so that the last substep writes dst
-  const void* src = in;
-  for (int i = 0; i < k; ++i) {
-    void* out = bufs[j];
-    const int rc = a->impl->step(src, out, t0 + i, st);
-    if (rc) return rc;
-    src = out;
-    j ^= 1;
-  }
   a->recomputed += k;
-  return AQ_OK;
+  return ad_chain(a, in, t0, k, [=](int j) { return (k - j) % 2 == 0 ? dst : tmp; }, false, st);
 }
 
 // Bisection checkpointing (the reference's logarithmic stash,
@@ -885,11 +1188,10 @@ static int ad_run(aq_adjoint* a, const void* in, int t0, int k, void* dst, void*
 static int ad_reverse_bisect(aq_adjoint* a, int t0, int t1, const void* buf, int level, void** ab, int& cur,
                              cudaStream_t st) {
   if (t1 - t0 == 1) {
-    int rc = a->impl->step_bwd(buf, ab[cur], ab[1 - cur], t0, st);
-    if (rc) return rc;
+    int rc = a->impl->p2g(buf, st);
+    if (rc == AQ_OK) rc = a->impl->step_bwd(buf, ab[cur], ab[1 - cur], t0, t0 >= 1, st);
     cur = 1 - cur;
-    if (t0 >= 1 && (rc = a->impl->accum(ab[cur], a->dsens, st))) return rc;
-    return AQ_OK;
+    return rc;
   }
   const int m = t0 + (t1 - t0 + 1) / 2;
   void* mid = a->stash[level];
@@ -897,6 +1199,20 @@ static int ad_reverse_bisect(aq_adjoint* a, int t0, int t1, const void* buf, int
   if (rc) return rc;
   if ((rc = ad_reverse_bisect(a, m, t1, mid, level + 1, ab, cur, st))) return rc;
   return ad_reverse_bisect(a, t0, m, buf, level, ab, cur, st);
+}
+
+// `want` state buffers in v; those it has are kept
+static int ad_buffers(aq_adjoint* a, std::vector<void*>& v, int want, cudaStream_t st) {
+  if ((int)v.size() > want) {
+    cudaDeviceSynchronize();  // another stream may still use them
+    for (; (int)v.size() > want; v.pop_back()) pool_free(v.back(), st);
+  }
+  while ((int)v.size() < want) {
+    void* p = nullptr;
+    AQ_CUDA_TRY(pool_alloc(&p, a->state_bytes(), st));
+    v.push_back(p);
+  }
+  return AQ_OK;
 }
 
 template <int D, class R>
@@ -908,17 +1224,11 @@ static AdBase* make_ad(aq_adjoint* a) {
 static void free_ad(aq_adjoint* a) {
   if (!a) return;
   delete a->impl;
-  for (void* p : a->ckpt)
-    if (p) cudaFree(p);
-  for (void* p : a->seg)
-    if (p) cudaFree(p);
-  for (void* p : a->stash)
-    if (p) cudaFree(p);
-  if (a->perm) cudaFree(a->perm);
-  if (a->grid) cudaFree(a->grid);
-  if (a->gv) cudaFree(a->gv);
-  if (a->gvb) cudaFree(a->gvb);
-  if (a->dsens) cudaFree(a->dsens);
+  for (auto* v : {&a->ckpt, &a->seg, &a->stash})
+    for (void* p : *v) pool_free(p, 0);
+  pool_free(a->perm, 0);
+  for (void* p : a->g) pool_free(p, 0);
+  pool_free(a->dsens, 0);
   delete a;
 }
 
@@ -950,12 +1260,17 @@ int aq_adjoint_create(const aq_params* P, aq_adjoint** out) {
   a->rsz = P->precision ? sizeof(double) : sizeof(float);
   a->ncell = 1;
   for (int d = 0; d < D; ++d) a->ncell *= P->res[d];
-  cudaError_t e = cudaMalloc(&a->grid, a->rsz * 4 * a->ncell);
-  if (e == cudaSuccess) e = cudaMalloc(&a->gv, a->rsz * 4 * a->ncell);
-  if (e == cudaSuccess) e = cudaMalloc(&a->gvb, a->rsz * 4 * a->ncell);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&a->dsens, sizeof(double) * a->NS);
+  const size_t gbytes = a->rsz * 4 * a->ncell;
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < 3; ++k) {
+    if (e == cudaSuccess) e = pool_alloc(&a->g[k], gbytes, 0);
+    if (e == cudaSuccess) e = cudaMemsetAsync(a->g[k], 0, gbytes, 0);
+  }
+  if (e == cudaSuccess) e = pool_alloc((void**)&a->dsens, sizeof(double) * AD_SENS_COPIES * a->NS, 0);
+  if (e == cudaSuccess) e = pool_alloc((void**)&a->perm, sizeof(int32_t) * a->n, 0);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // the memory is there for every stream
   if (e != cudaSuccess) {
-    set_last_cuda_error(e, "cudaMalloc");
+    set_last_cuda_error(e, "cudaMallocFromPoolAsync");
     free_ad(a);
     return AQ_E_NOMEM;
   }
@@ -966,6 +1281,11 @@ int aq_adjoint_create(const aq_params* P, aq_adjoint** out) {
   if (!a->impl) {
     free_ad(a);
     return AQ_E_NOMEM;
+  }
+  const int rc = a->impl->setup();
+  if (rc != AQ_OK) {
+    free_ad(a);
+    return rc;
   }
   *out = a;
   return AQ_OK;
@@ -1008,87 +1328,88 @@ int aq_adjoint_forward(aq_adjoint* a, const void* d_s0, int32_t n_substeps, int3
                        void* stream) {
   if (!a || !d_s0 || !d_sT || n_substeps < 1 || every < 0) return AQ_E_ARG;
   cudaStream_t st = as_stream(stream);
-  const size_t sbytes = a->rsz * a->NS * a->n;
   const bool bisect = every == 0;
-  const int nck = bisect ? 1 : (n_substeps + every - 1) / every;
-  const int nseg = bisect ? 2 : every + 1;
-  for (void* p : a->ckpt) cudaFree(p);
-  a->ckpt.assign(nck, nullptr);
-  for (int k = 0; k < nck; ++k) AQ_CUDA_TRY(cudaMalloc(&a->ckpt[k], sbytes));
-  if ((int)a->seg.size() != nseg) {
-    for (void* p : a->seg) cudaFree(p);
-    a->seg.assign(nseg, nullptr);
-    for (int k = 0; k < nseg; ++k) AQ_CUDA_TRY(cudaMalloc(&a->seg[k], sbytes));
-  }
-  for (void* p : a->stash) cudaFree(p);
-  a->stash.clear();
+  int rc;
+  a->T = 0;  // no valid run until this one is queued
+  if ((rc = ad_buffers(a, a->ckpt, bisect ? 1 : (n_substeps + every - 1) / every, st))) return rc;
+  if ((rc = ad_buffers(a, a->seg, bisect ? 2 : every, st))) return rc;
+  if (!bisect && (rc = ad_buffers(a, a->stash, 0, st))) return rc;
+  // the state is kept in the library's order and layout; the caller's is
+  // restored for d_sT here and for the gradients in aq_adjoint_backward
+  if ((rc = ad_make_perm(a, d_s0, st))) return rc;
+  if ((rc = a->impl->permute(d_s0, a->ckpt[0], true, st))) return rc;
+  // state t goes to its checkpoint or to its place in the segment; the last
+  // segment's states stay there for the backward pass
+  const auto buf = [&](int t) -> void* {
+    if (bisect) return a->seg[t & 1];
+    if (t % every) return a->seg[t % every];
+    return t < n_substeps ? a->ckpt[t / every] : a->seg[0];
+  };
+  if ((rc = ad_chain(a, a->ckpt[0], 0, n_substeps, buf, false, st))) return rc;
   a->T = n_substeps;
   a->every = every;
-  // the state is kept sorted by base cell (a->perm); the caller's order is
-  // restored for d_sT here and for the gradients in aq_adjoint_backward
-  int rc = ad_make_perm(a, d_s0, st);
-  if (rc) return rc;
-  if ((rc = a->impl->permute(d_s0, a->seg[0], true, st))) return rc;
-  int cur = 0;
-  for (int t = 0; t < n_substeps; ++t) {
-    if ((bisect && t == 0) || (!bisect && t % every == 0))
-      AQ_CUDA_TRY(cudaMemcpyAsync(a->ckpt[bisect ? 0 : t / every], a->seg[cur], sbytes, cudaMemcpyDeviceToDevice, st));
-    rc = a->impl->step(a->seg[cur], a->seg[1 - cur], t, st);
-    if (rc) return rc;
-    cur = 1 - cur;
-  }
-  return a->impl->permute(a->seg[cur], d_sT, false, st);
+  a->seg_of = bisect ? -1 : (n_substeps - 1) / every;
+  return a->impl->permute(buf(n_substeps), d_sT, false, st);
 }
 
 int aq_adjoint_backward(aq_adjoint* a, const void* d_seed, void* d_grad_s0, double* h_sens, void* stream) {
   if (!a || !d_seed || a->T < 1) return AQ_E_ARG;
   cudaStream_t st = as_stream(stream);
-  const size_t sbytes = a->rsz * a->NS * a->n;
-  void* ab[2] = {nullptr, nullptr};
-  AQ_CUDA_TRY(cudaMallocAsync(&ab[0], sbytes, st));
-  AQ_CUDA_TRY(cudaMallocAsync(&ab[1], sbytes, st));
-  int rc0 = a->impl->permute(d_seed, ab[0], true, st);  // into the sorted order of the forward pass
-  if (rc0) return rc0;
-  AQ_CUDA_TRY(cudaMemsetAsync(a->dsens, 0, sizeof(double) * a->NS, st));
-  int cur = 0;  // ab[cur] = adjoint of state t+1
   const int T = a->T, every = a->every;
+  int rc = AQ_OK, levels = 1;
+  while ((1 << levels) < T) ++levels;
+  // one stash per level, the last one is scratch
+  if (every == 0 && (rc = ad_buffers(a, a->stash, levels + 1, st))) return rc;
+  void* ab[2] = {nullptr, nullptr};
+  for (void*& p : ab) {
+    const cudaError_t e = pool_alloc(&p, a->state_bytes(), st);
+    if (e != cudaSuccess) {
+      pool_free(ab[0], st);
+      set_last_cuda_error(e, "cudaMallocFromPoolAsync");
+      return AQ_E_CUDA;
+    }
+  }
+  rc = a->impl->permute(d_seed, ab[0], true, st);  // into the order of the forward pass
+  const size_t sens_bytes = sizeof(double) * AD_SENS_COPIES * a->NS;
+  if (rc == AQ_OK && cudaMemsetAsync(a->dsens, 0, sens_bytes, st) != cudaSuccess) rc = AQ_E_CUDA;
+  int cur = 0;  // ab[cur] = adjoint of state t+1
   a->recomputed = 0;
-  if (every == 0) {
-    int levels = 1;
-    while ((1 << levels) < T) ++levels;
-    if (a->stash.empty()) {
-      a->stash.assign(levels + 1, nullptr);  // one per level, the last one is scratch
-      for (void*& p : a->stash) AQ_CUDA_TRY(cudaMalloc(&p, sbytes));
-    }
-    const int rc = ad_reverse_bisect(a, 0, T, a->ckpt[0], 0, ab, cur, st);
-    if (rc) return rc;
-  }
-  for (int sgi = every == 0 ? -1 : (T - 1) / every; sgi >= 0; --sgi) {
+  if (every == 0 && rc == AQ_OK) rc = ad_reverse_bisect(a, 0, T, a->ckpt[0], 0, ab, cur, st);
+  for (int sgi = every == 0 ? -1 : (T - 1) / every; sgi >= 0 && rc == AQ_OK; --sgi) {
     const int t0 = sgi * every, t1 = std::min(T, t0 + every);
-    AQ_CUDA_TRY(cudaMemcpyAsync(a->seg[0], a->ckpt[sgi], sbytes, cudaMemcpyDeviceToDevice, st));
-    for (int t = t0; t < t1 - 1; ++t) {
-      const int rc = a->impl->step(a->seg[t - t0], a->seg[t - t0 + 1], t, st);
-      if (rc) return rc;
-    }
-    for (int t = t1 - 1; t >= t0; --t) {
-      const int rc = a->impl->step_bwd(a->seg[t - t0], ab[cur], ab[1 - cur], t, st);
-      if (rc) return rc;
-      cur = 1 - cur;  // ab[cur] = adjoint of state t
-      if (t >= 1) {
-        const int rc2 = a->impl->accum(ab[cur], a->dsens, st);
-        if (rc2) return rc2;
+    const auto state = [&](int t) -> void* { return t == t0 ? a->ckpt[sgi] : a->seg[t - t0]; };
+    bool sums = false;  // g[rot] holds the sums of state t1 - 1
+    if (sgi != a->seg_of) {
+      a->seg_of = -1;
+      if (t1 - 1 > t0) {
+        rc = ad_chain(a, a->ckpt[sgi], t0, t1 - 1 - t0, [&](int j) { return state(t0 + j); }, true, st);
+        sums = true;
       }
+      if (rc == AQ_OK) a->seg_of = sgi;
+    }
+    for (int t = t1 - 1; t >= t0 && rc == AQ_OK; --t) {
+      if (!sums) rc = a->impl->p2g(state(t), st);
+      sums = false;
+      if (rc == AQ_OK) rc = a->impl->step_bwd(state(t), ab[cur], ab[1 - cur], t, t >= 1, st);
+      cur = 1 - cur;  // ab[cur] = adjoint of state t
     }
   }
-  if (d_grad_s0) {
-    const int rc = a->impl->permute(ab[cur], d_grad_s0, false, st);
-    if (rc) return rc;
-  }
-  if (h_sens) AQ_CUDA_TRY(cudaMemcpyAsync(h_sens, a->dsens, sizeof(double) * a->NS, cudaMemcpyDeviceToHost, st));
-  AQ_CUDA_TRY(cudaFreeAsync(ab[0], st));
-  AQ_CUDA_TRY(cudaFreeAsync(ab[1], st));
-  AQ_CUDA_TRY(cudaStreamSynchronize(st));
-  return AQ_OK;
+  if (rc == AQ_OK && d_grad_s0) rc = a->impl->permute(ab[cur], d_grad_s0, false, st);
+  std::vector<double> part((size_t)AD_SENS_COPIES * a->NS);
+  cudaError_t e = cudaSuccess;
+  if (rc == AQ_OK && h_sens) e = cudaMemcpyAsync(part.data(), a->dsens, sens_bytes, cudaMemcpyDeviceToHost, st);
+  pool_free(ab[0], st);
+  pool_free(ab[1], st);
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = es;
+  if (e != cudaSuccess) set_last_cuda_error(e, "aq_adjoint_backward");
+  if (rc == AQ_OK && e != cudaSuccess) rc = AQ_E_CUDA;
+  if (rc == AQ_OK && h_sens)
+    for (int s = 0; s < a->NS; ++s) {
+      h_sens[s] = 0;
+      for (int k = 0; k < AD_SENS_COPIES; ++k) h_sens[s] += part[(size_t)k * a->NS + s];
+    }
+  return rc;
 }
 
 }  // extern "C"
