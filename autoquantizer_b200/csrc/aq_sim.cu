@@ -25,6 +25,7 @@
 #include "aq_common.cuh"
 #include "aq_jit.h"
 #include "aq_kernels.cuh"
+#include "aq_records.cuh"
 
 namespace aq {
 
@@ -456,40 +457,6 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_apply(const int32_t* __restrict
   }
 }
 
-// decode records into particle order
-template <class T>
-__global__ void __launch_bounds__(128) k_get_state(const __grid_constant__ aq_layout L,
-                                                   const uint64_t* __restrict__ words,
-                                                   const int32_t* __restrict__ pid, T* __restrict__ out, int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int ns = L.n_slots;
-  const GRec w{words, i, L.n_words};
-  const int64_t dst = pid[i];
-  for (int s = 0; s < ns; ++s) out[dst * ns + s] = (T)decode_slot<double>(L, s, w);
-}
-
-// Records from the simulator's grouped storage to contiguous records in
-// particle order (record i goes to out[pid[i]]).
-// base: the id of out's first record (a streamed chunk's first particle).
-__global__ void k_words_ungroup(const uint64_t* __restrict__ in, const int32_t* __restrict__ pid,
-                                uint64_t* __restrict__ out, int64_t n, int W, int64_t base = 0) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int64_t a = pid[i] - base;
-  for (int j = 0; j < W; ++j) out[a * W + j] = in[grec_word(i, j, W)];
-}
-
-// Contiguous records (record i at in[i W]) into grouped storage, same order,
-// from grouped position base on (appended records: base = records already
-// stored; the words of records below base are not touched).
-__global__ void k_words_group(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, int64_t n, int W,
-                              int64_t base = 0) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  for (int j = 0; j < W; ++j) out[grec_word(base + i, j, W)] = in[i * W + j];
-}
-
 // Grouped records back to the order of their ids (record i to grouped
 // position pid[i] - base): a streamed chunk from its binned order to
 // particle order.
@@ -498,7 +465,13 @@ __global__ void k_words_unpermute(const uint64_t* __restrict__ in, const int32_t
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int64_t a = pid[i] - base;
-  for (int j = 0; j < W; ++j) out[grec_word(a, j, W)] = in[grec_word(i, j, W)];
+  const uint64_t* p = in + (i >> 5) * 32 * (int64_t)W;
+  uint64_t* q = out + (a >> 5) * 32 * (int64_t)W;
+  const int li = (int)(i & 31), la = (int)(a & 31), W2 = W & ~1;
+  for (int k = 0; k < W2; k += 2)  // 16-byte pairs, coalesced on the reading side
+    *reinterpret_cast<ulonglong2*>(q + (k >> 1) * 64 + 2 * la) =
+        __ldg(reinterpret_cast<const ulonglong2*>(p + (k >> 1) * 64 + 2 * li));
+  if (W & 1) q[W2 * 32 + la] = __ldg(p + W2 * 32 + li);
 }
 
 __global__ void k_iota(int32_t* p, int64_t n, int64_t base = 0) {
@@ -543,47 +516,61 @@ __global__ void __launch_bounds__(256) k_loss(const __grid_constant__ aq_layout 
 }
 
 // Per-slot statistics of the decoded state (features of the sensitivity
-// surrogate).  blockIdx.y is the slot; out[slot * 5 + k] accumulates
+// surrogate); out[slot * 5 + k] accumulates
 // k = 0: sum |v|, 1: sum v, 2: sum v^2, 3: max |v| (as the bit pattern of a
 // non-negative double, which orders like the value), 4: sum |v - ref|
 // (ref: n x n_slots values in particle order, or null).
+//
+// A warp decodes 32 records at a time, a lane per record, into shared memory
+// and then takes them a lane per slot, so that the sums stay in the lane's
+// registers and the rows of ref are read in contiguous runs.  (One pass over
+// the records per slot: 1,000,003 records of 24 slots with a float ref took
+// 406 us.)
 template <class T>
-__global__ void __launch_bounds__(256) k_field_stats(const __grid_constant__ aq_layout L,
-                                                     const uint64_t* __restrict__ words,
-                                                     const int32_t* __restrict__ pid, const T* __restrict__ ref,
-                                                     int64_t n, double* __restrict__ out) {
-  __shared__ double sh[8][5];
-  const int s = blockIdx.y, ns = L.n_slots;
+__global__ void __launch_bounds__(REC_T) k_field_stats(const __grid_constant__ aq_layout L,
+                                                       const uint64_t* __restrict__ words,
+                                                       const int32_t* __restrict__ pid, const T* __restrict__ ref,
+                                                       int64_t n, double* __restrict__ out) {
+  extern __shared__ __align__(16) unsigned char rec_sm[];
+  __shared__ double sh[REC_T / 32][5][32];
+  const int ns = L.n_slots, W = L.n_words, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, np = rec_vals_stride(ns);
+  const RecSmem sm = rec_smem(rec_sm, W, ns, sizeof(double));
+  double* const sv = static_cast<double*>(sm.vals);
   double a[5] = {0, 0, 0, 0, 0};
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double v = decode_slot<double>(L, s, GRec{words, i, L.n_words});
-    const double av = fabs(v);
-    a[0] += av;
-    a[1] += v;
-    a[2] += v * v;
-    a[3] = fmax(a[3], av);
-    if (ref) a[4] += fabs(v - (double)ref[(int64_t)pid[i] * ns + s]);
-  }
-#pragma unroll
-  for (int k = 16; k; k >>= 1) {
-#pragma unroll
-    for (int j = 0; j < 5; ++j) {
-      const double o = __shfl_xor_sync(0xffffffffu, a[j], k);
-      a[j] = j == 3 ? fmax(a[j], o) : a[j] + o;
+  for (int64_t g = (int64_t)blockIdx.x * (REC_T / 32) + warp; g * 32 < n; g += (int64_t)gridDim.x * (REC_T / 32)) {
+    const int cnt = (int)min((int64_t)32, n - g * 32);
+    rec_load_group(words, g, cnt, W, sm.words);
+    sm.row[lane] = lane < cnt ? (int64_t)__ldg(pid + g * 32 + lane) * ns : 0;
+    __syncwarp();
+    if (lane < cnt)
+      for (int s = 0; s < ns; ++s) sv[lane * np + s] = decode_slot<double>(L, s, SRec{sm.words + lane});
+    __syncwarp();
+    if (lane < ns) {
+#pragma unroll 8
+      for (int r = 0; r < cnt; ++r) {
+        const double v = sv[r * np + lane];
+        const double av = fabs(v);
+        a[0] += av;
+        a[1] += v;
+        a[2] += v * v;
+        a[3] = fmax(a[3], av);
+        if (ref) a[4] += fabs(v - (double)__ldg(ref + sm.row[r] + lane));
+      }
     }
+    __syncwarp();
   }
-  const int warp = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0)
-    for (int j = 0; j < 5; ++j) sh[warp][j] = a[j];
+#pragma unroll
+  for (int j = 0; j < 5; ++j) sh[warp][j][lane] = a[j];
   __syncthreads();
-  if (threadIdx.x < 5) {
-    const int j = threadIdx.x;
-    double t = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t = j == 3 ? fmax(t, sh[w][j]) : t + sh[w][j];
+  for (int e = threadIdx.x; e < 5 * ns; e += REC_T) {
+    const int s = e / 5, j = e - 5 * s;
+    double t = sh[0][j][s];
+#pragma unroll
+    for (int w = 1; w < REC_T / 32; ++w) t = j == 3 ? fmax(t, sh[w][j][s]) : t + sh[w][j][s];
     if (j == 3)
-      atomicMax(reinterpret_cast<unsigned long long*>(out + s * 5 + 3), (unsigned long long)__double_as_longlong(t));
+      atomicMax(reinterpret_cast<unsigned long long*>(out + e), (unsigned long long)__double_as_longlong(t));
     else
-      atomicAdd(out + s * 5 + j, t);
+      atomicAdd(out + e, t);
   }
 }
 
@@ -1287,6 +1274,25 @@ static void free_sim(aq_sim* s) {
   delete s;
 }
 
+// Encode `count` particles from values into the current records at position
+// base onward, with ids base, base + 1, ... (dithering keyed on them at the
+// initial-state step).
+static int store_values(aq_sim* s, const void* values, int32_t values_f64, int64_t base, int64_t count,
+                        cudaStream_t st) {
+  const uint64_t sk = step_key(s->P.seed, -1);
+  uint64_t* w = s->words[s->cur];
+  int32_t* ids = s->pid[s->cur];
+  const size_t smem = rec_smem_cta(s->W, s->NS, values_f64 ? sizeof(double) : sizeof(float));
+  if (values_f64)
+    k_encode<double, true><<<grid_for(count, REC_T), REC_T, smem, st>>>(s->L, (const double*)values, w, count, nullptr,
+                                                                        ids, base, sk, nullptr, nullptr);
+  else
+    k_encode<float, true><<<grid_for(count, REC_T), REC_T, smem, st>>>(s->L, (const float*)values, w, count, nullptr,
+                                                                       ids, base, sk, nullptr, nullptr);
+  AQ_CUDA_TRY(cudaGetLastError());
+  return AQ_OK;
+}
+
 }  // namespace aq
 
 using namespace aq;
@@ -1528,7 +1534,7 @@ int aq_sim_stream_set_words(aq_sim* s, const uint64_t* h_words, void* stream) {
   for (int64_t c = 0; c < nc; ++c) {
     const int64_t base = c * s->chunk, m = std::min(s->chunk, s->n_total - base);
     AQ_CUDA_TRY(cudaMemcpyAsync(tmp, h_words + base * s->W, sizeof(uint64_t) * m * s->W, cudaMemcpyHostToDevice, st));
-    k_words_group<<<grid_for(m, 256), 256, 0, st>>>(tmp, s->words[s->cur], m, s->W);
+    k_words_group<<<grid_for(m, REC_T), REC_T, rec_smem_cta(s->W, 0, 0), st>>>(tmp, s->words[s->cur], m, s->W);
     AQ_CUDA_TRY(cudaGetLastError());
     AQ_CUDA_TRY(cudaMemcpyAsync(s->h_words + c * grouped_words(s->chunk, s->W), s->words[s->cur],
                                 sizeof(uint64_t) * grouped_words(m, s->W), cudaMemcpyDeviceToHost, st));
@@ -1549,7 +1555,7 @@ int aq_sim_stream_get_words(aq_sim* s, uint64_t* h_words, void* stream) {
     const int64_t base = c * s->chunk, m = std::min(s->chunk, s->n_total - base);
     int rc;
     if ((rc = s->impl->load_chunk(c, st))) return rc;  // particle order, ids base, base + 1, ...
-    k_words_ungroup<<<grid_for(m, 256), 256, 0, st>>>(s->words[s->cur], s->pid[s->cur], tmp, m, s->W, base);
+    k_words_ungroup<<<grid_for(m, REC_T), REC_T, rec_smem_cta(s->W, 0, 0), st>>>(s->words[s->cur], s->pid[s->cur], tmp, m, s->W, base);
     AQ_CUDA_TRY(cudaGetLastError());
     AQ_CUDA_TRY(cudaMemcpyAsync(h_words + base * s->W, tmp, sizeof(uint64_t) * m * s->W, cudaMemcpyDeviceToHost, st));
     s->launches += 1;
@@ -1573,19 +1579,11 @@ int aq_sim_append(aq_sim* s, const void* values, int32_t values_f64, int64_t cou
   if (count > s->cap - s->n) return AQ_E_LIMIT;
   cudaStream_t st = as_stream(stream);
   const int64_t base = s->n;
-  int32_t* ids = s->pid[s->cur] + base;
-  k_iota<<<grid_for(count, 256), 256, 0, st>>>(ids, count, base);
-  AQ_CUDA_TRY(cudaGetLastError());
-  // contiguous records into the other buffer (scratch between binnings),
-  // then grouped behind the stored ones
-  uint64_t* tmp = s->words[1 - s->cur];
-  int rc = aq_encode(&s->L, values, values_f64, tmp, count, ids, s->P.seed, -1, nullptr, stream);
-  if (rc != AQ_OK) return rc;
-  k_words_group<<<grid_for(count, 256), 256, 0, st>>>(tmp, s->words[s->cur], count, s->W, base);
-  AQ_CUDA_TRY(cudaGetLastError());
+  int rc;
+  if ((rc = store_values(s, values, values_f64, base, count, st))) return rc;
   s->n = base + count;
   s->sorted = false;
-  s->launches += 3;
+  s->launches += 1;
   return AQ_OK;
 }
 
@@ -1614,16 +1612,10 @@ int aq_sim_set_state(aq_sim* s, const void* values, int32_t values_f64, void* st
   if (!s || !values) return AQ_E_ARG;
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
-  k_iota<<<grid_for(s->n, 256), 256, 0, st>>>(s->pid[s->cur], s->n);
-  AQ_CUDA_TRY(cudaGetLastError());
-  // contiguous records into the other buffer, then grouped into the current
-  uint64_t* tmp = s->words[1 - s->cur];
-  int rc = aq_encode(&s->L, values, values_f64, tmp, s->n, nullptr, s->P.seed, -1, nullptr, stream);
-  if (rc != AQ_OK) return rc;
-  k_words_group<<<grid_for(s->n, 256), 256, 0, st>>>(tmp, s->words[s->cur], s->n, s->W);
-  AQ_CUDA_TRY(cudaGetLastError());
+  int rc;
+  if ((rc = store_values(s, values, values_f64, 0, s->n, st))) return rc;
   s->sorted = false;
-  s->launches += 3;
+  s->launches += 1;
   return AQ_OK;
 }
 
@@ -1631,12 +1623,13 @@ int aq_sim_get_state(aq_sim* s, void* values, int32_t values_f64, void* stream) 
   if (!s || !values) return AQ_E_ARG;
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
+  const size_t smem = rec_smem_cta(s->W, s->NS, values_f64 ? sizeof(double) : sizeof(float));
   if (values_f64)
-    k_get_state<double><<<grid_for(s->n, 128), 128, 0, st>>>(s->L, s->words[s->cur], s->pid[s->cur], (double*)values,
-                                                             s->n);
+    k_decode<double, true><<<grid_for(s->n, REC_T), REC_T, smem, st>>>(s->L, s->words[s->cur], s->pid[s->cur],
+                                                                       (double*)values, s->n);
   else
-    k_get_state<float><<<grid_for(s->n, 128), 128, 0, st>>>(s->L, s->words[s->cur], s->pid[s->cur], (float*)values,
-                                                            s->n);
+    k_decode<float, true><<<grid_for(s->n, REC_T), REC_T, smem, st>>>(s->L, s->words[s->cur], s->pid[s->cur],
+                                                                      (float*)values, s->n);
   AQ_CUDA_TRY(cudaGetLastError());
   s->launches += 1;
   return AQ_OK;
@@ -1709,13 +1702,13 @@ int aq_sim_field_stats(aq_sim* s, const void* ref, int32_t ref_f64, double* h_ou
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
   AQ_CUDA_TRY(cudaMemsetAsync(s->dstats, 0, sizeof(double) * 5 * AQ_MAX_SLOTS, st));
-  const unsigned nb = (unsigned)std::min<int64_t>(grid_for(s->n, 256), (int64_t)num_sms() * 4);
-  const dim3 grid(nb > 0 ? nb : 1, s->NS);
+  const unsigned grid = (unsigned)std::min<int64_t>(grid_for(s->n, REC_T), (int64_t)num_sms() * 12);
+  const size_t smem = rec_smem_cta(s->W, s->NS, sizeof(double));
   if (ref_f64)
-    k_field_stats<double><<<grid, 256, 0, st>>>(s->L, s->words[s->cur], s->pid[s->cur], (const double*)ref, s->n,
+    k_field_stats<double><<<grid, REC_T, smem, st>>>(s->L, s->words[s->cur], s->pid[s->cur], (const double*)ref, s->n,
                                                 s->dstats);
   else
-    k_field_stats<float><<<grid, 256, 0, st>>>(s->L, s->words[s->cur], s->pid[s->cur], (const float*)ref, s->n,
+    k_field_stats<float><<<grid, REC_T, smem, st>>>(s->L, s->words[s->cur], s->pid[s->cur], (const float*)ref, s->n,
                                                s->dstats);
   AQ_CUDA_TRY(cudaGetLastError());
   s->launches += 1;
@@ -1729,7 +1722,7 @@ int aq_sim_set_words(aq_sim* s, const uint64_t* words, void* stream) {
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
   k_iota<<<grid_for(s->n, 256), 256, 0, st>>>(s->pid[s->cur], s->n);
-  k_words_group<<<grid_for(s->n, 256), 256, 0, st>>>(words, s->words[s->cur], s->n, s->W);
+  k_words_group<<<grid_for(s->n, REC_T), REC_T, rec_smem_cta(s->W, 0, 0), st>>>(words, s->words[s->cur], s->n, s->W);
   AQ_CUDA_TRY(cudaGetLastError());
   s->sorted = false;
   s->launches += 2;
@@ -1740,7 +1733,7 @@ int aq_sim_get_words(aq_sim* s, uint64_t* words, void* stream) {
   if (!s || !words) return AQ_E_ARG;
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
-  k_words_ungroup<<<grid_for(s->n, 256), 256, 0, st>>>(s->words[s->cur], s->pid[s->cur], words, s->n, s->W);
+  k_words_ungroup<<<grid_for(s->n, REC_T), REC_T, rec_smem_cta(s->W, 0, 0), st>>>(s->words[s->cur], s->pid[s->cur], words, s->n, s->W, 0);
   AQ_CUDA_TRY(cudaGetLastError());
   s->launches += 1;
   return AQ_OK;
