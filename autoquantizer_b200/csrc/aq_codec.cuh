@@ -318,14 +318,13 @@ __device__ __forceinline__ void decode_record(const aq_layout& L, const WP& w, R
   }
 }
 
-// Decode one slot (runtime index).
+// Decode one slot.
 template <class R, class WP>
-__device__ __forceinline__ R decode_slot(const aq_layout& L, int s, const WP& w) {
-  const aq_slot& S = L.slot[s];
+__device__ __forceinline__ R decode_of(const aq_slot& S, bool f64, const WP& w) {
   const uint64_t code = get_bits(w, S.bit_offset, S.bits);
   switch (S.kind) {
     case AQ_FIXED:
-      return dequant_fixed<R>(S, L.compute_f64 != 0, (uint32_t)code);
+      return dequant_fixed<R>(S, f64, (uint32_t)code);
     case AQ_INT:
       return S.is_signed ? (R)sext32((uint32_t)code, S.bits) : (R)(uint32_t)code;
     case AQ_FLOAT_EXP:
@@ -337,6 +336,12 @@ __device__ __forceinline__ R decode_slot(const aq_layout& L, int s, const WP& w)
     default:
       return (R)__longlong_as_double((long long)code);
   }
+}
+
+// Decode one slot (runtime index).
+template <class R, class WP>
+__device__ __forceinline__ R decode_slot(const aq_layout& L, int s, const WP& w) {
+  return decode_of<R>(L.slot[s], L.compute_f64 != 0, w);
 }
 
 // Encode vals into record `out` (sequential word writes) and replace each

@@ -8,7 +8,7 @@
 
 #include "aq_codec.cuh"
 #include "aq_common.cuh"
-#include "aq_records.cuh"
+#include "aq_records.h"
 
 namespace aq {
 
@@ -257,13 +257,7 @@ int aq_encode(const aq_layout* L, const void* values, int32_t values_f64, uint64
   const uint64_t sk = step_key(seed, step);
   const float* uf = (uniforms && !L->compute_f64) ? (const float*)uniforms : nullptr;
   const double* ud = (uniforms && L->compute_f64) ? (const double*)uniforms : nullptr;
-  if (values_f64)
-    k_encode<double, false><<<grid_for(n, REC_T), REC_T, rec_smem_cta(L->n_words, L->n_slots, sizeof(double)),
-                              as_stream(stream)>>>(*L, (const double*)values, words, n, pid, nullptr, 0, sk, uf, ud);
-  else
-    k_encode<float, false><<<grid_for(n, REC_T), REC_T, rec_smem_cta(L->n_words, L->n_slots, sizeof(float)),
-                             as_stream(stream)>>>(*L, (const float*)values, words, n, pid, nullptr, 0, sk, uf, ud);
-  AQ_CUDA_TRY(cudaGetLastError());
+  AQ_CUDA_TRY(rec_encode_rows(*L, values, values_f64 != 0, words, n, pid, sk, uf, ud, as_stream(stream)));
   return AQ_OK;
 }
 
@@ -272,13 +266,7 @@ int aq_decode(const aq_layout* L, const uint64_t* words, void* values, int32_t v
   if (!L || n < 0 || (n > 0 && (!values || !words))) return AQ_E_ARG;
   if (L->n_slots < 1 || L->n_slots > AQ_MAX_SLOTS) return AQ_E_ARG;
   if (n == 0) return AQ_OK;
-  if (values_f64)
-    k_decode<double, false><<<grid_for(n, REC_T), REC_T, rec_smem_cta(L->n_words, L->n_slots, sizeof(double)),
-                              as_stream(stream)>>>(*L, words, nullptr, (double*)values, n);
-  else
-    k_decode<float, false><<<grid_for(n, REC_T), REC_T, rec_smem_cta(L->n_words, L->n_slots, sizeof(float)),
-                             as_stream(stream)>>>(*L, words, nullptr, (float*)values, n);
-  AQ_CUDA_TRY(cudaGetLastError());
+  AQ_CUDA_TRY(rec_decode_rows(*L, words, values, values_f64 != 0, n, as_stream(stream)));
   return AQ_OK;
 }
 

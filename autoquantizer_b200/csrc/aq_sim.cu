@@ -25,7 +25,7 @@
 #include "aq_common.cuh"
 #include "aq_jit.h"
 #include "aq_kernels.cuh"
-#include "aq_records.cuh"
+#include "aq_records.h"
 
 namespace aq {
 
@@ -512,65 +512,6 @@ __global__ void __launch_bounds__(256) k_loss(const __grid_constant__ aq_layout 
     double s = 0;
     for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += sh[k];
     atomicAdd(out, s);
-  }
-}
-
-// Per-slot statistics of the decoded state (features of the sensitivity
-// surrogate); out[slot * 5 + k] accumulates
-// k = 0: sum |v|, 1: sum v, 2: sum v^2, 3: max |v| (as the bit pattern of a
-// non-negative double, which orders like the value), 4: sum |v - ref|
-// (ref: n x n_slots values in particle order, or null).
-//
-// A warp decodes 32 records at a time, a lane per record, into shared memory
-// and then takes them a lane per slot, so that the sums stay in the lane's
-// registers and the rows of ref are read in contiguous runs.  (One pass over
-// the records per slot: 1,000,003 records of 24 slots with a float ref took
-// 406 us.)
-template <class T>
-__global__ void __launch_bounds__(REC_T) k_field_stats(const __grid_constant__ aq_layout L,
-                                                       const uint64_t* __restrict__ words,
-                                                       const int32_t* __restrict__ pid, const T* __restrict__ ref,
-                                                       int64_t n, double* __restrict__ out) {
-  extern __shared__ __align__(16) unsigned char rec_sm[];
-  __shared__ double sh[REC_T / 32][5][32];
-  const int ns = L.n_slots, W = L.n_words, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, np = rec_vals_stride(ns);
-  const RecSmem sm = rec_smem(rec_sm, W, ns, sizeof(double));
-  double* const sv = static_cast<double*>(sm.vals);
-  double a[5] = {0, 0, 0, 0, 0};
-  for (int64_t g = (int64_t)blockIdx.x * (REC_T / 32) + warp; g * 32 < n; g += (int64_t)gridDim.x * (REC_T / 32)) {
-    const int cnt = (int)min((int64_t)32, n - g * 32);
-    rec_load_group(words, g, cnt, W, sm.words);
-    sm.row[lane] = lane < cnt ? (int64_t)__ldg(pid + g * 32 + lane) * ns : 0;
-    __syncwarp();
-    if (lane < cnt)
-      for (int s = 0; s < ns; ++s) sv[lane * np + s] = decode_slot<double>(L, s, SRec{sm.words + lane});
-    __syncwarp();
-    if (lane < ns) {
-#pragma unroll 8
-      for (int r = 0; r < cnt; ++r) {
-        const double v = sv[r * np + lane];
-        const double av = fabs(v);
-        a[0] += av;
-        a[1] += v;
-        a[2] += v * v;
-        a[3] = fmax(a[3], av);
-        if (ref) a[4] += fabs(v - (double)__ldg(ref + sm.row[r] + lane));
-      }
-    }
-    __syncwarp();
-  }
-#pragma unroll
-  for (int j = 0; j < 5; ++j) sh[warp][j][lane] = a[j];
-  __syncthreads();
-  for (int e = threadIdx.x; e < 5 * ns; e += REC_T) {
-    const int s = e / 5, j = e - 5 * s;
-    double t = sh[0][j][s];
-#pragma unroll
-    for (int w = 1; w < REC_T / 32; ++w) t = j == 3 ? fmax(t, sh[w][j][s]) : t + sh[w][j][s];
-    if (j == 3)
-      atomicMax(reinterpret_cast<unsigned long long*>(out + e), (unsigned long long)__double_as_longlong(t));
-    else
-      atomicAdd(out + e, t);
   }
 }
 
@@ -1279,17 +1220,8 @@ static void free_sim(aq_sim* s) {
 // initial-state step).
 static int store_values(aq_sim* s, const void* values, int32_t values_f64, int64_t base, int64_t count,
                         cudaStream_t st) {
-  const uint64_t sk = step_key(s->P.seed, -1);
-  uint64_t* w = s->words[s->cur];
-  int32_t* ids = s->pid[s->cur];
-  const size_t smem = rec_smem_cta(s->W, s->NS, values_f64 ? sizeof(double) : sizeof(float));
-  if (values_f64)
-    k_encode<double, true><<<grid_for(count, REC_T), REC_T, smem, st>>>(s->L, (const double*)values, w, count, nullptr,
-                                                                        ids, base, sk, nullptr, nullptr);
-  else
-    k_encode<float, true><<<grid_for(count, REC_T), REC_T, smem, st>>>(s->L, (const float*)values, w, count, nullptr,
-                                                                       ids, base, sk, nullptr, nullptr);
-  AQ_CUDA_TRY(cudaGetLastError());
+  AQ_CUDA_TRY(rec_store(s->L, values, values_f64 != 0, s->words[s->cur], s->pid[s->cur], base, count,
+                        step_key(s->P.seed, -1), st));
   return AQ_OK;
 }
 
@@ -1534,8 +1466,7 @@ int aq_sim_stream_set_words(aq_sim* s, const uint64_t* h_words, void* stream) {
   for (int64_t c = 0; c < nc; ++c) {
     const int64_t base = c * s->chunk, m = std::min(s->chunk, s->n_total - base);
     AQ_CUDA_TRY(cudaMemcpyAsync(tmp, h_words + base * s->W, sizeof(uint64_t) * m * s->W, cudaMemcpyHostToDevice, st));
-    k_words_group<<<grid_for(m, REC_T), REC_T, rec_smem_cta(s->W, 0, 0), st>>>(tmp, s->words[s->cur], m, s->W);
-    AQ_CUDA_TRY(cudaGetLastError());
+    AQ_CUDA_TRY(rec_group(tmp, s->words[s->cur], m, s->W, st));
     AQ_CUDA_TRY(cudaMemcpyAsync(s->h_words + c * grouped_words(s->chunk, s->W), s->words[s->cur],
                                 sizeof(uint64_t) * grouped_words(m, s->W), cudaMemcpyDeviceToHost, st));
     s->launches += 1;
@@ -1555,8 +1486,7 @@ int aq_sim_stream_get_words(aq_sim* s, uint64_t* h_words, void* stream) {
     const int64_t base = c * s->chunk, m = std::min(s->chunk, s->n_total - base);
     int rc;
     if ((rc = s->impl->load_chunk(c, st))) return rc;  // particle order, ids base, base + 1, ...
-    k_words_ungroup<<<grid_for(m, REC_T), REC_T, rec_smem_cta(s->W, 0, 0), st>>>(s->words[s->cur], s->pid[s->cur], tmp, m, s->W, base);
-    AQ_CUDA_TRY(cudaGetLastError());
+    AQ_CUDA_TRY(rec_ungroup(s->words[s->cur], s->pid[s->cur], tmp, m, s->W, base, st));
     AQ_CUDA_TRY(cudaMemcpyAsync(h_words + base * s->W, tmp, sizeof(uint64_t) * m * s->W, cudaMemcpyDeviceToHost, st));
     s->launches += 1;
   }
@@ -1623,14 +1553,7 @@ int aq_sim_get_state(aq_sim* s, void* values, int32_t values_f64, void* stream) 
   if (!s || !values) return AQ_E_ARG;
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
-  const size_t smem = rec_smem_cta(s->W, s->NS, values_f64 ? sizeof(double) : sizeof(float));
-  if (values_f64)
-    k_decode<double, true><<<grid_for(s->n, REC_T), REC_T, smem, st>>>(s->L, s->words[s->cur], s->pid[s->cur],
-                                                                       (double*)values, s->n);
-  else
-    k_decode<float, true><<<grid_for(s->n, REC_T), REC_T, smem, st>>>(s->L, s->words[s->cur], s->pid[s->cur],
-                                                                      (float*)values, s->n);
-  AQ_CUDA_TRY(cudaGetLastError());
+  AQ_CUDA_TRY(rec_fetch(s->L, s->words[s->cur], s->pid[s->cur], values, values_f64 != 0, s->n, st));
   s->launches += 1;
   return AQ_OK;
 }
@@ -1702,15 +1625,7 @@ int aq_sim_field_stats(aq_sim* s, const void* ref, int32_t ref_f64, double* h_ou
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
   AQ_CUDA_TRY(cudaMemsetAsync(s->dstats, 0, sizeof(double) * 5 * AQ_MAX_SLOTS, st));
-  const unsigned grid = (unsigned)std::min<int64_t>(grid_for(s->n, REC_T), (int64_t)num_sms() * 12);
-  const size_t smem = rec_smem_cta(s->W, s->NS, sizeof(double));
-  if (ref_f64)
-    k_field_stats<double><<<grid, REC_T, smem, st>>>(s->L, s->words[s->cur], s->pid[s->cur], (const double*)ref, s->n,
-                                                s->dstats);
-  else
-    k_field_stats<float><<<grid, REC_T, smem, st>>>(s->L, s->words[s->cur], s->pid[s->cur], (const float*)ref, s->n,
-                                               s->dstats);
-  AQ_CUDA_TRY(cudaGetLastError());
+  AQ_CUDA_TRY(rec_stats(s->L, s->words[s->cur], s->pid[s->cur], ref, ref_f64 != 0, s->n, s->dstats, st));
   s->launches += 1;
   AQ_CUDA_TRY(cudaMemcpyAsync(h_out, s->dstats, sizeof(double) * 5 * s->NS, cudaMemcpyDeviceToHost, st));
   AQ_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1722,8 +1637,8 @@ int aq_sim_set_words(aq_sim* s, const uint64_t* words, void* stream) {
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
   k_iota<<<grid_for(s->n, 256), 256, 0, st>>>(s->pid[s->cur], s->n);
-  k_words_group<<<grid_for(s->n, REC_T), REC_T, rec_smem_cta(s->W, 0, 0), st>>>(words, s->words[s->cur], s->n, s->W);
   AQ_CUDA_TRY(cudaGetLastError());
+  AQ_CUDA_TRY(rec_group(words, s->words[s->cur], s->n, s->W, st));
   s->sorted = false;
   s->launches += 2;
   return AQ_OK;
@@ -1733,8 +1648,7 @@ int aq_sim_get_words(aq_sim* s, uint64_t* words, void* stream) {
   if (!s || !words) return AQ_E_ARG;
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
-  k_words_ungroup<<<grid_for(s->n, REC_T), REC_T, rec_smem_cta(s->W, 0, 0), st>>>(s->words[s->cur], s->pid[s->cur], words, s->n, s->W, 0);
-  AQ_CUDA_TRY(cudaGetLastError());
+  AQ_CUDA_TRY(rec_ungroup(s->words[s->cur], s->pid[s->cur], words, s->n, s->W, 0, st));
   s->launches += 1;
   return AQ_OK;
 }
