@@ -15,6 +15,8 @@
 #include <cuda_bf16.h>
 #include <math.h>
 
+#include <algorithm>
+
 #include "aq_common.cuh"
 
 namespace aq {
@@ -248,6 +250,303 @@ static MlpOffsets offsets(int in, int h, int out) {
   return o;
 }
 
+// ------------------------------------------------------ whole-network kernels
+//
+// For the surrogate's own sizes a layer's GEMM is a few hundred nanoseconds of
+// work behind several microseconds of launch, staging and waiting: forward at
+// batch 1 took 28 us of kernels in three launches, forward and backward at
+// batch 128 104 us in eleven.  These take the network in one launch forward
+// and two backward:
+//   k_mlp_forward   a CTA per 16 rows of the batch: the rows' activations stay
+//                   in shared memory from layer to layer
+//   k_mlp_dz        the same for the hidden layers' output gradients
+//   k_mlp_dw        all weight and bias gradients, a warp per 16 x 32 tile
+// Every product is the same m16n8k16 as k_gemm_bf16's, in the same order of k,
+// so the results are the same bits.  A weight fragment is used once per CTA,
+// so it goes from L2 to registers directly.
+// Rule (mlp_fused): in and h multiples of 64 (whole chunks of four k-steps)
+// and at most 512 (16 rows of two layers fit 48 KB), out at most 128, weights
+// aligned for paired loads.  k_gemm_bf16 keeps the other sizes.  64-128-128-12,
+// forward / gradient, before -> now: batch 1 31 / 102 -> 17 / 41 us (the calls'
+// own host time), 128 37 / 121 -> 17 / 38, 2048 37 / 535 -> 17 / 49, 32768
+// 117 / 7456 -> 58 / 229.
+constexpr int FT = 256;  // threads: eight warps, each every eighth tile of 8 columns
+constexpr int FROWS = 16;
+constexpr int FMAX = 512;
+
+// a[row][k] in shared memory, padded so that fragment loads are conflict-free
+__device__ __forceinline__ int f_ld(int K) { return K + 8; }
+
+__device__ __forceinline__ void f_afrag(uint32_t (&a)[4], const __nv_bfloat16* sa, int ld, int kk) {
+  const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+  a[0] = *reinterpret_cast<const uint32_t*>(sa + g * ld + kk + 2 * t);
+  a[1] = *reinterpret_cast<const uint32_t*>(sa + (g + 8) * ld + kk + 2 * t);
+  a[2] = *reinterpret_cast<const uint32_t*>(sa + g * ld + kk + 2 * t + 8);
+  a[3] = *reinterpret_cast<const uint32_t*>(sa + (g + 8) * ld + kk + 2 * t + 8);
+}
+
+// acc[16 x 8] = A (16 x K, shared) times the columns n of B over k in whole
+// chunks of 64; bfrag(k, b): the fragment's two registers.
+template <class F>
+__device__ __forceinline__ void f_tile(float (&acc)[4], const __nv_bfloat16* sa, int ld, int K, const F& bfrag) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) acc[e] = 0.f;
+  for (int k0 = 0; k0 < K; k0 += GK) {
+    uint32_t b[4][2];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) bfrag(k0 + 16 * q, b[q]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      uint32_t a[4];
+      f_afrag(a, sa, ld, k0 + 16 * q);
+      mma_bf16(acc, a[0], a[1], a[2], a[3], b[q][0], b[q][1]);
+    }
+  }
+}
+
+// Fragment of B(n, k) = W[n][k] (rows of k): two aligned pairs.
+__device__ __forceinline__ void f_brow(uint32_t (&b)[2], const __nv_bfloat16* __restrict__ W, int K, int n, int N, int k) {
+  const int t = threadIdx.x & 3;
+  const uint32_t* p = reinterpret_cast<const uint32_t*>(W + (int64_t)n * K + k + 2 * t);
+  b[0] = n < N ? __ldg(p) : 0u;
+  b[1] = n < N ? __ldg(p + 4) : 0u;
+}
+
+// Fragment of B(n, k) = W[k][n] (rows of n, K rows).
+__device__ __forceinline__ void f_bcol(uint32_t (&b)[2], const __nv_bfloat16* __restrict__ W, int N, int n, int K, int k) {
+  const int t = threadIdx.x & 3;
+  const unsigned short* p = reinterpret_cast<const unsigned short*>(W) + n;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int kk = k + 2 * t + 8 * q;
+    const uint32_t lo = kk < K ? __ldg(p + (int64_t)kk * N) : 0u, hi = kk + 1 < K ? __ldg(p + (int64_t)(kk + 1) * N) : 0u;
+    b[q] = lo | hi << 16;
+  }
+}
+
+// rows [r0, r0 + 16) of an fp32 matrix (B x K) -> bf16 in shared memory,
+// zeros outside and up to Kp columns
+__device__ __forceinline__ void f_rows(__nv_bfloat16* sa, int ld, const float* __restrict__ x, int r0, int B, int K, int Kp) {
+  for (int i = threadIdx.x; i < FROWS * Kp / 2; i += FT) {
+    const int r = i / (Kp / 2), k = 2 * (i - r * (Kp / 2));
+    float v0 = 0.f, v1 = 0.f;
+    if (r0 + r < B) {
+      const float* p = x + (int64_t)(r0 + r) * K + k;
+      if (k < K) v0 = __ldg(p);
+      if (k + 1 < K) v1 = __ldg(p + 1);
+    }
+    *reinterpret_cast<__nv_bfloat162*>(sa + r * ld + k) = __floats2bfloat162_rn(v0, v1);
+  }
+}
+
+// A hidden layer: z = A W^T + b and gelu(z), saved when asked for, and gelu(z)
+// as bf16 for the next layer.
+__device__ __forceinline__ void f_hidden(const __nv_bfloat16* sa, int K, const __nv_bfloat16* __restrict__ W,
+                                         const float* __restrict__ bias, int N, int r0, int B, float* __restrict__ z,
+                                         float* __restrict__ act, __nv_bfloat16* so) {
+  const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3, ldo = f_ld(N);
+  for (int nt = threadIdx.x >> 5; nt < N / 8; nt += FT / 32) {
+    float acc[4];
+    f_tile(acc, sa, f_ld(K), K, [&](int k, uint32_t (&b)[2]) { f_brow(b, W, K, nt * 8 + g, N, k); });
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = g + 8 * h, n = nt * 8 + 2 * t;
+      const float z0 = acc[2 * h] + bias[n], z1 = acc[2 * h + 1] + bias[n + 1];
+      const float a0 = gelu(z0), a1 = gelu(z1);
+      if (z && r0 + r < B) {
+        const int64_t o = (int64_t)(r0 + r) * N + n;
+        z[o] = z0;
+        z[o + 1] = z1;
+        act[o] = a0;
+        act[o + 1] = a1;
+      }
+      *reinterpret_cast<__nv_bfloat162*>(so + r * ldo + n) = __floats2bfloat162_rn(a0, a1);
+    }
+  }
+  __syncthreads();
+}
+
+struct MlpPtrs {
+  const __nv_bfloat16 *w1, *w2, *w3;
+  const float *b1, *b2, *b3;
+};
+
+__global__ void __launch_bounds__(FT) k_mlp_forward(int in, int h, int out, const MlpPtrs P, const float* __restrict__ x,
+                                                    int B, float* __restrict__ y, float* __restrict__ z1,
+                                                    float* __restrict__ a1, float* __restrict__ z2,
+                                                    float* __restrict__ a2) {
+  extern __shared__ __align__(16) __nv_bfloat16 f_sm[];
+  __nv_bfloat16* s0 = f_sm;  // x, then a2
+  __nv_bfloat16* s1 = f_sm + FROWS * f_ld(in > h ? in : h);
+  const int r0 = blockIdx.x * FROWS;
+  f_rows(s0, f_ld(in), x, r0, B, in, in);
+  __syncthreads();
+  f_hidden(s0, in, P.w1, P.b1, h, r0, B, z1, a1, s1);
+  f_hidden(s1, h, P.w2, P.b2, h, r0, B, z2, a2, s0);
+  const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+  for (int nt = threadIdx.x >> 5; nt * 8 < out; nt += FT / 32) {
+    float acc[4];
+    f_tile(acc, s0, f_ld(h), h, [&](int k, uint32_t (&b)[2]) { f_brow(b, P.w3, h, nt * 8 + g, out, k); });
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int r = r0 + g + (e >= 2 ? 8 : 0), n = nt * 8 + 2 * t + (e & 1);
+      if (r < B && n < out) y[(int64_t)r * out + n] = acc[e] + P.b3[n];
+    }
+  }
+}
+
+// dz = (A W) gelu'(z): one hidden layer back; A (16 x K, shared), W [K][N]
+__device__ __forceinline__ void f_back(const __nv_bfloat16* sa, int ld, int K, int Kp, const __nv_bfloat16* __restrict__ W,
+                                       int N, int r0, int B, const float* __restrict__ z, float* __restrict__ dz,
+                                       __nv_bfloat16* so) {
+  const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3, ldo = f_ld(N);
+  for (int nt = threadIdx.x >> 5; nt < N / 8; nt += FT / 32) {
+    float acc[4];
+    f_tile(acc, sa, ld, Kp, [&](int k, uint32_t (&b)[2]) { f_bcol(b, W, N, nt * 8 + g, K, k); });
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = g + 8 * h, n = nt * 8 + 2 * t;
+      float v[2] = {0.f, 0.f};
+      if (r0 + r < B) {
+        const int64_t o = (int64_t)(r0 + r) * N + n;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          v[e] = acc[2 * h + e] * gelu_grad(z[o + e]);
+          dz[o + e] = v[e];
+        }
+      }
+      if (so) *reinterpret_cast<__nv_bfloat162*>(so + r * ldo + n) = __floats2bfloat162_rn(v[0], v[1]);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(FT) k_mlp_dz(int h, int out, const MlpPtrs P, const float* __restrict__ dy, int B,
+                                               const float* __restrict__ z1, const float* __restrict__ z2,
+                                               float* __restrict__ dz1, float* __restrict__ dz2) {
+  extern __shared__ __align__(16) __nv_bfloat16 f_sm[];
+  const int op = (out + GK - 1) / GK * GK, r0 = blockIdx.x * FROWS;
+  __nv_bfloat16* s0 = f_sm;
+  __nv_bfloat16* s1 = f_sm + FROWS * f_ld(op);
+  f_rows(s0, f_ld(op), dy, r0, B, out, op);
+  __syncthreads();
+  f_back(s0, f_ld(op), out, op, P.w3, h, r0, B, z2, dz2, s1);
+  __syncthreads();
+  f_back(s1, f_ld(h), h, h, P.w2, h, r0, B, z1, dz1, nullptr);
+}
+
+// One weight gradient dW[m][n] = sum_b dZ[b][m] X[b][n] (M x N) and its bias
+// gradient, the column sums of dZ.
+struct DwJob {
+  const float* dz;
+  const float* x;
+  float* dw;
+  float* db;
+  int M, N, first;  // first: this job's first warp
+};
+struct DwJobs {
+  DwJob j[3];
+};
+
+// tiles of 16 x 32 of a job, then its columns eight at a time
+__host__ __device__ __forceinline__ int dw_tiles(int M, int N) { return ((M + 15) / 16) * ((N + 31) / 32); }
+__host__ __device__ __forceinline__ int dw_warps(int M, int N) { return dw_tiles(M, N) + (M + 7) / 8; }
+
+constexpr int DWT = 64;  // threads: two warps, so that the tiles spread over the SMs
+
+// Rows [y seg, (y + 1) seg) of the batch, y = blockIdx.y, into the y-th of
+// gridDim.y gradients `stride` floats apart.
+__global__ void __launch_bounds__(DWT) k_mlp_dw(const DwJobs J, int rows, int seg, int64_t stride, int warps) {
+  const int wid = (int)((blockIdx.x * DWT + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (wid >= warps) return;
+  DwJob j = J.j[wid >= J.j[2].first ? 2 : wid >= J.j[1].first ? 1 : 0];
+  const int b0 = blockIdx.y * seg, B = min(seg, rows - b0);
+  j.dz += (int64_t)b0 * j.M;
+  j.x += (int64_t)b0 * j.N;
+  j.dw += blockIdx.y * stride;
+  j.db += blockIdx.y * stride;
+  const int w = wid - j.first, M = j.M, N = j.N, nt = (N + 31) / 32, tiles = dw_tiles(M, N);
+  if (w >= tiles) {
+    // eight columns, four lanes each over every fourth row
+    const int m = (w - tiles) * 8 + (lane & 7), q = lane >> 3;
+    float acc = 0.f;
+    if (m < M)
+      for (int b = q; b < B; b += 32) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = b + 4 * i < B ? __ldg(j.dz + (int64_t)(b + 4 * i) * M + m) : 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc += v[i];
+      }
+    acc += __shfl_xor_sync(0xffffffffu, acc, 8);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+    if (m < M && q == 0) j.db[m] = acc;
+    return;
+  }
+  const int m0 = (w / nt) * 16, n0 = (w % nt) * 32, g = lane >> 2, t = lane & 3;
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
+  // pair (k, k + 1) of column c of a B x C matrix as bf16
+  const auto pair = [&](const float* __restrict__ p, int C, int c, int k) {
+    const float lo = c < C && k < B ? __ldg(p + (int64_t)k * C + c) : 0.f;
+    const float hi = c < C && k + 1 < B ? __ldg(p + (int64_t)(k + 1) * C + c) : 0.f;
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  };
+  for (int k0 = 0; k0 < B; k0 += 32) {
+    uint32_t a[2][4], b[2][4][2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int k = k0 + 16 * s + 2 * t;
+      a[s][0] = pair(j.dz, M, m0 + g, k);
+      a[s][1] = pair(j.dz, M, m0 + g + 8, k);
+      a[s][2] = pair(j.dz, M, m0 + g, k + 8);
+      a[s][3] = pair(j.dz, M, m0 + g + 8, k + 8);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        b[s][i][0] = pair(j.x, N, n0 + 8 * i + g, k);
+        b[s][i][1] = pair(j.x, N, n0 + 8 * i + g, k + 8);
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) mma_bf16(acc[i], a[s][0], a[s][1], a[s][2], a[s][3], b[s][i][0], b[s][i][1]);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int m = m0 + g + (e >= 2 ? 8 : 0), n = n0 + 8 * i + 2 * t + (e & 1);
+      if (m < M && n < N) j.dw[(int64_t)m * N + n] = acc[i][e];
+    }
+}
+
+// grad = sum over the segments' gradients, in their order
+__global__ void k_mlp_dw_sum(const float* __restrict__ part, int segs, int64_t n, float* __restrict__ grad) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float v = 0.f;
+#pragma unroll 8
+  for (int s = 0; s < segs; ++s) v += __ldg(part + s * n + i);
+  grad[i] = v;
+}
+
+// Batch rows a warp of k_mlp_dw sums over, at least: a longer batch is split
+// into up to DW_SEGS segments (batch 2048: 133 us in one segment).
+constexpr int DW_ROWS = 256, DW_SEGS = 32;
+
+static bool mlp_fused(int in, int h, int out, const void* weights, const MlpOffsets& o) {
+  return in % GK == 0 && h % GK == 0 && in <= FMAX && h <= FMAX && out <= 128 && (uintptr_t)weights % 4 == 0 &&
+         o.w2 % 2 == 0 && o.w3 % 2 == 0;
+}
+
+static MlpPtrs mlp_ptrs(const __nv_bfloat16* wb, const float* p, const MlpOffsets& o) {
+  return MlpPtrs{wb + o.w1, wb + o.w2, wb + o.w3, p ? p + o.b1 : nullptr, p ? p + o.b2 : nullptr, p ? p + o.b3 : nullptr};
+}
+
 }  // namespace aq
 
 using namespace aq;
@@ -280,7 +579,15 @@ int aq_mlp_forward(int32_t in, int32_t h, int32_t out, const float* d_params, co
     a1 = z1 + (size_t)B * h;
     z2 = a1 + (size_t)B * h;
     a2 = z2 + (size_t)B * h;
-  } else {
+  }
+  if (mlp_fused(in, h, out, wb, o)) {
+    const int smem = FROWS * (std::max(in, h) + 8 + h + 8) * (int)sizeof(__nv_bfloat16);
+    k_mlp_forward<<<(B + FROWS - 1) / FROWS, FT, smem, st>>>(in, h, out, mlp_ptrs(wb, d_params, o), d_x, B, d_y, z1, a1,
+                                                             z2, a2);
+    AQ_CUDA_TRY(cudaGetLastError());
+    return AQ_OK;
+  }
+  if (!d_act) {
     AQ_CUDA_TRY(pool_alloc((void**)&tmp, sizeof(float) * 2 * (size_t)B * h, st));
     a1 = tmp;
     a2 = tmp + (size_t)B * h;
@@ -310,6 +617,34 @@ int aq_mlp_backward(int32_t in, int32_t h, int32_t out, const uint16_t* d_params
   AQ_CUDA_TRY(pool_alloc((void**)&dz, sizeof(float) * 2 * (size_t)B * h, st));
   float* dz2 = dz;
   float* dz1 = dz + (size_t)B * h;
+  if (mlp_fused(in, h, out, wb, o)) {
+    const int op = (out + GK - 1) / GK * GK;
+    const int smem = FROWS * (op + 8 + h + 8) * (int)sizeof(__nv_bfloat16);
+    k_mlp_dz<<<(B + FROWS - 1) / FROWS, FT, smem, st>>>(h, out, mlp_ptrs(wb, nullptr, o), d_dy, B, z1, z2, dz1, dz2);
+    const int segs = std::min(DW_SEGS, (B + DW_ROWS - 1) / DW_ROWS), seg = ((B + segs - 1) / segs + 31) / 32 * 32;
+    float* g = d_grad;
+    if (segs > 1) {
+      const cudaError_t e = pool_alloc((void**)&g, sizeof(float) * segs * (size_t)o.total, st);
+      if (e != cudaSuccess) {
+        pool_free(dz, st);
+        AQ_CUDA_TRY(e);
+      }
+    }
+    DwJobs J;
+    J.j[0] = DwJob{dz2, a1, g + o.w2, g + o.b2, h, h, 0};
+    J.j[1] = DwJob{dz1, d_x, g + o.w1, g + o.b1, h, in, dw_warps(h, h)};
+    J.j[2] = DwJob{d_dy, a2, g + o.w3, g + o.b3, out, h, J.j[1].first + dw_warps(h, in)};
+    const int warps = J.j[2].first + dw_warps(out, h), ny = (B + seg - 1) / seg;
+    k_mlp_dw<<<dim3((warps * 32 + DWT - 1) / DWT, ny), DWT, 0, st>>>(J, B, seg, o.total, warps);
+    if (segs > 1) {
+      k_mlp_dw_sum<<<grid_for(o.total, 128), 128, 0, st>>>(g, ny, o.total, d_grad);
+      pool_free(g, st);
+    }
+    const cudaError_t e = cudaGetLastError();
+    pool_free(dz, st);
+    AQ_CUDA_TRY(e);
+    return AQ_OK;
+  }
   // layer 3: dW3 = dy^T a2, db3, dz2 = (dy W3) * gelu'(z2)
   k_gemm_bf16<float, float, EPI_STORE><<<gemm_grid(out, h), GTHREADS, 0, st>>>(
       d_dy, out, 0, a2, h, 0, out, h, B, nullptr, nullptr, nullptr, d_grad + o.w3, 0);
