@@ -150,26 +150,29 @@ constexpr int IB = 64;
 
 __device__ __forceinline__ int item_bucket(int c) { return IB - 1 - min(IB - 1, (c - 1) >> 4); }
 
-// parts of a block of c records, and the records per part (the last has the rest)
-__device__ __forceinline__ int item_part(int c, int item_max) {
+// Records per part of block b's c records (the last part has the rest).
+// item_tail > 0: every fourth block is cut into parts of that many, which,
+// ordered last, fill the end of the launch, where the CTAs run out of items.
+__device__ __forceinline__ int item_part(int c, int item_max, int item_tail, int b) {
+  if (item_tail > 0 && (b & 3) == 0) item_max = min(item_max, item_tail);
   const int parts = (c + item_max - 1) / item_max;
   return ((c + parts - 1) / parts + 31) & ~31;
 }
 
-__global__ void k_items_count(const int32_t* __restrict__ start, int nblk, int item_max,
+__global__ void k_items_count(const int32_t* __restrict__ start, int nblk, int item_max, int item_tail,
                               int32_t* __restrict__ item_info) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nblk) return;
   const int c = start[(int64_t)(b + 1) * 64] - start[(int64_t)b * 64];
   if (c <= 0) return;
-  const int per = item_part(c, item_max), full = c / per, rest = c - full * per;
+  const int per = item_part(c, item_max, item_tail, b), full = c / per, rest = c - full * per;
   if (full) atomicAdd(item_info + 1 + item_bucket(per), full);
   if (rest) atomicAdd(item_info + 1 + item_bucket(rest), 1);
 }
 
 // blk_of (sparse grids): the grid block of each compact block index, else null
-__global__ void k_items(const int32_t* __restrict__ start, int nblk, int item_max, int4* __restrict__ items,
-                        int32_t* __restrict__ item_info, const int32_t* __restrict__ blk_of) {
+__global__ void k_items(const int32_t* __restrict__ start, int nblk, int item_max, int item_tail,
+                        int4* __restrict__ items, int32_t* __restrict__ item_info, const int32_t* __restrict__ blk_of) {
   __shared__ int off[IB];
   if (threadIdx.x == 0) {
     int acc = 0;
@@ -185,7 +188,7 @@ __global__ void k_items(const int32_t* __restrict__ start, int nblk, int item_ma
   const int s = start[(int64_t)b * 64], c = start[(int64_t)(b + 1) * 64] - s;
   if (c <= 0) return;
   const int blk = blk_of ? blk_of[b] : b;
-  const int per = item_part(c, item_max), full = c / per, rest = c - full * per;
+  const int per = item_part(c, item_max, item_tail, b), full = c / per, rest = c - full * per;
   if (full) {
     const int k = item_bucket(per);
     const int at = off[k] + atomicAdd(item_info + 1 + IB + k, full);
@@ -690,13 +693,25 @@ struct SimImpl final : SimBase {
     return b + (reg_record ? 0 : sizeof(uint64_t) * (size_t)CH * s->WS);
   }
 
-  // Records per work item, at most.
-  int item_max() const {
-    return (int)std::max<int64_t>(64, (s->n / s->step_grid + 63) / 64 * 64);
-  }
+  // Records per work item, at most: a resident CTA's share of the records.
+  // Fewer leave CTAs idle (3D, 262,144 particles in 512 blocks: 2.32 ms a
+  // frame of 32 substeps with whole blocks, 2.04 with this; 2D, 8,192
+  // particles in 16 blocks: 0.92 and 0.51); more items stage and flush more
+  // tiles than they balance (3D, 2,097,152: 13.5 ms with 64 records, 11.7 with
+  // 256, 10.4 with whole blocks, which this gives).
+  int item_max() const { return (int)std::max<int64_t>(64, (s->n / s->step_grid + 63) / 64 * 64); }
+
+  // Small parts for the end of the launch (item_part) where a CTA has little
+  // more than one item's worth: 262,144 to 550,000 particles 3 to 8 % faster;
+  // with several items a CTA the extra tiles cost more (800,000: 2 % slower,
+  // 2,097,152: 5 %).
+  int item_tail() const { return s->n < (int64_t)400 * s->step_grid ? 128 : 0; }
 
   // Work items there can be, at most: a launch needs no more CTAs.
-  int64_t items_bound() const { return std::min<int64_t>(s->nblk, s->n) + s->n / item_max() + 1; }
+  int64_t items_bound() const {
+    const int part = item_tail() ? std::min(item_max(), item_tail()) : item_max();
+    return std::min<int64_t>(s->nblk, s->n) + s->n / part + 1;
+  }
 
   int sort(cudaStream_t st) override {
     if (s->P.sparse) return sort_sparse(st);
@@ -713,9 +728,9 @@ struct SimImpl final : SimBase {
     const int nxt = 1 - S_->cur;
     k_scatter<<<grid_for(n, SCATTER_T), SCATTER_T, 0, st>>>(S_->words[S_->cur], S_->pid[S_->cur], S_->words[nxt], S_->pid[nxt],
                                                 S_->keys, S_->ranks, S_->cell_start, n, S_->W);
-    const int im = item_max();
-    k_items_count<<<grid_for(S_->nblk, 256), 256, 0, st>>>(S_->cell_start, S_->nblk, im, S_->n_items);
-    k_items<<<grid_for(S_->nblk, 256), 256, 0, st>>>(S_->cell_start, S_->nblk, im, S_->items, S_->n_items, nullptr);
+    const int im = item_max(), it = item_tail();
+    k_items_count<<<grid_for(S_->nblk, 256), 256, 0, st>>>(S_->cell_start, S_->nblk, im, it, S_->n_items);
+    k_items<<<grid_for(S_->nblk, 256), 256, 0, st>>>(S_->cell_start, S_->nblk, im, it, S_->items, S_->n_items, nullptr);
     AQ_CUDA_TRY(cudaGetLastError());
     S_->cur = nxt;
     S_->launches += 7;
@@ -779,9 +794,9 @@ struct SimImpl final : SimBase {
     k_scatter<<<grid_for(n, SCATTER_T), SCATTER_T, 0, st>>>(
         S_->words[S_->cur], S_->pid[S_->cur], S_->words[nxt], S_->pid[nxt], S_->keys, S_->ranks, S_->cstart, n, S_->W);
     AQ_CUDA_TRY(cudaMemsetAsync(S_->n_items, 0, sizeof(int32_t) * (1 + 2 * IB), st));
-    const int im = item_max();
-    k_items_count<<<grid_for(n_occ, 256), 256, 0, st>>>(S_->cstart, n_occ, im, S_->n_items);
-    k_items<<<grid_for(n_occ, 256), 256, 0, st>>>(S_->cstart, n_occ, im, S_->items, S_->n_items, S_->occ_blk);
+    const int im = item_max(), it = item_tail();
+    k_items_count<<<grid_for(n_occ, 256), 256, 0, st>>>(S_->cstart, n_occ, im, it, S_->n_items);
+    k_items<<<grid_for(n_occ, 256), 256, 0, st>>>(S_->cstart, n_occ, im, it, S_->items, S_->n_items, S_->occ_blk);
     // the active blocks: empty the pools, then the 3^D blocks around every
     // occupied block; pools grow (dropping their contents, which the next
     // launch rebuilds from the records) when the new set may not fit
