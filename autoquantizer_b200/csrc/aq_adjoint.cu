@@ -258,19 +258,24 @@ __device__ __forceinline__ void ad_load(const R* __restrict__ st, int64_t p, R (
 // and to the grid.  No two warps share a tile, so there is no CTA barrier.
 // Particle by particle with scalar global atomics, from rows of 96 bytes and
 // with the grid's operation in kernels of its own, a substep of the 3D
-// falling block (262,144 particles, FP32) took 127 us forward (now 52) and
-// 287 us backward, recomputed sums and squares included (now 141).
+// falling block (262,144 particles, FP32) took 127 us forward (now 49) and
+// 287 us backward, recomputed sums and squares included (now 124).
 //
 // Half a block's cells (4 x 2 x 4, and 4 x 8 in 2D) reach 6 x 4 x 6 = 144
 // nodes (6 x 10 = 60); AdTile leaves room for a cell of drift on every side,
 // and for the warps whose particles lie in two blocks.
 template <int D>
 struct AdTile {
-  static constexpr int N = D == 3 ? 384 : 192;
+  static constexpr int N = D == 3 ? 416 : 192;
 };
 
+// In 3D the tile's stride of axis 0 is padded to 4 mod 8 nodes, so that the
+// planes of a warp's neighbouring cells fall in different 16-byte bank groups
+// (a forward pass 52 -> 49 us at 262,144 particles).
 struct AdBox {
   int o[3], e1, e2, n;  // origin, extents of axes 1 and 2, nodes
+  int sa;               // tile stride of axis 0
+  int size;             // tile nodes with the padding
   bool fits;
 };
 
@@ -295,26 +300,31 @@ __device__ __forceinline__ AdBox ad_box(bool on, const int (&base)[3]) {
   b.fits = any;
 #pragma unroll
   for (int d = 0; d < D; ++d) b.fits = b.fits && e[d] <= AdTile<D>::N;
-  b.n = b.fits ? e[0] * e[1] * e[2] : 0;  // each extent <= 384: no overflow
-  b.fits = b.fits && b.n <= AdTile<D>::N;
+  // each extent <= AdTile::N: no overflow
+  b.n = b.fits ? e[0] * e[1] * e[2] : 0;
+  b.sa = D == 3 ? ((b.e1 * b.e2 + 3) & ~7) + 4 : b.e1;
+  b.size = b.fits ? e[0] * b.sa : 0;
+  b.fits = b.fits && b.size <= AdTile<D>::N;
   return b;
 }
 
-// node j of a box: its index in axis order (exact float floors: j < 2^10)
+// node j of a box: its grid index; returns its place in the tile (exact float
+// floors: j < 2^10)
 template <int D>
-__device__ __forceinline__ void ad_node(const AdBox& b, int j, int (&I)[3]) {
+__device__ __forceinline__ int ad_node(const AdBox& b, int j, int (&I)[3]) {
   if (D == 3) {
     const int q = (int)(((float)j + 0.5f) / (float)b.e2);
-    const int i0 = (int)(((float)q + 0.5f) / (float)b.e1);
+    const int i0 = (int)(((float)q + 0.5f) / (float)b.e1), i1 = q - i0 * b.e1, i2 = j - q * b.e2;
     I[0] = b.o[0] + i0;
-    I[1] = b.o[1] + (q - i0 * b.e1);
-    I[2] = b.o[2] + (j - q * b.e2);
-  } else {
-    const int i0 = (int)(((float)j + 0.5f) / (float)b.e1);
-    I[0] = b.o[0] + i0;
-    I[1] = b.o[1] + (j - i0 * b.e1);
-    I[2] = 0;
+    I[1] = b.o[1] + i1;
+    I[2] = b.o[2] + i2;
+    return i0 * b.sa + i1 * b.e2 + i2;
   }
+  const int i0 = (int)(((float)j + 0.5f) / (float)b.e1);
+  I[0] = b.o[0] + i0;
+  I[1] = b.o[1] + (j - i0 * b.e1);
+  I[2] = 0;
+  return j;
 }
 
 // wall mask of component k at node I given the velocity sign (grid_op)
@@ -327,10 +337,13 @@ __device__ __forceinline__ bool ad_wall(const AdK<R>& K, const int (&I)[3], int 
 template <int D, class R>
 struct AdGridOp {
   typedef typename R4T<R>::type R4;
+  typedef R4 Raw;
+  static constexpr int STAGE = 3;
   const AdK<R>& K;
   const R4* grid;
-  __device__ __forceinline__ R4 operator()(const int (&I)[3]) const {
-    R4 g = grid[ad_cell<D>(K.res, I)];
+  __device__ __forceinline__ Raw fetch(const int (&I)[3]) const { return grid[ad_cell<D>(K.res, I)]; }
+  __device__ __forceinline__ R4 operator()(const int (&I)[3]) const { return apply(fetch(I), I); }
+  __device__ __forceinline__ R4 apply(R4 g, const int (&I)[3]) const {
     const R inv_m = (R)1 / (g.x + (R)1e-10);
     R v[3] = {inv_m * g.y, inv_m * g.z, D == 3 ? inv_m * g.w : (R)0};
     v[1] -= K.dt * K.grav;
@@ -351,12 +364,20 @@ struct AdGridOp {
 template <int D, class R>
 struct AdGridOpT {
   typedef typename R4T<R>::type R4;
+  struct Raw {
+    R4 g, b;
+  };
+  static constexpr int STAGE = 2;
   const AdK<R>& K;
   const R4* grid;
   const R4* gvb;
-  __device__ __forceinline__ R4 operator()(const int (&I)[3]) const {
+  __device__ __forceinline__ Raw fetch(const int (&I)[3]) const {
     const int64_t c = ad_cell<D>(K.res, I);
-    const R4 g = grid[c], b = gvb[c];
+    return Raw{grid[c], gvb[c]};
+  }
+  __device__ __forceinline__ R4 operator()(const int (&I)[3]) const { return apply(fetch(I), I); }
+  __device__ __forceinline__ R4 apply(const Raw& raw, const int (&I)[3]) const {
+    const R4 g = raw.g, b = raw.b;
     const R P[3] = {g.y, g.z, g.w};
     const R inv_m = (R)1 / (g.x + (R)1e-10);
     R v[3] = {inv_m * P[0], inv_m * P[1], D == 3 ? inv_m * P[2] : (R)0};
@@ -396,13 +417,24 @@ struct AdGridOpT {
   }
 };
 
-// copy a box into a tile through the node's operation
+// copy a box into a tile through the node's operation, F::STAGE nodes of a
+// lane in flight at a time
 template <int D, class R4, class F>
 __device__ __forceinline__ void ad_stage(const AdBox& b, R4* tile, const F& node) {
-  for (int j = threadIdx.x & 31; j < b.n; j += 32) {
-    int I[3];
-    ad_node<D>(b, j, I);
-    tile[j] = node(I);
+  for (int j0 = threadIdx.x & 31; j0 < b.n; j0 += 32 * F::STAGE) {
+    typename F::Raw raw[F::STAGE];
+    int I[F::STAGE][3], at[F::STAGE];
+#pragma unroll
+    for (int q = 0; q < F::STAGE; ++q) {
+      at[q] = -1;
+      if (j0 + 32 * q < b.n) {
+        at[q] = ad_node<D>(b, j0 + 32 * q, I[q]);
+        raw[q] = node.fetch(I[q]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < F::STAGE; ++q)
+      if (at[q] >= 0) tile[at[q]] = node.apply(raw[q], I[q]);
   }
   __syncwarp();
 }
@@ -411,7 +443,7 @@ template <class R4>
 __device__ __forceinline__ void ad_zero(const AdBox& b, R4* tile) {
   R4 z;
   z.x = z.y = z.z = z.w = 0;
-  for (int j = threadIdx.x & 31; j < b.n; j += 32) tile[j] = z;
+  for (int j = threadIdx.x & 31; j < b.size; j += 32) tile[j] = z;
   __syncwarp();
 }
 
@@ -419,17 +451,16 @@ template <int D, class R, class R4>
 __device__ __forceinline__ void ad_flush(const AdK<R>& K, const AdBox& b, const R4* tile, R4* grid) {
   __syncwarp();
   for (int j = threadIdx.x & 31; j < b.n; j += 32) {
-    const R4 v = tile[j];
-    if (v.x == (R)0 && v.y == (R)0 && v.z == (R)0 && v.w == (R)0) continue;
     int I[3];
-    ad_node<D>(b, j, I);
+    const R4 v = tile[ad_node<D>(b, j, I)];
+    if (v.x == (R)0 && v.y == (R)0 && v.z == (R)0 && v.w == (R)0) continue;
     red_add_node(grid + ad_cell<D>(K.res, I), v.x, v.y, v.z, v.w);
   }
 }
 
 template <int D>
 __device__ __forceinline__ int ad_local(const AdBox& b, const int (&base)[3]) {
-  return D == 3 ? ((base[0] - b.o[0]) * b.e1 + (base[1] - b.o[1])) * b.e2 + (base[2] - b.o[2])
+  return D == 3 ? (base[0] - b.o[0]) * b.sa + (base[1] - b.o[1]) * b.e2 + (base[2] - b.o[2])
                 : (base[0] - b.o[0]) * b.e1 + (base[1] - b.o[1]);
 }
 
@@ -482,34 +513,50 @@ __device__ __forceinline__ void ad_gather(const S& src, const R (&w)[3][3], R (&
     }
 }
 
-// xb += sum_i h_i grad w_i with h_i = c0 g.x + (g.y, g.z, g.w) . (q + Aff off)
+// ad_gather, and xb += sum_i h_i grad w_i with h_i = c0 g.x + (g.y, g.z, g.w) .
+// (q + Aff off), in one walk over the nodes (in two, the reverse kernels took
+// 61 and 42 us instead of 52 and 37).
 template <int D, class R, bool TILE, class S>
-__device__ __forceinline__ void ad_grad_w(const S& src, const R (&w)[3][3], const R (&dw)[3][3], R c0, const R (&q)[3],
-                                          const R (&Aff)[9], R (&xb)[3]) {
+__device__ __forceinline__ void ad_gather_grad(const S& src, const R (&w)[3][3], const R (&dw)[3][3], R c0,
+                                               const R (&q)[3], const R (&Aff)[9], R (&nv)[3], R (&Sm)[3][3],
+                                               R (&xb)[3]) {
+#pragma unroll
+  for (int d = 0; d < 3; ++d) nv[d] = Sm[d][0] = Sm[d][1] = Sm[d][2] = 0;
 #pragma unroll(TILE ? 3 : 1)
   for (int a = 0; a < 3; ++a)
 #pragma unroll(TILE ? 3 : 1)
     for (int b = 0; b < 3; ++b) {
-      R qab[3], H = 0, Hd = 0;
+      R qab[3], P[3] = {0, 0, 0}, Q[3] = {0, 0, 0}, H = 0, Hd = 0;
 #pragma unroll
       for (int d = 0; d < D; ++d) qab[d] = q[d] + (R)a * Aff[d * D] + (R)b * Aff[d * D + 1];
 #pragma unroll(TILE ? 3 : 1)
       for (int c = 0; c < (D == 3 ? 3 : 1); ++c) {
         const auto g = src(a, b, c);
+        const R wc = D == 3 ? w[c][2] : (R)1;
         const R gv[3] = {g.y, g.z, g.w};
         R h = c0 * g.x;
 #pragma unroll
-        for (int d = 0; d < D; ++d) h += gv[d] * (D == 3 ? qab[d] + (R)c * Aff[d * D + 2] : qab[d]);
-        if (D == 3) {
-          H += w[c][2] * h;
-          Hd += dw[c][2] * h;
-        } else {
-          H = h;
+        for (int d = 0; d < D; ++d) {
+          const R wg = wc * gv[d];
+          P[d] += wg;
+          if (D == 3 && c) Q[d] += (R)c * wg;
+          h += gv[d] * (D == 3 ? qab[d] + (R)c * Aff[d * D + 2] : qab[d]);
         }
+        H += wc * h;
+        if (D == 3) Hd += dw[c][2] * h;
+      }
+      const R wab = w[a][0] * w[b][1];
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        const R wp = wab * P[d];
+        nv[d] += wp;
+        Sm[d][0] += (R)a * wp;
+        Sm[d][1] += (R)b * wp;
+        if (D == 3) Sm[d][2] += wab * Q[d];
       }
       xb[0] += dw[a][0] * w[b][1] * H;
       xb[1] += w[a][0] * dw[b][1] * H;
-      if (D == 3) xb[2] += w[a][0] * w[b][1] * Hd;
+      if (D == 3) xb[2] += wab * Hd;
     }
 }
 
@@ -529,7 +576,7 @@ __device__ __forceinline__ void ad_scatter(const AdK<R>& K, bool on, const int (
     rank = __popc(peers & ((1u << lane) - 1u));
     rounds = (int)__reduce_max_sync(0xffffffffu, (unsigned)__popc(peers));
   }
-  const int sb = D == 3 ? box.e2 : 1, sa = D == 3 ? box.e1 * box.e2 : box.e1;
+  const int sb = D == 3 ? box.e2 : 1, sa = box.sa;
   for (int r = 0; r < rounds; ++r) {
     const bool mine = on && rank == r;
     const unsigned tm = __ballot_sync(0xffffffffu, mine);
@@ -629,7 +676,7 @@ __global__ void __launch_bounds__(AD_T) k_ad_pass(const __grid_constant__ AdK<R>
     if (box.fits) {
       ad_stage<D>(box, tile, node);
       const AdSrc<D, R, true, AdGridOp<D, R>> src{tile + (on ? ad_local<D>(box, base) : 0),
-                                                  D == 3 ? box.e1 * box.e2 : box.e1, D == 3 ? box.e2 : 1, node, base};
+                                                  box.sa, D == 3 ? box.e2 : 1, node, base};
       if (on) ad_gather<D, R, true>(src, w, nv, Sm);
       __syncwarp();
     } else if (on) {
@@ -722,71 +769,73 @@ __global__ void __launch_bounds__(AD_T) k_ad_g2p_bwd(const __grid_constant__ AdK
   }
   const AdBox box = ad_box<D>(on, base);
   const AdGridOp<D, R> node{K, grid};
-  R nv[3], Sm[3][3];
-  const AdSrc<D, R, true, AdGridOp<D, R>> src{tile + (on && box.fits ? ad_local<D>(box, base) : 0),
-                                              D == 3 ? box.e1 * box.e2 : box.e1, D == 3 ? box.e2 : 1, node, base};
-  const AdSrc<D, R, false, AdGridOp<D, R>> gsrc{nullptr, 0, 0, node, base};
+  R nv[3], Sm[3][3], q[3], Aff[9], dw[3][3], xb[3];
+  if (on) {
+    R Cpb[9];  // the new C's adjoint, with F' = (I + dt C') F's (J' = (1 + dt tr C') J's) part
+#pragma unroll
+    for (int k = 0; k < D * D; ++k) Cpb[k] = bo[S::C + k];
+    if (HF) {
+#pragma unroll
+      for (int i = 0; i < D; ++i)
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+          R c = 0;
+#pragma unroll
+          for (int k = 0; k < D; ++k) c += bo[S::FJ + i * D + k] * s[S::FJ + j * D + k];  // F'bar F^T
+          Cpb[i * D + j] += K.dt * c;
+        }
+    } else {
+      const R trb = K.dt * s[S::FJ] * bo[S::FJ];
+#pragma unroll
+      for (int d = 0; d < D; ++d) Cpb[d * D + d] += trb;
+    }
+#pragma unroll
+    for (int k = 0; k < D * D; ++k) Aff[k] = K.four_inv_dx * Cpb[k];
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      xb[d] = bo[S::X + d];
+      q[d] = bo[S::V + d] + K.dt * bo[S::X + d];
+#pragma unroll
+      for (int e = 0; e < D; ++e) q[d] -= Aff[d * D + e] * fx[e];
+    }
+    ad_dweights<D, R>(K, fx, dw);
+  }
   if (box.fits) {
     ad_stage<D>(box, tile, node);
     ad_zero(box, stile);
-    if (on) ad_gather<D, R, true>(src, w, nv, Sm);
+    const AdSrc<D, R, true, AdGridOp<D, R>> src{tile + (on ? ad_local<D>(box, base) : 0), box.sa, D == 3 ? box.e2 : 1,
+                                                node, base};
+    if (on) ad_gather_grad<D, R, true>(src, w, dw, (R)0, q, Aff, nv, Sm, xb);
   } else if (on) {
-    ad_gather<D, R, false>(gsrc, w, nv, Sm);
+    const AdSrc<D, R, false, AdGridOp<D, R>> src{nullptr, 0, 0, node, base};
+    ad_gather_grad<D, R, false>(src, w, dw, (R)0, q, Aff, nv, Sm, xb);
   }
-  R q[3], Aff[9], xb[3] = {0, 0, 0};
   if (on) {
     R nC[9];
 #pragma unroll
     for (int d = 0; d < D; ++d)
 #pragma unroll
-      for (int e = 0; e < D; ++e) nC[d * D + e] = K.four_inv_dx * (Sm[d][e] - nv[d] * fx[e]);
-    R Cpb[9];
-#pragma unroll
-    for (int k = 0; k < D * D; ++k) Cpb[k] = bo[S::C + k];
+      for (int e = 0; e < D; ++e) {
+        nC[d * D + e] = K.four_inv_dx * (Sm[d][e] - nv[d] * fx[e]);
+        xb[e] -= Aff[d * D + e] * K.inv_dx * nv[d];
+      }
     if (HF) {
-      // F' = (I + dt C') F
 #pragma unroll
       for (int i = 0; i < D; ++i)
 #pragma unroll
         for (int j = 0; j < D; ++j) {
-          R a = 0, c = 0;
+          R a = 0;
 #pragma unroll
-          for (int k = 0; k < D; ++k) {
+          for (int k = 0; k < D; ++k)
             a += ((k == i ? (R)1 : (R)0) + K.dt * nC[k * D + i]) * bo[S::FJ + k * D + j];  // (I+dtC')^T F'bar
-            c += bo[S::FJ + i * D + k] * s[S::FJ + j * D + k];                            // F'bar F^T
-          }
           ab_in[ad_at<NS>(p, S::FJ + i * D + j)] = a;
-          Cpb[i * D + j] += K.dt * c;
         }
     } else {
       R tr = 0;
 #pragma unroll
       for (int d = 0; d < D; ++d) tr += nC[d * D + d];
       ab_in[ad_at<NS>(p, S::FJ)] = ((R)1 + K.dt * tr) * bo[S::FJ];
-      const R trb = K.dt * s[S::FJ] * bo[S::FJ];
-#pragma unroll
-      for (int d = 0; d < D; ++d) Cpb[d * D + d] += trb;
     }
-#pragma unroll
-    for (int e = 0; e < D; ++e) {
-      xb[e] = bo[S::X + e];
-#pragma unroll
-      for (int d = 0; d < D; ++d) xb[e] -= K.four_inv_dx2 * Cpb[d * D + e] * nv[d];
-    }
-#pragma unroll
-    for (int k = 0; k < D * D; ++k) Aff[k] = K.four_inv_dx * Cpb[k];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      q[d] = bo[S::V + d] + K.dt * bo[S::X + d];
-#pragma unroll
-      for (int e = 0; e < D; ++e) q[d] -= Aff[d * D + e] * fx[e];
-    }
-    R dw[3][3];
-    ad_dweights<D, R>(K, fx, dw);
-    if (box.fits)
-      ad_grad_w<D, R, true>(src, w, dw, (R)0, q, Aff, xb);
-    else
-      ad_grad_w<D, R, false>(gsrc, w, dw, (R)0, q, Aff, xb);
 #pragma unroll
     for (int d = 0; d < D; ++d) ab_in[ad_at<NS>(p, S::X + d)] = xb[d];
   }
@@ -855,15 +904,13 @@ __global__ void __launch_bounds__(AD_T) k_ad_p2g_bwd(const __grid_constant__ AdK
   if (box.fits) {
     ad_stage<D>(box, tile, node);
     const AdSrc<D, R, true, AdGridOpT<D, R>> src{tile + (on ? ad_local<D>(box, base) : 0),
-                                                 D == 3 ? box.e1 * box.e2 : box.e1, D == 3 ? box.e2 : 1, node, base};
+                                                 box.sa, D == 3 ? box.e2 : 1, node, base};
     if (on) {
-      ad_gather<D, R, true>(src, w, nv, Sm);
-      ad_grad_w<D, R, true>(src, w, dw, K.p_mass, q, Aff, xb);
+      ad_gather_grad<D, R, true>(src, w, dw, K.p_mass, q, Aff, nv, Sm, xb);
     }
   } else if (on) {
     const AdSrc<D, R, false, AdGridOpT<D, R>> src{nullptr, 0, 0, node, base};
-    ad_gather<D, R, false>(src, w, nv, Sm);
-    ad_grad_w<D, R, false>(src, w, dw, K.p_mass, q, Aff, xb);
+    ad_gather_grad<D, R, false>(src, w, dw, K.p_mass, q, Aff, nv, Sm, xb);
   }
   if (on) {
     R sb[9];
