@@ -615,6 +615,14 @@ __device__ __forceinline__ void ad_scatter(const AdK<R>& K, bool on, const int (
   }
 }
 
+// Launched while the kernel before it in the stream may still run (launch_pdl):
+// everything before this is the launch itself, nothing of the other kernel's
+// is touched; the kernel after may in turn start being launched.
+__device__ __forceinline__ void ad_begin() {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // zero a grid for a later scatter (grid-stride over its nodes)
 template <class R4>
 __device__ __forceinline__ void ad_clear(R4* g, int64_t nodes) {
@@ -661,6 +669,7 @@ __global__ void __launch_bounds__(AD_T) k_ad_pass(const __grid_constant__ AdK<R>
   constexpr int NS = S::NS;
   __shared__ __align__(16) R4 tiles[AD_T / 32][AdTile<D>::N];
   R4* const tile = tiles[threadIdx.x >> 5];
+  ad_begin();
   ad_clear(gclr, nodes);
   const int64_t p = (int64_t)blockIdx.x * AD_T + threadIdx.x;
   const bool on = p < n;
@@ -755,6 +764,7 @@ __global__ void __launch_bounds__(AD_T) k_ad_g2p_bwd(const __grid_constant__ AdK
   extern __shared__ __align__(16) unsigned char ad_smem[];
   R4* const tile = reinterpret_cast<R4*>(ad_smem) + (threadIdx.x >> 5) * 2 * AdTile<D>::N;
   R4* const stile = tile + AdTile<D>::N;
+  ad_begin();
   ad_clear(gclr, nodes);
   const int64_t p = (int64_t)blockIdx.x * AD_T + threadIdx.x;
   const bool on = p < n;
@@ -883,6 +893,7 @@ __global__ void __launch_bounds__(AD_T) k_ad_p2g_bwd(const __grid_constant__ AdK
   constexpr int NS = S::NS;
   __shared__ __align__(16) R4 tiles[AD_T / 32][AdTile<D>::N];
   R4* const tile = tiles[threadIdx.x >> 5];
+  ad_begin();
   const int64_t p = (int64_t)blockIdx.x * AD_T + threadIdx.x;
   const bool on = p < n;
   R s[NS], bi[NS];
@@ -1129,9 +1140,8 @@ struct AdImpl final : AdBase {
 
   // the sums of state `in` into g[rot]
   int p2g(const void* in, cudaStream_t st) override {
-    k_ad_pass<D, HF, R, false, true><<<blocks(), AD_T, 0, st>>>(K, (const R*)in, nullptr, a->n, nullptr, g(0), g(1),
-                                                                a->ncell);
-    AQ_CUDA_TRY(cudaGetLastError());
+    AQ_CUDA_TRY(launch_pdl(k_ad_pass<D, HF, R, false, true>, blocks(), AD_T, 0, st, K, (const R*)in, (R*)nullptr, a->n,
+                           (const R4*)nullptr, g(0), g(1), a->ncell));
     return AQ_OK;
   }
   // substep t from the state whose sums are in g[rot], and the new state's
@@ -1139,23 +1149,21 @@ struct AdImpl final : AdBase {
   int g2p(const void* in, void* out, int t, bool then_p2g, cudaStream_t st) override {
     set_substep(t);
     if (then_p2g)
-      k_ad_pass<D, HF, R, true, true><<<blocks(), AD_T, 0, st>>>(K, (const R*)in, (R*)out, a->n, g(0), g(1), g(2),
-                                                                 a->ncell);
+      AQ_CUDA_TRY(launch_pdl(k_ad_pass<D, HF, R, true, true>, blocks(), AD_T, 0, st, K, (const R*)in, (R*)out, a->n,
+                             (const R4*)g(0), g(1), g(2), a->ncell));
     else
-      k_ad_pass<D, HF, R, true, false><<<blocks(), AD_T, 0, st>>>(K, (const R*)in, (R*)out, a->n, g(0), nullptr,
-                                                                  nullptr, 0);
-    AQ_CUDA_TRY(cudaGetLastError());
+      AQ_CUDA_TRY(launch_pdl(k_ad_pass<D, HF, R, true, false>, blocks(), AD_T, 0, st, K, (const R*)in, (R*)out, a->n,
+                             (const R4*)g(0), (R4*)nullptr, (R4*)nullptr, (int64_t)0));
     a->rot = (a->rot + 1) % 3;
     return AQ_OK;
   }
   // reverse of substep t, whose old state's sums are in g[rot]
   int step_bwd(const void* s_in, const void* ab_out, void* ab_in, int t, bool accumulate, cudaStream_t st) override {
     set_substep(t);
-    k_ad_g2p_bwd<D, HF, R><<<blocks(), AD_T, G2P_BWD_SMEM, st>>>(K, (const R*)s_in, (const R*)ab_out, (R*)ab_in, a->n,
-                                                                 g(0), g(1), g(2), a->ncell);
-    k_ad_p2g_bwd<D, HF, R><<<blocks(), AD_T, 0, st>>>(K, (const R*)s_in, (R*)ab_in, a->n, g(0), g(1),
-                                                      accumulate ? a->dsens : nullptr);
-    AQ_CUDA_TRY(cudaGetLastError());
+    AQ_CUDA_TRY(launch_pdl(k_ad_g2p_bwd<D, HF, R>, blocks(), AD_T, G2P_BWD_SMEM, st, K, (const R*)s_in,
+                           (const R*)ab_out, (R*)ab_in, a->n, (const R4*)g(0), g(1), g(2), a->ncell));
+    AQ_CUDA_TRY(launch_pdl(k_ad_p2g_bwd<D, HF, R>, blocks(), AD_T, 0, st, K, (const R*)s_in, (R*)ab_in, a->n,
+                           (const R4*)g(0), (const R4*)g(1), accumulate ? a->dsens : (double*)nullptr));
     a->rot = (a->rot + 2) % 3;
     return AQ_OK;
   }
