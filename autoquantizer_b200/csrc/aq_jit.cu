@@ -114,13 +114,13 @@ void fmt_f64(std::string& s, double v) {
 
 }  // namespace
 
-std::string jit_layout_source(const aq_layout& L) {
+std::string jit_layout_source(const aq_layout& L, int min_blocks) {
   std::string s;
   char b[256];
   snprintf(b, sizeof b,
            "struct JitLayout {\n  static constexpr bool kRegRecord = %s;\n  static constexpr int kWords = %d;\n"
            "  static constexpr int kMinBlocks = %d;\n",
-           jit_reg_record(L) ? "true" : "false", L.n_words, jit_min_blocks(L));
+           jit_reg_record(L) ? "true" : "false", L.n_words, min_blocks);
   s += b;
   s += "  static __device__ __forceinline__ aq_layout get(const aq_layout&) {\n    return aq_layout{";
   snprintf(b, sizeof b, "%d, %d, %d, %d, %d, %d, {0, 0}, {", L.n_slots, L.n_words, L.total_bits, L.compute_f64,
@@ -167,7 +167,7 @@ void* jit_k_step(int D, bool HF, bool HM, bool f64, bool col, bool sparse, bool 
   snprintf(name, sizeof name, "aq::k_step<%d, %s, %s, %s, aq::JitLayout, %s, %s, %s>", D, HF ? "true" : "false",
            HM ? "true" : "false", f64 ? "double" : "float", col ? "true" : "false", sparse ? "true" : "false", multi ? "true" : "false");
   std::string src = "#include \"aq_kernels.cuh\"\nnamespace aq {\n";
-  src += jit_layout_source(L);
+  src += jit_layout_source(L, jit_min_blocks(L, D, multi));
   src += "}\n";
   // AQ_JIT_SOURCE_DIR (environment, kernel development): compile from the
   // aq_kernels.cuh found in this folder (and the headers it includes from

@@ -15,7 +15,7 @@ bool jit_available();
 // col, sparse, multi> for layout L; returns a CUfunction, or null with *err set.
 void* jit_k_step(int D, bool HF, bool HM, bool f64, bool col, bool sparse, bool multi, const aq_layout& L,
                  std::string* err);
-std::string jit_layout_source(const aq_layout& L);
+std::string jit_layout_source(const aq_layout& L, int min_blocks);
 
 // Whether the layout-specialized k_step keeps a record's words in registers
 // rather than in a shared-memory slot per thread: short records, and records
@@ -29,11 +29,19 @@ inline bool jit_raw_record(const aq_layout& L) {
   return true;
 }
 inline bool jit_reg_record(const aq_layout& L) { return L.n_words <= kJitRegRecordMaxWords || jit_raw_record(L); }
-// CTAs per SM k_step's registers are budgeted for: 80 registers a thread
-// with short register records, 128 otherwise
-constexpr int kJitShortRecordMinBlocks = 768 / AQ_CH, kJitLongRecordMinBlocks = 512 / AQ_CH;
-inline int jit_min_blocks(const aq_layout& L) {
-  return L.n_words <= kJitRegRecordMaxWords ? kJitShortRecordMinBlocks : kJitLongRecordMinBlocks;
+// CTAs per SM k_step's registers are budgeted for.  Several passes a launch
+// (MULTI) run one warp's work per scheduler or little more, so registers
+// count and warps do not: 128 a thread (2D, 65,536 quantized: 480 -> 424 us a
+// frame of 32 substeps against 80 registers; 3D, 20,000: 730 -> 695).  Else
+// short records take 80 registers in 3D (12 CTAs; 11 and 14 within 1 %, 9 and
+// 10 2 to 4 % slower at 2,097,152 particles) and 73 in 2D (14; 300,000: 936
+// -> 829 us against 12), long ones 113 (9; 262,144 to 1,200,000 FP32
+// particles: +1.5 to -4 % against 8).
+constexpr int kJitShortRecordMinBlocks = 768 / AQ_CH;
+inline int jit_min_blocks(const aq_layout& L, int D, bool multi) {
+  if (multi) return 512 / AQ_CH;
+  if (L.n_words > kJitRegRecordMaxWords) return 576 / AQ_CH;
+  return D == 2 ? 896 / AQ_CH : kJitShortRecordMinBlocks;
 }
 int jit_set_smem(void* fn, int bytes);
 int jit_occupancy(void* fn, int block, size_t smem, int* out);

@@ -68,9 +68,6 @@ constexpr int NWARP = CH / 32;
 // CTAs per SM the register allocation of k_step must allow: the layout's
 // choice (LA::kMinBlocks) for float, 256 / CH (255 registers) for double
 // (3D FP64 state, 200,000 particles: 15 % faster than with 128 registers).
-// Short records kept in registers run best at 768 / CH CTAs (80 registers:
-// more resident warps beat the extra spills); records in shared-memory
-// slots at 512 / CH.
 #ifndef AQ_STEP_MIN_BLOCKS
 #define AQ_STEP_MIN_BLOCKS(R, LA) (sizeof(R) == 8 ? 256 / AQ_CH : LA::kMinBlocks)
 #endif

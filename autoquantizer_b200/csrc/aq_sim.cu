@@ -4,12 +4,12 @@
 //
 // Per substep: one pass of k_step (grid_op of the accumulated grid as each
 // tile is staged, G2P of substep k, P2G of substep k+1 into the next of three
-// grids, the third being cleared for the substep after).  The passes between
-// two re-binnings are one cooperative launch with a grid barrier between
-// passes.  Every sort_interval substeps the records are re-binned: k_bin (cell key and rank), an exclusive scan of the
-// per-cell counts, k_scatter (records and ids into block-wide slot-major
-// order), k_items_count + k_items (one work item per occupied block, the
-// fullest blocks first).
+// grids, the third being cleared for the substep after).  In small scenes the
+// passes between two re-binnings are one cooperative launch with a grid
+// barrier between passes.  Every sort_interval substeps the records are
+// re-binned: k_bin (cell key and rank), an exclusive scan of the per-cell
+// counts, k_scatter (records and ids into block-wide slot-major
+// order), k_items (the work items, the largest first; the scan counts them).
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
@@ -159,15 +159,19 @@ __device__ __forceinline__ int item_part(int c, int item_max, int item_tail, int
   return ((c + parts - 1) / parts + 31) & ~31;
 }
 
+// the items of block b (c > 0 records) into the bucket sizes
+__device__ __forceinline__ void count_items(int c, int item_max, int item_tail, int b, int32_t* item_info) {
+  const int per = item_part(c, item_max, item_tail, b), full = c / per, rest = c - full * per;
+  if (full) atomicAdd(item_info + 1 + item_bucket(per), full);
+  if (rest) atomicAdd(item_info + 1 + item_bucket(rest), 1);
+}
+
 __global__ void k_items_count(const int32_t* __restrict__ start, int nblk, int item_max, int item_tail,
                               int32_t* __restrict__ item_info) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nblk) return;
   const int c = start[(int64_t)(b + 1) * 64] - start[(int64_t)b * 64];
-  if (c <= 0) return;
-  const int per = item_part(c, item_max, item_tail, b), full = c / per, rest = c - full * per;
-  if (full) atomicAdd(item_info + 1 + item_bucket(per), full);
-  if (rest) atomicAdd(item_info + 1 + item_bucket(rest), 1);
+  if (c > 0) count_items(c, item_max, item_tail, b, item_info);
 }
 
 // blk_of (sparse grids): the grid block of each compact block index, else null
@@ -441,8 +445,16 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_top(int32_t* __restrict__ sums,
   if (threadIdx.x == 0) out[n] = total;
 }
 
+// tops: sums holds the tiles' sums, not their exclusive scan: every CTA adds up
+// those before its own (one launch less than k_scan_top while there are few).
+// item_info: also k_items_count's bucket sizes, from the counts of the tile's
+// 64 blocks (16 threads of 4 cells each).
+constexpr int SCAN_TOPS = 1024;
+
 __global__ void __launch_bounds__(SCAN_T) k_scan_apply(const int32_t* __restrict__ in, int64_t n,
-                                                       const int32_t* __restrict__ offs, int32_t* __restrict__ out) {
+                                                       const int32_t* __restrict__ sums, int tops,
+                                                       int32_t* __restrict__ out, int item_max, int item_tail,
+                                                       int32_t* __restrict__ item_info) {
   __shared__ int sh[32];
   const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_V;
   int loc[SCAN_V], v = 0;
@@ -451,13 +463,23 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_apply(const int32_t* __restrict
     loc[k] = base + k < n ? in[base + k] : 0;
     v += loc[k];
   }
-  int total;
-  int run = block_excl_scan(v, sh, total) + offs[blockIdx.x];
+  int before = 0, total;
+  if (tops) {
+    block_excl_scan((int)threadIdx.x < (int)blockIdx.x ? sums[threadIdx.x] : 0, sh, before);
+  } else {
+    before = sums[blockIdx.x];
+  }
+  int run = block_excl_scan(v, sh, total) + before;
 #pragma unroll
   for (int k = 0; k < SCAN_V; ++k) {
     if (base + k < n) out[base + k] = run;
     run += loc[k];
   }
+  if (tops && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = before + total;
+  int c = v;
+#pragma unroll
+  for (int k = 8; k; k >>= 1) c += __shfl_xor_sync(0xffffffffu, c, k);
+  if ((threadIdx.x & 15) == 0 && c > 0) count_items(c, item_max, item_tail, (int)(base >> 6), item_info);
 }
 
 // Grouped records back to the order of their ids (record i to grouped
@@ -717,23 +739,25 @@ struct SimImpl final : SimBase {
     if (s->P.sparse) return sort_sparse(st);
     aq_sim* S_ = s;
     const int64_t n = S_->n;
-    AQ_CUDA_TRY(cudaMemsetAsync(S_->cell_count, 0, sizeof(int32_t) * S_->nkeys, st));
-    AQ_CUDA_TRY(cudaMemsetAsync(S_->n_items, 0, sizeof(int32_t) * (1 + 2 * IB), st));
+    // the cells' counts and the items' (they lie next to each other)
+    AQ_CUDA_TRY(cudaMemsetAsync(S_->cell_count, 0,
+                                (size_t)((char*)(S_->n_items + 1 + 2 * IB) - (char*)S_->cell_count), st));
     k_bin<D, R><<<grid_for(n, 256), 256, 0, st>>>(S_->L, K, S_->words[S_->cur], n, S_->keys, S_->ranks, S_->cell_count,
                                                   S_->status);
     const int nt = (int)((S_->nkeys + SCAN_TILE - 1) / SCAN_TILE);
     k_scan_sums<<<nt, SCAN_T, 0, st>>>(S_->cell_count, S_->nkeys, S_->scan_sums);
-    k_scan_top<<<1, SCAN_T, 0, st>>>(S_->scan_sums, nt, S_->cell_start, S_->nkeys);
-    k_scan_apply<<<nt, SCAN_T, 0, st>>>(S_->cell_count, S_->nkeys, S_->scan_sums, S_->cell_start);
+    const int im = item_max(), it = item_tail();
+    const int tops = nt <= SCAN_TOPS;
+    if (!tops) k_scan_top<<<1, SCAN_T, 0, st>>>(S_->scan_sums, nt, S_->cell_start, S_->nkeys);
+    k_scan_apply<<<nt, SCAN_T, 0, st>>>(S_->cell_count, S_->nkeys, S_->scan_sums, tops, S_->cell_start, im, it,
+                                        S_->n_items);
     const int nxt = 1 - S_->cur;
     k_scatter<<<grid_for(n, SCATTER_T), SCATTER_T, 0, st>>>(S_->words[S_->cur], S_->pid[S_->cur], S_->words[nxt], S_->pid[nxt],
                                                 S_->keys, S_->ranks, S_->cell_start, n, S_->W);
-    const int im = item_max(), it = item_tail();
-    k_items_count<<<grid_for(S_->nblk, 256), 256, 0, st>>>(S_->cell_start, S_->nblk, im, it, S_->n_items);
     k_items<<<grid_for(S_->nblk, 256), 256, 0, st>>>(S_->cell_start, S_->nblk, im, it, S_->items, S_->n_items, nullptr);
     AQ_CUDA_TRY(cudaGetLastError());
     S_->cur = nxt;
-    S_->launches += 7;
+    S_->launches += tops ? 5 : 6;
     S_->since_sort = 0;
     S_->sorted = true;
     return AQ_OK;
@@ -1339,11 +1363,12 @@ int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
     alloc(&s->grid[0], rsz * 4 * s->ncell);
     alloc(&s->grid[1], rsz * 4 * s->ncell);
     alloc((void**)&s->cell_count, sizeof(int32_t) * s->nkeys);
+    alloc((void**)&s->n_items, sizeof(int32_t) * (1 + 2 * IB));  // right behind: cleared together (sort)
     alloc((void**)&s->cell_start, sizeof(int32_t) * (s->nkeys + 1));
     alloc((void**)&s->scan_sums, sizeof(int32_t) * (nt + 1));
   }
   alloc((void**)&s->items, sizeof(int4) * s->max_items);
-  alloc((void**)&s->n_items, sizeof(int32_t) * (1 + 2 * IB));
+  if (P->sparse) alloc((void**)&s->n_items, sizeof(int32_t) * (1 + 2 * IB));
   alloc((void**)&s->sync, sizeof(int32_t) * (AQ_SYNC_WORDS + 2));
   alloc((void**)&s->status, sizeof(unsigned));
   alloc((void**)&s->fallbacks, sizeof(unsigned long long));
