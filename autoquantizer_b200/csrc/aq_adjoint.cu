@@ -615,14 +615,6 @@ __device__ __forceinline__ void ad_scatter(const AdK<R>& K, bool on, const int (
   }
 }
 
-// Launched while the kernel before it in the stream may still run (launch_pdl):
-// everything before this is the launch itself, nothing of the other kernel's
-// is touched; the kernel after may in turn start being launched.
-__device__ __forceinline__ void ad_begin() {
-  asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // zero a grid for a later scatter (grid-stride over its nodes)
 template <class R4>
 __device__ __forceinline__ void ad_clear(R4* g, int64_t nodes) {
@@ -669,7 +661,7 @@ __global__ void __launch_bounds__(AD_T) k_ad_pass(const __grid_constant__ AdK<R>
   constexpr int NS = S::NS;
   __shared__ __align__(16) R4 tiles[AD_T / 32][AdTile<D>::N];
   R4* const tile = tiles[threadIdx.x >> 5];
-  ad_begin();
+  kernel_begin();
   ad_clear(gclr, nodes);
   const int64_t p = (int64_t)blockIdx.x * AD_T + threadIdx.x;
   const bool on = p < n;
@@ -764,7 +756,7 @@ __global__ void __launch_bounds__(AD_T) k_ad_g2p_bwd(const __grid_constant__ AdK
   extern __shared__ __align__(16) unsigned char ad_smem[];
   R4* const tile = reinterpret_cast<R4*>(ad_smem) + (threadIdx.x >> 5) * 2 * AdTile<D>::N;
   R4* const stile = tile + AdTile<D>::N;
-  ad_begin();
+  kernel_begin();
   ad_clear(gclr, nodes);
   const int64_t p = (int64_t)blockIdx.x * AD_T + threadIdx.x;
   const bool on = p < n;
@@ -893,7 +885,7 @@ __global__ void __launch_bounds__(AD_T) k_ad_p2g_bwd(const __grid_constant__ AdK
   constexpr int NS = S::NS;
   __shared__ __align__(16) R4 tiles[AD_T / 32][AdTile<D>::N];
   R4* const tile = tiles[threadIdx.x >> 5];
-  ad_begin();
+  kernel_begin();
   const int64_t p = (int64_t)blockIdx.x * AD_T + threadIdx.x;
   const bool on = p < n;
   R s[NS], bi[NS];

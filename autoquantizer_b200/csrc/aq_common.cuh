@@ -39,21 +39,28 @@ inline int num_sms() {
 }
 
 // Launch a kernel that waits for the one before it in the stream by itself
-// (griddepcontrol.wait ahead of its first global access), so that its launch
+// (kernel_begin, ahead of its first global access), so that its launch
 // overlaps that one's end.
+struct PdlConfig {
+  cudaLaunchAttribute at;
+  cudaLaunchConfig_t c;
+  PdlConfig(unsigned grid, unsigned block, size_t smem, cudaStream_t st) : c() {
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+  }
+  PdlConfig(const PdlConfig&) = delete;
+};
+
 template <class... P, class... A>
 inline cudaError_t launch_pdl(void (*f)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t c = {};
-  c.gridDim = dim3(grid);
-  c.blockDim = dim3(block);
-  c.dynamicSmemBytes = smem;
-  c.stream = st;
-  c.attrs = &at;
-  c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, f, P(args)...);
+  const PdlConfig c(grid, block, smem, st);
+  return cudaLaunchKernelEx(&c.c, f, P(args)...);
 }
 
 inline unsigned grid_for(int64_t n, int threads) {

@@ -49,10 +49,9 @@ struct Nvrtc {
 struct Driver {
   CUresult (*load)(CUmodule*, const void*) = nullptr;
   CUresult (*getfn)(CUfunction*, CUmodule, const char*) = nullptr;
-  CUresult (*launch)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream,
-                     void**, void**) = nullptr;
   CUresult (*launch_coop)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream,
                           void**) = nullptr;
+  CUresult (*launch_ex)(const CUlaunchConfig*, CUfunction, void**, void**) = nullptr;
   CUresult (*setattr)(CUfunction, CUfunction_attribute, int) = nullptr;
   CUresult (*occ)(int*, CUfunction, int, size_t) = nullptr;
   bool ok = false;
@@ -96,7 +95,7 @@ void init_once() {
               sym(g_nv.h, "nvrtcGetLoweredName", g_nv.lowered) && sym(g_nv.h, "nvrtcDestroyProgram", g_nv.destroy);
   }
   g_dr.ok = drv("cuModuleLoadData", g_dr.load) && drv("cuModuleGetFunction", g_dr.getfn) &&
-            drv("cuLaunchKernel", g_dr.launch) && drv("cuLaunchCooperativeKernel", g_dr.launch_coop) && drv("cuFuncSetAttribute", g_dr.setattr) &&
+            drv("cuLaunchKernelEx", g_dr.launch_ex) && drv("cuLaunchCooperativeKernel", g_dr.launch_coop) && drv("cuFuncSetAttribute", g_dr.setattr) &&
             drv("cuOccupancyMaxActiveBlocksPerMultiprocessor", g_dr.occ);
 }
 
@@ -244,10 +243,21 @@ int jit_occupancy(void* fn, int block, size_t smem, int* out) {
 }
 
 int jit_launch(void* fn, unsigned grid, unsigned block, size_t smem, cudaStream_t st, void** args) {
-  return g_dr.launch((CUfunction)fn, grid, 1, 1, block, 1, 1, (unsigned)smem, (CUstream)st, args, nullptr) ==
-                 CUDA_SUCCESS
-             ? AQ_OK
-             : AQ_E_CUDA;
+  CUlaunchAttribute at;
+  memset(&at, 0, sizeof(at));
+  at.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+  at.value.programmaticStreamSerializationAllowed = 1;
+  CUlaunchConfig c;
+  memset(&c, 0, sizeof(c));
+  c.gridDimX = grid;
+  c.gridDimY = c.gridDimZ = 1;
+  c.blockDimX = block;
+  c.blockDimY = c.blockDimZ = 1;
+  c.sharedMemBytes = (unsigned)smem;
+  c.hStream = (CUstream)st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return g_dr.launch_ex(&c, (CUfunction)fn, args, nullptr) == CUDA_SUCCESS ? AQ_OK : AQ_E_CUDA;
 }
 
 int jit_launch_cooperative(void* fn, unsigned grid, unsigned block, size_t smem, cudaStream_t st, void** args) {

@@ -45,6 +45,7 @@ inline int jit_min_blocks(const aq_layout& L, int D, bool multi) {
 }
 int jit_set_smem(void* fn, int bytes);
 int jit_occupancy(void* fn, int block, size_t smem, int* out);
+// launched while the kernel before it in the stream ends (the kernel waits, kernel_begin)
 int jit_launch(void* fn, unsigned grid, unsigned block, size_t smem, cudaStream_t st, void** args);
 // the same with every CTA resident at once (kernels with a grid barrier)
 int jit_launch_cooperative(void* fn, unsigned grid, unsigned block, size_t smem, cudaStream_t st, void** args);

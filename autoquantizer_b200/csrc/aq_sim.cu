@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(256) k_bin(const __grid_constant__ aq_layout L
                                              const uint64_t* __restrict__ words, int64_t n,
                                              int32_t* __restrict__ keys, int32_t* __restrict__ ranks,
                                              int32_t* __restrict__ cell_count, unsigned* __restrict__ status) {
+  kernel_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const GRec w{words, i, K.W};
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(SCATTER_T) k_scatter(const uint64_t* __restric
                                                        int32_t* __restrict__ pout, const int32_t* __restrict__ keys,
                                                        const int32_t* __restrict__ ranks,
                                                        const int32_t* __restrict__ start, int64_t n, int W) {
+  kernel_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t i0 = (int64_t)blockIdx.x * SCATTER_T + warp * 32;  // first record of a group
   const int64_t i = i0 + lane;
@@ -178,6 +180,7 @@ __global__ void k_items_count(const int32_t* __restrict__ start, int nblk, int i
 __global__ void k_items(const int32_t* __restrict__ start, int nblk, int item_max, int item_tail,
                         int4* __restrict__ items, int32_t* __restrict__ item_info, const int32_t* __restrict__ blk_of) {
   __shared__ int off[IB];
+  kernel_begin();
   if (threadIdx.x == 0) {
     int acc = 0;
     for (int k = 0; k < IB; ++k) {
@@ -417,6 +420,7 @@ __device__ __forceinline__ int block_excl_scan(int v, int* sh, int& total) {
 __global__ void __launch_bounds__(SCAN_T) k_scan_sums(const int32_t* __restrict__ in, int64_t n,
                                                       int32_t* __restrict__ sums) {
   __shared__ int sh[32];
+  kernel_begin();
   const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_V;
   int v = 0;
 #pragma unroll
@@ -429,6 +433,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_sums(const int32_t* __restrict_
 __global__ void __launch_bounds__(SCAN_T) k_scan_top(int32_t* __restrict__ sums, int nt, int32_t* __restrict__ out,
                                                      int64_t n) {
   __shared__ int sh[32];
+  kernel_begin();
   const int per = (nt + SCAN_T - 1) / SCAN_T;
   const int b = threadIdx.x * per;
   int v = 0;
@@ -456,6 +461,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_apply(const int32_t* __restrict
                                                        int32_t* __restrict__ out, int item_max, int item_tail,
                                                        int32_t* __restrict__ item_info) {
   __shared__ int sh[32];
+  kernel_begin();
   const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_V;
   int loc[SCAN_V], v = 0;
 #pragma unroll
@@ -742,20 +748,18 @@ struct SimImpl final : SimBase {
     // the cells' counts and the items' (they lie next to each other)
     AQ_CUDA_TRY(cudaMemsetAsync(S_->cell_count, 0,
                                 (size_t)((char*)(S_->n_items + 1 + 2 * IB) - (char*)S_->cell_count), st));
-    k_bin<D, R><<<grid_for(n, 256), 256, 0, st>>>(S_->L, K, S_->words[S_->cur], n, S_->keys, S_->ranks, S_->cell_count,
-                                                  S_->status);
-    const int nt = (int)((S_->nkeys + SCAN_TILE - 1) / SCAN_TILE);
-    k_scan_sums<<<nt, SCAN_T, 0, st>>>(S_->cell_count, S_->nkeys, S_->scan_sums);
-    const int im = item_max(), it = item_tail();
-    const int tops = nt <= SCAN_TOPS;
-    if (!tops) k_scan_top<<<1, SCAN_T, 0, st>>>(S_->scan_sums, nt, S_->cell_start, S_->nkeys);
-    k_scan_apply<<<nt, SCAN_T, 0, st>>>(S_->cell_count, S_->nkeys, S_->scan_sums, tops, S_->cell_start, im, it,
-                                        S_->n_items);
-    const int nxt = 1 - S_->cur;
-    k_scatter<<<grid_for(n, SCATTER_T), SCATTER_T, 0, st>>>(S_->words[S_->cur], S_->pid[S_->cur], S_->words[nxt], S_->pid[nxt],
-                                                S_->keys, S_->ranks, S_->cell_start, n, S_->W);
-    k_items<<<grid_for(S_->nblk, 256), 256, 0, st>>>(S_->cell_start, S_->nblk, im, it, S_->items, S_->n_items, nullptr);
-    AQ_CUDA_TRY(cudaGetLastError());
+    const int nt = (int)((S_->nkeys + SCAN_TILE - 1) / SCAN_TILE), nxt = 1 - S_->cur;
+    const int im = item_max(), it = item_tail(), tops = nt <= SCAN_TOPS;
+    AQ_CUDA_TRY(launch_pdl(k_bin<D, R>, grid_for(n, 256), 256, 0, st, S_->L, K, S_->words[S_->cur], n, S_->keys,
+                           S_->ranks, S_->cell_count, S_->status));
+    AQ_CUDA_TRY(launch_pdl(k_scan_sums, nt, SCAN_T, 0, st, S_->cell_count, S_->nkeys, S_->scan_sums));
+    if (!tops) AQ_CUDA_TRY(launch_pdl(k_scan_top, 1, SCAN_T, 0, st, S_->scan_sums, nt, S_->cell_start, S_->nkeys));
+    AQ_CUDA_TRY(launch_pdl(k_scan_apply, nt, SCAN_T, 0, st, S_->cell_count, S_->nkeys, S_->scan_sums, tops,
+                           S_->cell_start, im, it, S_->n_items));
+    AQ_CUDA_TRY(launch_pdl(k_scatter, grid_for(n, SCATTER_T), SCATTER_T, 0, st, S_->words[S_->cur], S_->pid[S_->cur],
+                           S_->words[nxt], S_->pid[nxt], S_->keys, S_->ranks, S_->cell_start, n, S_->W));
+    AQ_CUDA_TRY(launch_pdl(k_items, grid_for(S_->nblk, 256), 256, 0, st, S_->cell_start, S_->nblk, im, it, S_->items,
+                           S_->n_items, nullptr));
     S_->cur = nxt;
     S_->launches += tops ? 5 : 6;
     S_->since_sort = 0;
@@ -967,7 +971,8 @@ struct SimImpl final : SimBase {
     } else {
       const void* f = S_->P.sparse ? (const void*)k_step<D, HF, HM, R, RtLayout, true, true>
                                    : (const void*)k_step<D, HF, HM, R, RtLayout>;
-      AQ_CUDA_TRY(cudaLaunchKernel(f, dim3(ctas), dim3(CH), args, S_->step_smem, st));
+      const PdlConfig c(ctas, CH, S_->step_smem, st);
+      AQ_CUDA_TRY(cudaLaunchKernelExC(&c.c, f, args));
     }
     if (prof) {
       AQ_CUDA_TRY(cudaEventRecord(S_->prof_ev[0][2 * S_->prof_n[0]++ + 1], st));
