@@ -33,11 +33,12 @@ inline bool jit_reg_record(const aq_layout& L) { return L.n_words <= kJitRegReco
 // (MULTI) run one warp's work per scheduler or little more, so registers
 // count and warps do not: 128 a thread (2D, 65,536 quantized: 480 -> 424 us a
 // frame of 32 substeps against 80 registers; 3D, 20,000: 730 -> 695).  Else
-// short records take 80 registers in 3D (12 CTAs; 11 and 14 within 1 %, 9 and
-// 10 2 to 4 % slower at 2,097,152 particles) and 73 in 2D (14; 300,000: 936
+// short records are budgeted for 11 CTAs in 3D (254 us a substep of 2,097,152
+// quantized particles at rest, 261 with 12, 262 with 13: of the bench layout
+// ptxas still makes 80 registers, with fewer spills, and 12 CTAs fit) and 73 in 2D (14; 300,000: 936
 // -> 829 us against 12), long ones 113 (9; 262,144 to 1,200,000 FP32
 // particles: +1.5 to -4 % against 8).
-constexpr int kJitShortRecordMinBlocks = 768 / AQ_CH;
+constexpr int kJitShortRecordMinBlocks = 704 / AQ_CH;
 inline int jit_min_blocks(const aq_layout& L, int D, bool multi) {
   if (multi) return 512 / AQ_CH;
   if (L.n_words > kJitRegRecordMaxWords) return 576 / AQ_CH;

@@ -522,19 +522,28 @@ __device__ __forceinline__ R bspline_w(R fx, int o) {
   return o == 0 ? a : (o == 1 ? b : c);
 }
 
-// G2P sums of lane src's particle (base, fx: each lane's own): part[d] = sum
-// w g_d, part[D + d D + e] = sum w g_d off_e, in every lane.
+// Out of line, with the particle handed over in shared memory, so that the
+// unit loop pays neither registers nor instruction cache for them (inlined:
+// 2,097,152 quantized particles at rest, where few leave their tiles, 4.5 %
+// slower).
+
+// values of a particle in a warp's scratch: base, fx, then q and Aff or, from
+// gather_outside, the sums
+constexpr int OUTSIDE_WORDS = 18;
+
+// G2P sums of the particle in sc (base, fx), every lane calling: sc[6 + d] =
+// sum w g_d, sc[6 + D + d D + e] = sum w g_d off_e.
 template <int D, class R, bool COL, bool SP, class R4>
-__device__ __forceinline__ void gather_outside(const SimK<R>& K, const ColPose<R>& pose, const R4* gin, int src,
-                                               int lane, const int (&base)[3], const R (&fx)[3], R (&part)[D + D * D]) {
+static __device__ __noinline__ void gather_outside(const SimK<R>& K, const ColPose<R>& pose, const R4* gin, R* sc) {
   constexpr int NN = D == 3 ? 27 : 9;
+  const int lane = threadIdx.x & 31;
   const int off[3] = {D == 3 ? lane / 9 : lane / 3, D == 3 ? (lane / 3) % 3 : lane % 3, D == 3 ? lane % 3 : 0};
   int n[3] = {0, 0, 0};
   R weight = 1;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    n[d] = __shfl_sync(0xffffffffu, base[d], src) + off[d];
-    weight *= bspline_w<R>(__shfl_sync(0xffffffffu, fx[d], src), off[d]);
+    n[d] = (int)sc[d] + off[d];
+    weight *= bspline_w<R>(sc[3 + d], off[d]);
   }
   R4 g;
   g.x = g.y = g.z = g.w = 0;
@@ -548,6 +557,7 @@ __device__ __forceinline__ void gather_outside(const SimK<R>& K, const ColPose<R
     g = grid_op_node<D, R, COL>(K, pose, g, n[0], n[1], n[2]);
   }
   const R gv[3] = {g.y, g.z, g.w};
+  R part[D + D * D];
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     const R wg = lane < NN ? weight * gv[d] : (R)0;
@@ -556,34 +566,38 @@ __device__ __forceinline__ void gather_outside(const SimK<R>& K, const ColPose<R
     for (int e = 0; e < D; ++e) part[D + d * D + e] = (R)off[e] * wg;
   }
 #pragma unroll
-  for (int k = 0; k < D + D * D; ++k)
+  for (int k = 0; k < D + D * D; ++k) {
 #pragma unroll
     for (int m = 16; m; m >>= 1) part[k] += __shfl_xor_sync(0xffffffffu, part[k], m);
+    if (lane == k) sc[6 + k] = part[k];
+  }
+  __syncwarp();
 }
 
-// P2G of lane src's particle into the global grid: node value w (m, q + Aff off)
+// P2G of the particle in sc (base, fx, q, Aff) into the global grid, every
+// lane calling: node value w (m, q + Aff off).  Returns status flags.
 template <int D, class R, bool SP, class R4>
-__device__ __forceinline__ void scatter_outside(const SimK<R>& K, R4* gout, int src, int lane,
-                                             const int (&base)[3], const R (&fx)[3], const R (&q)[D],
-                                             const R (&Aff)[D * D], unsigned& fl) {
+static __device__ __noinline__ unsigned scatter_outside(const SimK<R>& K, R4* gout, const R* sc) {
   constexpr int BS = Geo<D>::BS, NN = D == 3 ? 27 : 9;
+  const int lane = threadIdx.x & 31;
   const int off[3] = {D == 3 ? lane / 9 : lane / 3, D == 3 ? (lane / 3) % 3 : lane % 3, D == 3 ? lane % 3 : 0};
   int b[3] = {0, 0, 0}, n[3] = {0, 0, 0};
   R weight = 1;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    b[d] = __shfl_sync(0xffffffffu, base[d], src);
+    b[d] = (int)sc[d];
     n[d] = b[d] + off[d];
-    weight *= bspline_w<R>(__shfl_sync(0xffffffffu, fx[d], src), off[d]);
+    weight *= bspline_w<R>(sc[3 + d], off[d]);
   }
   R mv[3] = {0, 0, 0};
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    R s = __shfl_sync(0xffffffffu, q[d], src);
+    R s = sc[6 + d];
 #pragma unroll
-    for (int e = 0; e < D; ++e) s += (R)off[e] * __shfl_sync(0xffffffffu, Aff[d * D + e], src);
+    for (int e = 0; e < D; ++e) s += (R)off[e] * sc[6 + D + d * D + e];
     mv[d] = weight * s;
   }
+  unsigned fl = 0;
   if (SP) {
     // slots of the (at most 2^D) blocks under the stencil, lane qb claims block qb's
     const int f0 = b[0] / BS, f1 = b[1] / BS, f2 = D == 3 ? b[2] / BS : 0;
@@ -605,6 +619,8 @@ __device__ __forceinline__ void scatter_outside(const SimK<R>& K, R4* gout, int 
   } else if (lane < NN) {
     red_add_node(gout + cell_index<D>(K.res, n[0], n[1], n[2]), weight * K.p_mass, mv[0], mv[1], mv[2]);
   }
+  __syncwarp();
+  return fl;
 }
 
 // Kernels that may be launched while the kernel before them in the stream
@@ -679,6 +695,7 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
   R4* gtile = reinterpret_cast<R4*>(smem_raw);                      // TNP nodes (m, v): G2P source
   R4* ptile = gtile + TNP;                                     // NWARP x TNP (m, m v): P2G, per warp
   uint64_t* srec = reinterpret_cast<uint64_t*>(ptile + NWARP * TNP);  // CH x WS: each thread's record (RtLayout)
+  __shared__ R s_out[NWARP][OUTSIDE_WORDS];  // a particle outside its tile (gather_outside)
   __shared__ int sbox[6];  // tile-coordinate box of the item's P2G base cells (min[3], max[3])
   // MULTI: this pass's G2P source, P2G target and dithering key (in shared
   // memory: held in registers over the whole unit loop they spill)
@@ -767,10 +784,11 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
       __syncthreads();
     }
     // stage the grid tile (m, v after grid_op), three loads of a thread in
-    // flight at a time (one: 2 to 6 % slower; all six of 3D: 5 % slower where
-    // registers are short)
+    // flight at a time (one: 2 to 6 % slower), but one where registers are
+    // scarce (3D, short records: 262 -> 260 us a substep at rest, 10.24 ->
+    // 10.10 ms a frame in motion, 2,097,152 particles)
     if (do_g2p) {
-      constexpr int NL = 3;
+      constexpr int NL = D == 3 && LA::kMinBlocks * CH > 640 ? 1 : 3;
 #pragma unroll 1
       for (int jb = tid; jb < TNP; jb += NL * CH) {
       R4 gv[NL];
@@ -911,18 +929,26 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
         // half the units had such a lane.)
         #pragma unroll 1
         for (unsigned om = __ballot_sync(0xffffffffu, active && !in_tile); om; om &= om - 1) {
-          const int src = __ffs(om) - 1;
-          R part[D + D * D];
-          gather_outside<D, R, COL, SP>(K, pose, AQ_GIN, src, lane, base, fx, part);
-          if (lane == src) {
+          R* const sc = s_out[warp];
+          if (lane == __ffs(om) - 1) {
             ++nfall;
 #pragma unroll
             for (int d = 0; d < D; ++d) {
-              nv[d] = part[d];
-#pragma unroll
-              for (int e = 0; e < D; ++e) Sm[d][e] = part[D + d * D + e];
+              sc[d] = (R)base[d];
+              sc[3 + d] = fx[d];
             }
           }
+          __syncwarp();
+          gather_outside<D, R, COL, SP>(K, pose, AQ_GIN, sc);
+          if (lane == __ffs(om) - 1) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+              nv[d] = sc[6 + d];
+#pragma unroll
+              for (int e = 0; e < D; ++e) Sm[d][e] = sc[6 + D + d * D + e];
+            }
+          }
+          __syncwarp();
         }
         if (active) {
         // new_C = 4 inv_dx sum w g_v (off - fx)^T;  new_x = x + dt new_v
@@ -1106,8 +1132,21 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
         }
         // lanes outside the tile: straight to the global grid, a lane per node
 #pragma unroll 1
-        for (unsigned om = __ballot_sync(0xffffffffu, active && !in_tile); om; om &= om - 1)
-          scatter_outside<D, R, SP>(K, AQ_GOUT, __ffs(om) - 1, lane, base, fx, q, Aff, fl);
+        for (unsigned om = __ballot_sync(0xffffffffu, active && !in_tile); om; om &= om - 1) {
+          R* const sc = s_out[warp];
+          if (lane == __ffs(om) - 1) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+              sc[d] = (R)base[d];
+              sc[3 + d] = fx[d];
+              sc[6 + d] = q[d];
+#pragma unroll
+              for (int e = 0; e < D; ++e) sc[6 + D + d * D + e] = Aff[d * D + e];
+            }
+          }
+          __syncwarp();
+          fl |= scatter_outside<D, R, SP>(K, AQ_GOUT, sc);
+        }
         __syncwarp();
       }
     }  // units
