@@ -1052,6 +1052,7 @@ struct aq_adjoint {
   std::vector<void*> ckpt;  // states at multiples of the checkpoint interval (every > 0), or the initial state
   std::vector<void*> seg;   // states between two checkpoints; two ping-pong states (every == 0)
   std::vector<void*> stash;  // bisection checkpointing: one state per recursion level, plus a scratch state
+  std::vector<void*> ab;     // the adjoints of two states, of the backward pass
   int T = 0, every = 0;
   int seg_of = -1;           // the segment whose states seg holds
   int32_t* perm = nullptr;  // sorted position -> caller's particle index (length n)
@@ -1271,7 +1272,7 @@ static AdBase* make_ad(aq_adjoint* a) {
 static void free_ad(aq_adjoint* a) {
   if (!a) return;
   delete a->impl;
-  for (auto* v : {&a->ckpt, &a->seg, &a->stash})
+  for (auto* v : {&a->ckpt, &a->seg, &a->stash, &a->ab})
     for (void* p : *v) pool_free(p, 0);
   pool_free(a->perm, 0);
   for (void* p : a->g) pool_free(p, 0);
@@ -1407,15 +1408,8 @@ int aq_adjoint_backward(aq_adjoint* a, const void* d_seed, void* d_grad_s0, doub
   while ((1 << levels) < T) ++levels;
   // one stash per level, the last one is scratch
   if (every == 0 && (rc = ad_buffers(a, a->stash, levels + 1, st))) return rc;
-  void* ab[2] = {nullptr, nullptr};
-  for (void*& p : ab) {
-    const cudaError_t e = pool_alloc(&p, a->state_bytes(), st);
-    if (e != cudaSuccess) {
-      pool_free(ab[0], st);
-      set_last_cuda_error(e, "cudaMallocFromPoolAsync");
-      return AQ_E_CUDA;
-    }
-  }
+  if ((rc = ad_buffers(a, a->ab, 2, st))) return rc;
+  void** ab = a->ab.data();
   rc = a->impl->permute(d_seed, ab[0], true, st);  // into the order of the forward pass
   const size_t sens_bytes = sizeof(double) * AD_SENS_COPIES * a->NS;
   if (rc == AQ_OK && cudaMemsetAsync(a->dsens, 0, sens_bytes, st) != cudaSuccess) rc = AQ_E_CUDA;
@@ -1445,8 +1439,6 @@ int aq_adjoint_backward(aq_adjoint* a, const void* d_seed, void* d_grad_s0, doub
   std::vector<double> part((size_t)AD_SENS_COPIES * a->NS);
   cudaError_t e = cudaSuccess;
   if (rc == AQ_OK && h_sens) e = cudaMemcpyAsync(part.data(), a->dsens, sens_bytes, cudaMemcpyDeviceToHost, st);
-  pool_free(ab[0], st);
-  pool_free(ab[1], st);
   const cudaError_t es = cudaStreamSynchronize(st);
   if (e == cudaSuccess) e = es;
   if (e != cudaSuccess) set_last_cuda_error(e, "aq_adjoint_backward");

@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <unordered_map>
 
 #include "aq_codec.cuh"
 #include "aq_common.cuh"
@@ -22,7 +23,9 @@ void set_last_cuda_error(cudaError_t e, const char* what) {
 //
 // Simulators, adjoints and the scratch of single calls take their memory
 // from one pool per device.  The pool keeps up to POOL_KEEP bytes that were
-// given back (the driver's own default keeps none past the next
+// given back beyond what is in use (the release threshold counts both, so it
+// follows: with 1.4 GB in use and a threshold of 1 GiB, each call's scratch was
+// unmapped and mapped again; the driver's own default keeps none past the next
 // synchronization, and mapping memory anew took 0.1 to 10 ms an allocation,
 // more than the work of small calls), and gives back everything it can when
 // an allocation fails.  The driver's pool is safe for several threads and
@@ -32,6 +35,20 @@ constexpr int POOL_DEVICES = 64;
 
 static std::mutex g_pool_mu;
 static cudaMemPool_t g_pool[POOL_DEVICES];
+struct PoolBlock {
+  cudaMemPool_t pool;
+  size_t bytes;
+};
+static std::unordered_map<void*, PoolBlock> g_pool_live;
+static std::unordered_map<cudaMemPool_t, uint64_t> g_pool_used;
+
+// `by` more (or fewer) bytes in use in a pool; g_pool_mu held
+static void pool_count(cudaMemPool_t pool, int64_t by) {
+  uint64_t& used = g_pool_used[pool];
+  used += by;
+  uint64_t keep = used + POOL_KEEP;
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
 
 static cudaError_t pool_of(cudaMemPool_t* out) {
   int dev = 0;
@@ -47,8 +64,6 @@ static cudaError_t pool_of(cudaMemPool_t* out) {
     props.location.id = dev;
     cudaMemPool_t p;
     if ((e = cudaMemPoolCreate(&p, &props)) != cudaSuccess) return e;
-    uint64_t keep = POOL_KEEP;
-    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
     g_pool[dev] = p;
   }
   *out = g_pool[dev];
@@ -68,11 +83,25 @@ cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st) {
     e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, st);
     if (e != cudaSuccess) cudaGetLastError();
   }
+  if (e == cudaSuccess) {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    g_pool_live[*p] = PoolBlock{pool, bytes};
+    pool_count(pool, (int64_t)bytes);
+  }
   return e;
 }
 
 void pool_free(void* p, cudaStream_t st) {
-  if (p) cudaFreeAsync(p, st);
+  if (!p) return;
+  {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    const auto it = g_pool_live.find(p);
+    if (it != g_pool_live.end()) {
+      pool_count(it->second.pool, -(int64_t)it->second.bytes);
+      g_pool_live.erase(it);
+    }
+  }
+  cudaFreeAsync(p, st);
 }
 
 // ----------------------------------------------------------- state error
