@@ -242,7 +242,7 @@ __device__ __forceinline__ int64_t ad_at(int64_t p, int s) {
 }
 
 template <int NS, int LO, int HI, class R>
-__device__ __forceinline__ void ad_load(const R* __restrict__ st, int64_t p, R (&s)[NS]) {
+__device__ __forceinline__ void ad_load(const R* st, int64_t p, R (&s)[NS]) {
 #pragma unroll
   for (int k = LO; k < HI; ++k) s[k] = st[ad_at<NS>(p, k)];
 }
@@ -646,9 +646,9 @@ constexpr int AD_T = 64;
 // sums in gin) and / or P2G of the next (of the new state, or of `in`) into
 // gout, which is zero; gclr (may be null) is zeroed for the pass after.
 template <int D, bool HF, class R, bool G2P, bool P2G>
-__global__ void __launch_bounds__(AD_T) k_ad_pass(const __grid_constant__ AdK<R> K, const R* __restrict__ in,
-                                                  R* __restrict__ out, int64_t n,
-                                                  const typename R4T<R>::type* __restrict__ gin,
+__global__ void __launch_bounds__(AD_T) k_ad_pass(const __grid_constant__ AdK<R> K, const R* in,
+                                                  R* out, int64_t n,
+                                                  const typename R4T<R>::type* gin,
                                                   typename R4T<R>::type* gout, typename R4T<R>::type* gclr,
                                                   int64_t nodes) {
   typedef Sch<D, HF, false> S;
@@ -738,9 +738,9 @@ __global__ void __launch_bounds__(AD_T) k_ad_pass(const __grid_constant__ AdK<R>
 // vbar_i += w h, wbar_i = v_i . h, and through dpos
 // xbar -= 4/dx^2 w C'bar^T v_i.
 template <int D, bool HF, class R>
-__global__ void __launch_bounds__(AD_T) k_ad_g2p_bwd(const __grid_constant__ AdK<R> K, const R* __restrict__ st,
-                                                     const R* __restrict__ ab_out, R* __restrict__ ab_in, int64_t n,
-                                                     const typename R4T<R>::type* __restrict__ grid,
+__global__ void __launch_bounds__(AD_T) k_ad_g2p_bwd(const __grid_constant__ AdK<R> K, const R* st,
+                                                     const R* ab_out, R* ab_in, int64_t n,
+                                                     const typename R4T<R>::type* grid,
                                                      typename R4T<R>::type* gvb, typename R4T<R>::type* gclr,
                                                      int64_t nodes) {
   typedef Sch<D, HF, false> S;
@@ -889,11 +889,11 @@ constexpr int AD_SENS_COPIES = 32;  // copies of the sensitivity sums, so that C
 // P2G^T: the old state's adjoint, completed (ab_in holds G2P^T's part on
 // entry); with sens, its squares are added to the sensitivity sums in FP64.
 template <int D, bool HF, class R>
-__global__ void __launch_bounds__(AD_T) k_ad_p2g_bwd(const __grid_constant__ AdK<R> K, const R* __restrict__ st,
+__global__ void __launch_bounds__(AD_T) k_ad_p2g_bwd(const __grid_constant__ AdK<R> K, const R* st,
                                                      R* ab_in, int64_t n,
-                                                     const typename R4T<R>::type* __restrict__ grid,
-                                                     const typename R4T<R>::type* __restrict__ gvb,
-                                                     double* __restrict__ sens) {
+                                                     const typename R4T<R>::type* grid,
+                                                     const typename R4T<R>::type* gvb,
+                                                     double* sens) {
   typedef Sch<D, HF, false> S;
   typedef typename R4T<R>::type R4;
   constexpr int NS = S::NS;

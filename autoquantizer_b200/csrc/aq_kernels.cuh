@@ -629,6 +629,10 @@ static __device__ __noinline__ unsigned scatter_outside(const SimK<R>& K, R4* go
 // be launched in turn (k_step, whose CTAs stay, lets it at its end: earlier, the
 // next launch's CTAs settled unevenly where this one's had nothing to do,
 // 130,000 particles 7 % slower).  Without such a launch it does nothing.
+// What such a kernel reads may still be written while it waits, so its
+// pointers carry no __restrict__ and it reads with plain or __ldcg loads,
+// never __ldg: both promise memory that no one writes during the kernel, and
+// loads so marked may be moved ahead of the wait.
 __device__ __forceinline__ void kernel_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void kernel_let_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void kernel_begin() {
@@ -837,7 +841,7 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
       int32_t pid = 0;
       if (active) {  // grouped storage: the warp's 16-byte pair loads coalesce
         load_grec<LA::kWords>(A.words, rec, W, myrec);
-        pid = __ldg(A.pid + rec);
+        pid = A.pid[rec];
       }
       R vals[NS];
       if (active) {

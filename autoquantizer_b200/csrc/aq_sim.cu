@@ -33,9 +33,9 @@ namespace aq {
 
 template <int D, class R>
 __global__ void __launch_bounds__(256) k_bin(const __grid_constant__ aq_layout L, const SimK<R> K,
-                                             const uint64_t* __restrict__ words, int64_t n,
-                                             int32_t* __restrict__ keys, int32_t* __restrict__ ranks,
-                                             int32_t* __restrict__ cell_count, unsigned* __restrict__ status) {
+                                             const uint64_t* words, int64_t n,
+                                             int32_t* keys, int32_t* ranks,
+                                             int32_t* cell_count, unsigned* status) {
   kernel_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -71,17 +71,17 @@ __global__ void __launch_bounds__(256) k_bin(const __grid_constant__ aq_layout L
 // and writes each record's pairs to its destination as 16-byte vectors.
 constexpr int SCATTER_T = 128;
 
-__global__ void __launch_bounds__(SCATTER_T) k_scatter(const uint64_t* __restrict__ win,
-                                                       const int32_t* __restrict__ pin, uint64_t* __restrict__ wout,
-                                                       int32_t* __restrict__ pout, const int32_t* __restrict__ keys,
-                                                       const int32_t* __restrict__ ranks,
-                                                       const int32_t* __restrict__ start, int64_t n, int W) {
+__global__ void __launch_bounds__(SCATTER_T) k_scatter(const uint64_t* win,
+                                                       const int32_t* pin, uint64_t* wout,
+                                                       int32_t* pout, const int32_t* keys,
+                                                       const int32_t* ranks,
+                                                       const int32_t* start, int64_t n, int W) {
   kernel_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t i0 = (int64_t)blockIdx.x * SCATTER_T + warp * 32;  // first record of a group
   const int64_t i = i0 + lane;
   if (i >= n) return;
-  const int32_t p = __ldg(pin + i);
+  const int32_t p = pin[i];
   const int key = keys[i];
   const int rk = ranks[i];  // rank of the record in its cell
   const int64_t c0 = (int64_t)(key >> 6) * 64;
@@ -99,9 +99,9 @@ __global__ void __launch_bounds__(SCATTER_T) k_scatter(const uint64_t* __restric
     // previous binning's block order): the warp builds mask_r rank by rank
     // from two cells per lane, one ballot pair per rank
     const int* sc = start + c0;
-    const int n_lo = __ldg(sc + lane + 1) - __ldg(sc + lane);
-    const int n_hi = __ldg(sc + lane + 33) - __ldg(sc + lane + 32);
-    b0 = __ldg(sc);
+    const int n_lo = sc[lane + 1] - sc[lane];
+    const int n_hi = sc[lane + 33] - sc[lane + 32];
+    b0 = sc[0];
     const int rmax = (int)__reduce_max_sync(am, (unsigned)rk);
     const unsigned long long below = (1ull << myc) - 1ull;
     int acc = 0;
@@ -116,11 +116,11 @@ __global__ void __launch_bounds__(SCATTER_T) k_scatter(const uint64_t* __restric
     // block's 65 offsets are read as int4 vectors (start is 256-byte
     // aligned, c0 a multiple of 64).
     const int4* st4 = reinterpret_cast<const int4*>(start + c0);
-    int4 v = __ldg(st4);
+    int4 v = st4[0];
     b0 = v.x;
 #pragma unroll 4
     for (int q = 0; q < 16; ++q) {
-      const int4 nv = q < 15 ? __ldg(st4 + q + 1) : make_int4(__ldg(start + c0 + 64), 0, 0, 0);
+      const int4 nv = q < 15 ? st4[q + 1] : make_int4(start[c0 + 64], 0, 0, 0);
       const int ss[5] = {v.x, v.y, v.z, v.w, nv.x};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -134,10 +134,16 @@ __global__ void __launch_bounds__(SCATTER_T) k_scatter(const uint64_t* __restric
   const uint64_t* g = win + i0 * W;  // the group's words (i0 is a multiple of 32)
   uint64_t* go = wout + (dst >> 5) * 32 * (int64_t)W;
   const int lo = (int)(dst & 31), W2 = W & ~1;
-  for (int k = 0; k < W2; k += 2)
-    *reinterpret_cast<ulonglong2*>(go + (k >> 1) * 64 + 2 * lo) =
-        __ldg(reinterpret_cast<const ulonglong2*>(g + (k >> 1) * 64 + 2 * lane));
-  if (W & 1) go[W2 * 32 + lo] = __ldg(g + W2 * 32 + lane);
+  for (int k0 = 0; k0 < W2; k0 += 8) {  // four pairs in flight
+    ulonglong2 t[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (k0 + 2 * j < W2) t[j] = *reinterpret_cast<const ulonglong2*>(g + ((k0 >> 1) + j) * 64 + 2 * lane);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (k0 + 2 * j < W2) *reinterpret_cast<ulonglong2*>(go + ((k0 >> 1) + j) * 64 + 2 * lo) = t[j];
+  }
+  if (W & 1) go[W2 * 32 + lo] = g[W2 * 32 + lane];
   pout[dst] = p;
 }
 
@@ -177,8 +183,8 @@ __global__ void k_items_count(const int32_t* __restrict__ start, int nblk, int i
 }
 
 // blk_of (sparse grids): the grid block of each compact block index, else null
-__global__ void k_items(const int32_t* __restrict__ start, int nblk, int item_max, int item_tail,
-                        int4* __restrict__ items, int32_t* __restrict__ item_info, const int32_t* __restrict__ blk_of) {
+__global__ void k_items(const int32_t* start, int nblk, int item_max, int item_tail,
+                        int4* items, int32_t* item_info, const int32_t* blk_of) {
   __shared__ int off[IB];
   kernel_begin();
   if (threadIdx.x == 0) {
@@ -417,8 +423,8 @@ __device__ __forceinline__ int block_excl_scan(int v, int* sh, int& total) {
   return r;
 }
 
-__global__ void __launch_bounds__(SCAN_T) k_scan_sums(const int32_t* __restrict__ in, int64_t n,
-                                                      int32_t* __restrict__ sums) {
+__global__ void __launch_bounds__(SCAN_T) k_scan_sums(const int32_t* in, int64_t n,
+                                                      int32_t* sums) {
   __shared__ int sh[32];
   kernel_begin();
   const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_V;
@@ -430,7 +436,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_sums(const int32_t* __restrict_
   if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(SCAN_T) k_scan_top(int32_t* __restrict__ sums, int nt, int32_t* __restrict__ out,
+__global__ void __launch_bounds__(SCAN_T) k_scan_top(int32_t* sums, int nt, int32_t* out,
                                                      int64_t n) {
   __shared__ int sh[32];
   kernel_begin();
@@ -456,10 +462,10 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_top(int32_t* __restrict__ sums,
 // 64 blocks (16 threads of 4 cells each).
 constexpr int SCAN_TOPS = 1024;
 
-__global__ void __launch_bounds__(SCAN_T) k_scan_apply(const int32_t* __restrict__ in, int64_t n,
-                                                       const int32_t* __restrict__ sums, int tops,
-                                                       int32_t* __restrict__ out, int item_max, int item_tail,
-                                                       int32_t* __restrict__ item_info) {
+__global__ void __launch_bounds__(SCAN_T) k_scan_apply(const int32_t* in, int64_t n,
+                                                       const int32_t* sums, int tops,
+                                                       int32_t* out, int item_max, int item_tail,
+                                                       int32_t* item_info) {
   __shared__ int sh[32];
   kernel_begin();
   const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_V;
