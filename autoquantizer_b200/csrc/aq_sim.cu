@@ -577,7 +577,11 @@ struct aq_sim {
   int32_t* pid[2] = {nullptr, nullptr};
   int cur = 0;
   void* grid[3] = {nullptr, nullptr, nullptr};  // [2]: null in a simulator that keeps two (THIRD_GRID_MAX)
-  int rot = 0;  // three grids: grid[rot] is zero and takes the next chain's first P2G
+  int rot = 0;  // three grids: grid[rot] is zero (unless stale) and takes the next chain's first P2G
+  // grid[rot] and k_step's claim counters are not known to be zero: a chain
+  // was captured into a graph (the host's picture is not the device's) or
+  // did not run to its end
+  bool stale = false;
   int64_t ncell = 0, nkeys = 0;
   int nblk = 0;
   int32_t *keys = nullptr, *ranks = nullptr, *cell_count = nullptr, *cell_start = nullptr, *scan_sums = nullptr;
@@ -1114,17 +1118,35 @@ struct SimImpl final : SimBase {
     s->col_height += s->col_rate * s->P.dt;
   }
 
+  // The first P2G target and the claim counters zeroed in stream order.
+  int reset_chain(cudaStream_t st) {
+    aq_sim* S_ = s;
+    typedef typename R4T<R>::type R4;
+    if (S_->grid[2])
+      AQ_CUDA_TRY(cudaMemsetAsync(S_->grid[S_->rot], 0,
+                                  sizeof(R4) * (S_->P.sparse ? (size_t)S_->pool_cap * 64 : (size_t)S_->ncell), st));
+    AQ_CUDA_TRY(cudaMemsetAsync(S_->sync + AQ_SYNC_WORDS, 0, 2 * sizeof(int32_t), st));
+    return AQ_OK;
+  }
+
   int substeps(int n, cudaStream_t st) override {
     aq_sim* S_ = s;
     if (S_->chunk) return stream_substeps(n, st);
     const int interval = S_->P.sort_interval < 1 ? 1 : S_->P.sort_interval;
     int rc;
+    // A captured chain is replayed on grids that other chains have used since
+    // (and from the same rot each time), so it clears its own first target.
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    AQ_CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
+    const bool captured = capturing != cudaStreamCaptureStatusNone;
     while (n > 0) {
       if (!S_->sorted || S_->since_sort >= interval) {
         if ((rc = sort(st))) return rc;
       }
       int m = interval - S_->since_sort;
       if (m > n) m = n;
+      if ((captured || S_->stale) && (rc = reset_chain(st))) return rc;
+      S_->stale = true;  // until the chain's last launch is queued
       // m + 1 passes: P2G of the first substep, G2P of each fused with P2G
       // of the next, G2P of the last (grid_op applied as tiles are staged)
       if (S_->grid[2]) {
@@ -1149,6 +1171,7 @@ struct SimImpl final : SimBase {
           advance();
         }
       }
+      S_->stale = captured;
       S_->since_sort += m;
       n -= m;
     }
