@@ -165,6 +165,8 @@ struct StepArgs {
   void* gnext;
   uint64_t sk;             // pass0's dithering key
   unsigned* status;
+  int32_t* stalled;        // host memory: set by a launch whose barrier ran out of time
+  long long wait_limit;    // cycles a CTA waits in the barrier, at most
   unsigned long long* fallbacks;
   double* rmax;
   double* rmin;
@@ -645,9 +647,11 @@ __device__ __forceinline__ void kernel_begin() {
 // last one of a round stores the round's number to sync[32], which the others
 // poll (in another cache line than the arrivals).  The fences order the
 // CTA's grid and record writes before it and its reads after it.  False when
-// the wait ran out of time (2^34 cycles, some 9 s), which no launch whose
-// CTAs are resident comes near.
-__device__ __forceinline__ bool grid_barrier(int32_t* sync, unsigned k) {
+// the wait took longer than `limit` cycles (AQ_WAIT_LIMIT: some 9 s), which no
+// launch whose CTAs are resident comes near.
+constexpr long long AQ_WAIT_LIMIT = 1ll << 34;
+
+__device__ __forceinline__ bool grid_barrier(int32_t* sync, unsigned k, long long limit) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -662,7 +666,7 @@ __device__ __forceinline__ bool grid_barrier(int32_t* sync, unsigned k) {
       for (;;) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(sync + 32) : "memory");
         if (seen >= k) break;
-        if (clock64() - t0 > (1ll << 34)) {
+        if (clock64() - t0 > limit) {
           ok = 0;
           break;
         }
@@ -1199,13 +1203,14 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
   }
 #undef AQ_GIN
 #undef AQ_GOUT
-  if (MULTI && pass + 1 < A.pass1 && !grid_barrier(A.sync, (unsigned)(pass + 1 - A.pass0))) {
+  if (MULTI && pass + 1 < A.pass1 && !grid_barrier(A.sync, (unsigned)(pass + 1 - A.pass0), A.wait_limit)) {
     fl |= AQ_ST_STALLED;
     break;
   }
   }  // passes
   kernel_let_next();
   if (fl) atomicOr(A.status, fl);
+  if (MULTI && (fl & AQ_ST_STALLED)) *reinterpret_cast<volatile int32_t*>(A.stalled) = 1;
   if (nfall) atomicAdd(A.fallbacks, (unsigned long long)nfall);
   if (A.ranges && tid < NS) {  // one merge per CTA and slot
     if (s_rmax[tid] != 0ull) atomic_max_d(A.rmax + tid, ord_val(s_rmax[tid]));

@@ -18,6 +18,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_run_length_encode.cuh>
 #include <cub/device/device_scan.cuh>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -554,6 +555,37 @@ __global__ void __launch_bounds__(256) k_loss(const __grid_constant__ aq_layout 
 
 // ------------------------------------------------------------------ host
 
+// One int of page-locked host memory per simulator, which a launch that gave
+// up waiting sets (StepArgs::stalled) and the host reads without a copy.
+// Handed out of pages of AQ_STALL_PAGE that are kept: mapping one takes longer
+// than all else in setting up a small simulator.
+constexpr int AQ_STALL_PAGE = 1024;
+static std::mutex g_stall_mu;
+static std::vector<int32_t*> g_stall_free;
+
+static int32_t* stall_word() {
+  std::lock_guard<std::mutex> g(g_stall_mu);
+  if (g_stall_free.empty()) {
+    int32_t* page = nullptr;
+    if (cudaHostAlloc((void**)&page, sizeof(int32_t) * AQ_STALL_PAGE, cudaHostAllocPortable | cudaHostAllocMapped) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    for (int k = AQ_STALL_PAGE - 1; k >= 0; --k) g_stall_free.push_back(page + k);
+  }
+  int32_t* w = g_stall_free.back();
+  g_stall_free.pop_back();
+  *w = 0;
+  return w;
+}
+
+static void stall_word_back(int32_t* w) {
+  if (!w) return;
+  std::lock_guard<std::mutex> g(g_stall_mu);
+  g_stall_free.push_back(w);
+}
+
 struct SimBase {
   virtual ~SimBase() {}
   virtual int substeps(int n, cudaStream_t st) = 0;
@@ -591,6 +623,8 @@ struct aq_sim {
   int64_t step_launches = 0;  // launches without MULTI
   int64_t max_items = 0;
   unsigned* status = nullptr;
+  int32_t* stalled = nullptr;  // host memory (stall_word)
+  long long wait_limit = aq::AQ_WAIT_LIMIT;
   unsigned long long* fallbacks = nullptr;
   double *rmax = nullptr, *rmin = nullptr;
   double* dloss = nullptr;
@@ -930,6 +964,8 @@ struct SimImpl final : SimBase {
     a.n_items = S_->n_items;
     a.sync = S_->sync;
     a.status = S_->status;
+    a.stalled = S_->stalled;
+    a.wait_limit = S_->wait_limit;
     a.fallbacks = S_->fallbacks;
     a.rmax = S_->rmax;
     a.rmin = S_->rmin;
@@ -1276,6 +1312,7 @@ static void free_sim(aq_sim* s) {
     pool_free(s->cub_tmp, 0);
   }
   pool_free(s->slab, 0);
+  stall_word_back(s->stalled);
   if (s->h_words) cudaFreeHost(s->h_words);
   if (s->words_dl) cudaFree(s->words_dl);
   if (s->words_up[1]) cudaFree(s->words_up[1]);
@@ -1286,6 +1323,24 @@ static void free_sim(aq_sim* s) {
   if (s->up_st) cudaStreamDestroy(s->up_st);
   if (s->down_st) cudaStreamDestroy(s->down_st);
   delete s;
+}
+
+static int sim_check(const aq_sim* s) {
+  return *reinterpret_cast<const volatile int32_t*>(s->stalled) ? AQ_E_STALLED : AQ_OK;
+}
+
+// The state is set anew: after a launch that gave up, its status flag goes and
+// the next chain clears its grids.
+static int sim_recover(aq_sim* s) {
+  if (sim_check(s) == AQ_OK) return AQ_OK;
+  unsigned f = 0;
+  AQ_CUDA_TRY(cudaDeviceSynchronize());
+  AQ_CUDA_TRY(cudaMemcpy(&f, s->status, sizeof(f), cudaMemcpyDeviceToHost));
+  f &= ~AQ_ST_STALLED;
+  AQ_CUDA_TRY(cudaMemcpy(s->status, &f, sizeof(f), cudaMemcpyHostToDevice));
+  *s->stalled = 0;
+  s->stale = true;
+  return AQ_OK;
 }
 
 // Encode `count` particles from values into the current records at position
@@ -1348,6 +1403,11 @@ int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
   if (!P->sparse && nblk64 * 64 > 0x7fffffffLL) {
     delete s;
     return AQ_E_LIMIT;  // the dense binning's cell keys are int32
+  }
+  s->stalled = stall_word();
+  if (!s->stalled) {
+    free_sim(s);
+    return AQ_E_NOMEM;
   }
   s->nblk = (int)nblk64;
   s->nkeys = P->sparse ? 0 : (int64_t)s->nblk * 64;
@@ -1584,6 +1644,7 @@ int aq_sim_append(aq_sim* s, const void* values, int32_t values_f64, int64_t cou
   cudaStream_t st = as_stream(stream);
   const int64_t base = s->n;
   int rc;
+  if ((rc = sim_check(s))) return rc;
   if ((rc = store_values(s, values, values_f64, base, count, st))) return rc;
   s->n = base + count;
   s->sorted = false;
@@ -1617,6 +1678,7 @@ int aq_sim_set_state(aq_sim* s, const void* values, int32_t values_f64, void* st
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
   int rc;
+  if ((rc = sim_recover(s))) return rc;
   if ((rc = store_values(s, values, values_f64, 0, s->n, st))) return rc;
   s->sorted = false;
   s->launches += 1;
@@ -1627,6 +1689,8 @@ int aq_sim_get_state(aq_sim* s, void* values, int32_t values_f64, void* stream) 
   if (!s || !values) return AQ_E_ARG;
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
+  const int rc = sim_check(s);
+  if (rc != AQ_OK) return rc;
   AQ_CUDA_TRY(rec_fetch(s->L, s->words[s->cur], s->pid[s->cur], values, values_f64 != 0, s->n, st));
   s->launches += 1;
   return AQ_OK;
@@ -1703,13 +1767,15 @@ int aq_sim_field_stats(aq_sim* s, const void* ref, int32_t ref_f64, double* h_ou
   s->launches += 1;
   AQ_CUDA_TRY(cudaMemcpyAsync(h_out, s->dstats, sizeof(double) * 5 * s->NS, cudaMemcpyDeviceToHost, st));
   AQ_CUDA_TRY(cudaStreamSynchronize(st));
-  return AQ_OK;
+  return sim_check(s);
 }
 
 int aq_sim_set_words(aq_sim* s, const uint64_t* words, void* stream) {
   if (!s || !words) return AQ_E_ARG;
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
+  const int rc = sim_recover(s);
+  if (rc != AQ_OK) return rc;
   k_iota<<<grid_for(s->n, 256), 256, 0, st>>>(s->pid[s->cur], s->n);
   AQ_CUDA_TRY(cudaGetLastError());
   AQ_CUDA_TRY(rec_group(words, s->words[s->cur], s->n, s->W, st));
@@ -1722,6 +1788,8 @@ int aq_sim_get_words(aq_sim* s, uint64_t* words, void* stream) {
   if (!s || !words) return AQ_E_ARG;
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
+  const int rc = sim_check(s);
+  if (rc != AQ_OK) return rc;
   AQ_CUDA_TRY(rec_ungroup(s->words[s->cur], s->pid[s->cur], words, s->n, s->W, 0, st));
   s->launches += 1;
   return AQ_OK;
@@ -1730,11 +1798,15 @@ int aq_sim_get_words(aq_sim* s, uint64_t* words, void* stream) {
 int aq_sim_substeps(aq_sim* s, int32_t n, void* stream) {
   if (!s || n < 0) return AQ_E_ARG;
   if (n == 0) return AQ_OK;
+  const int rc = sim_check(s);
+  if (rc != AQ_OK) return rc;
   return s->impl->substeps(n, as_stream(stream));
 }
 
 int aq_sim_grid_mass(aq_sim* s, float* d_out, void* stream) {
   if (!s || !d_out) return AQ_E_ARG;
+  const int rc = sim_check(s);
+  if (rc != AQ_OK) return rc;
   cudaStream_t st = as_stream(stream);
   const unsigned nb = (unsigned)std::min<int64_t>(grid_for(s->ncell, 256), (int64_t)num_sms() * 8);
   if (s->P.sparse) {
@@ -1767,7 +1839,8 @@ int aq_sim_grid_mass(aq_sim* s, float* d_out, void* stream) {
 int aq_sim_loss(aq_sim* s, int32_t kind, double* h_out, void* stream) {
   if (!s || !h_out || kind != 0) return AQ_E_ARG;
   s->launches += 1;
-  return s->impl->loss(h_out, as_stream(stream));
+  const int rc = s->impl->loss(h_out, as_stream(stream));
+  return rc != AQ_OK ? rc : sim_check(s);
 }
 
 int aq_sim_ranges_enable(aq_sim* s, int32_t on, void* stream) {
@@ -1793,7 +1866,7 @@ int aq_sim_ranges_get(aq_sim* s, double* h_max, double* h_min, void* stream) {
   AQ_CUDA_TRY(cudaMemcpyAsync(h_max, s->rmax, sizeof(double) * s->NS, cudaMemcpyDeviceToHost, st));
   AQ_CUDA_TRY(cudaMemcpyAsync(h_min, s->rmin, sizeof(double) * s->NS, cudaMemcpyDeviceToHost, st));
   AQ_CUDA_TRY(cudaStreamSynchronize(st));
-  return AQ_OK;
+  return sim_check(s);
 }
 
 int aq_sim_status(aq_sim* s, uint32_t* h_flags, int64_t* h_fallbacks, int32_t clear, void* stream) {
@@ -1811,6 +1884,17 @@ int aq_sim_status(aq_sim* s, uint32_t* h_flags, int64_t* h_fallbacks, int32_t cl
   if (h_flags) *h_flags = f;
   if (h_fallbacks) *h_fallbacks = (int64_t)fb;
   return AQ_OK;
+}
+
+int aq_sim_wait_limit(aq_sim* s, int64_t cycles) {
+  if (!s || cycles < 1) return AQ_E_ARG;
+  s->wait_limit = cycles;
+  return AQ_OK;
+}
+
+int aq_sim_check(const aq_sim* s) {
+  if (!s) return AQ_E_ARG;
+  return sim_check(s);
 }
 
 int aq_sim_step_count(const aq_sim* s, int64_t* h_out) {

@@ -46,6 +46,7 @@ extern "C" {
 #define AQ_E_NOMEM (-4)    /* device allocation failed */
 #define AQ_E_STATE (-5)    /* call not valid in the current state */
 #define AQ_E_LIMIT (-6)    /* size above a documented maximum */
+#define AQ_E_STALLED (-7)  /* a substep launch gave up waiting for its own blocks: set the state anew */
 
 /* device status flags (aq_sim_status) */
 #define AQ_ST_OUT_OF_DOMAIN 0x1u  /* a particle stencil left the grid; base clamped */
@@ -314,6 +315,16 @@ int aq_sim_ranges_get(aq_sim* sim, double* h_max, double* h_min, void* stream);
  * stream.  clear != 0 resets them. */
 int aq_sim_status(aq_sim* sim, uint32_t* h_flags, int64_t* h_fallbacks,
                   int32_t clear, void* stream);
+/* In small scenes one launch makes several passes over the particles, with a
+ * barrier between them.  A launch whose blocks waited longer than this many
+ * SM clock cycles for one another (0 < cycles; default 2^34, some 9 s, which
+ * no launch comes near) gives up: AQ_ST_STALLED is set, and from then on
+ * substeps, append and every call that reads the state return AQ_E_STALLED
+ * until aq_sim_set_state or aq_sim_set_words sets it anew.
+ * aq_sim_check returns AQ_E_STALLED once a launch that the host has waited
+ * for gave up, AQ_OK else; it does not synchronize. */
+int aq_sim_wait_limit(aq_sim* sim, int64_t cycles);
+int aq_sim_check(const aq_sim* sim);
 int aq_sim_step_count(const aq_sim* sim, int64_t* h_out);
 /* Set the substep counter (the dithering generator's step index), e.g. when
  * resuming from saved records so that the continuation draws the same
