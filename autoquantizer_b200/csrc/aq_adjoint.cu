@@ -1074,9 +1074,11 @@ struct aq_adjoint {
   size_t rsz = 4;
   // three node grids in rotation: g[rot] takes (or holds) the current
   // state's sums (m, P); every kernel that fills one of the others clears
-  // the one after, so that g[rot] is zero whenever a chain starts
+  // the one after, so that g[rot] is zero whenever a chain starts (unless
+  // broken: a pass did not run to its end, or was only captured into a graph)
   void* g[3] = {nullptr, nullptr, nullptr};
   int rot = 0;
+  bool broken = false;
   std::vector<void*> ckpt;  // states at multiples of the checkpoint interval (every > 0), or the initial state
   std::vector<void*> seg;   // states between two checkpoints; two ping-pong states (every == 0)
   std::vector<void*> stash;  // bisection checkpointing: one state per recursion level, plus a scratch state
@@ -1219,9 +1221,11 @@ static int ad_make_perm(aq_adjoint* a, const void* d_s0, cudaStream_t st) {
   if (pool_alloc((void**)&tmp, 3 * n8 + tb, st) != cudaSuccess) return AQ_E_NOMEM;
   uint64_t *kin = (uint64_t*)tmp, *kout = (uint64_t*)(tmp + n8);
   int32_t* iin = (int32_t*)(tmp + 2 * n8);
-  // per-cell counts in a grid that is not in use; cleared again behind them
+  // per-cell counts in the grid that takes the first state's sums: cleared
+  // whole before them (a captured pass starts from what the one before left)
+  // and again behind them
   void* count = a->g[a->rot];
-  cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int32_t) * a->ncell, st);
+  cudaError_t e = cudaMemsetAsync(count, 0, a->rsz * 4 * a->ncell, st);
   int rc = e == cudaSuccess ? a->impl->sort_keys(d_s0, (int32_t*)count, kin, iin, st) : AQ_E_CUDA;
   if (rc == AQ_OK &&
       cub::DeviceRadixSort::SortPairs(tmp + 3 * n8, tb, kin, kout, iin, a->perm, (int)a->n, 0, bits, st) != cudaSuccess)
@@ -1287,6 +1291,14 @@ static int ad_buffers(aq_adjoint* a, std::vector<void*>& v, int want, cudaStream
     AQ_CUDA_TRY(pool_alloc(&p, a->state_bytes(), st));
     v.push_back(p);
   }
+  return AQ_OK;
+}
+
+// A pass begins: the grids zeroed if the last one broke off.
+static int ad_begin(aq_adjoint* a, cudaStream_t st) {
+  if (a->broken)
+    for (void* g : a->g) AQ_CUDA_TRY(cudaMemsetAsync(g, 0, a->rsz * 4 * a->ncell, st));
+  a->broken = true;  // until its last launch is queued
   return AQ_OK;
 }
 
@@ -1409,6 +1421,7 @@ int aq_adjoint_forward(aq_adjoint* a, const void* d_s0, int32_t n_substeps, int3
   if ((rc = ad_buffers(a, a->ckpt, bisect ? 1 : (n_substeps + every - 1) / every, st))) return rc;
   if ((rc = ad_buffers(a, a->seg, bisect ? 2 : every, st))) return rc;
   if (!bisect && (rc = ad_buffers(a, a->stash, 0, st))) return rc;
+  if ((rc = ad_begin(a, st))) return rc;
   // the state is kept in the library's order and layout; the caller's is
   // restored for d_sT here and for the gradients in aq_adjoint_backward
   if ((rc = ad_make_perm(a, d_s0, st))) return rc;
@@ -1421,6 +1434,9 @@ int aq_adjoint_forward(aq_adjoint* a, const void* d_s0, int32_t n_substeps, int3
     return t < n_substeps ? a->ckpt[t / every] : a->seg[0];
   };
   if ((rc = ad_chain(a, a->ckpt[0], 0, n_substeps, buf, false, st))) return rc;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  AQ_CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
+  a->broken = capturing != cudaStreamCaptureStatusNone;
   a->T = n_substeps;
   a->every = every;
   a->seg_of = bisect ? -1 : (n_substeps - 1) / every;
@@ -1436,6 +1452,7 @@ int aq_adjoint_backward(aq_adjoint* a, const void* d_seed, void* d_grad_s0, doub
   // one stash per level, the last one is scratch
   if (every == 0 && (rc = ad_buffers(a, a->stash, levels + 1, st))) return rc;
   if ((rc = ad_buffers(a, a->ab, 2, st))) return rc;
+  if ((rc = ad_begin(a, st))) return rc;
   void** ab = a->ab.data();
   rc = a->impl->permute(d_seed, ab[0], true, st);  // into the order of the forward pass
   const size_t sens_bytes = sizeof(double) * AD_SENS_COPIES * a->NS;
@@ -1470,6 +1487,7 @@ int aq_adjoint_backward(aq_adjoint* a, const void* d_seed, void* d_grad_s0, doub
   if (e == cudaSuccess) e = es;
   if (e != cudaSuccess) set_last_cuda_error(e, "aq_adjoint_backward");
   if (rc == AQ_OK && e != cudaSuccess) rc = AQ_E_CUDA;
+  a->broken = rc != AQ_OK;
   if (rc == AQ_OK && h_sens)
     for (int s = 0; s < a->NS; ++s) {
       h_sens[s] = 0;
