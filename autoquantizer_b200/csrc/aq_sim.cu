@@ -997,7 +997,12 @@ struct SimImpl final : SimBase {
     a.sk = step_key(a.seed, a.step0 + a.pass0 - 1);
     a.do_g2p = a.pass0 > 0;
     a.do_p2g = a.pass0 < a.n_sub;
-    const int ctas = (int)std::min<int64_t>(S_->step_grid, items_bound());
+    // CTAs: one per work item, and with few items on a large grid enough for
+    // the clear (16 nodes a thread; 256^3 nodes, 16 substeps of one particle:
+    // 65 ms on the two CTAs of its items, 0.92 with these)
+    int64_t busy = items_bound();
+    if (a.clear && !S_->P.sparse) busy = std::max(busy, (S_->ncell + 16 * CH - 1) / (16 * CH));
+    const int ctas = (int)std::min<int64_t>(S_->step_grid, busy);
     if (S_->multi) AQ_CUDA_TRY(cudaMemsetAsync(S_->sync, 0, sizeof(int32_t) * AQ_SYNC_WORDS, st));
     // two claim counters alternate between launches without MULTI; each launch
     // zeroes the one the next launch uses (both start at zero)
