@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from autoquantizer_b200 import scenes
+from autoquantizer_b200.adjoint import Adjoint, ek_seed
 from autoquantizer_b200.mpm_solver import MPMSolver
 
 pytestmark = pytest.mark.gpu
@@ -38,4 +39,28 @@ def _substeps_ms(n, n_grid):
 @pytest.mark.parametrize("n,n_grid", [(1, 128), (64, 256)])
 def test_substeps(n, n_grid):
     few, many = _substeps_ms(n, n_grid), _substeps_ms(1000, n_grid)
+    assert few <= 3 * many, (few, many)
+
+
+def _adjoint_ms(n, n_grid):
+    import torch
+
+    cfg, vals = scenes.falling_block_3d(n=n, n_grid=n_grid)
+    cfg.dt = 1e-5
+    s = MPMSolver(cfg)
+    s.set_particles(vals)
+    adj = Adjoint(s._params())
+    s0 = torch.from_numpy(np.ascontiguousarray(vals[:, :s.n_slots()])).cuda().float()
+
+    def run():
+        sT = adj.forward(s0, 8, 8)
+        adj.backward(ek_seed(sT, 3, s.p_mass, s.g))
+
+    ms = _median_ms(run)
+    adj.close()
+    return ms
+
+
+def test_adjoint():
+    few, many = _adjoint_ms(64, 128), _adjoint_ms(2000, 128)
     assert few <= 3 * many, (few, many)
