@@ -1072,6 +1072,7 @@ struct AdBase {
 struct aq_adjoint {
   aq_params P;
   int D = 0, NS = 0;
+  int device = 0;  // where its memory is
   int64_t n = 0, ncell = 0;
   size_t rsz = 4;
   // three node grids in rotation: g[rot] takes (or holds) the current
@@ -1354,7 +1355,7 @@ int aq_adjoint_create(const aq_params* P, aq_adjoint** out) {
   a->ncell = 1;
   for (int d = 0; d < D; ++d) a->ncell *= P->res[d];
   const size_t gbytes = a->rsz * 4 * a->ncell;
-  cudaError_t e = cudaSuccess;
+  cudaError_t e = cudaGetDevice(&a->device);
   for (int k = 0; k < 3; ++k) {
     if (e == cudaSuccess) e = pool_alloc(&a->g[k], gbytes, 0);
     if (e == cudaSuccess) e = cudaMemsetAsync(a->g[k], 0, gbytes, 0);
@@ -1412,6 +1413,7 @@ int aq_adjoint_set_collider(aq_adjoint* a, const float* d_sdf, const float* d_no
 
 int aq_adjoint_destroy(aq_adjoint* a) {
   if (!a) return AQ_E_ARG;
+  const OnDevice on(a->device);
   cudaDeviceSynchronize();
   free_ad(a);
   return AQ_OK;

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "../../include/aq.h"
+#include "aq_pool.h"
 
 #define AQ_CUDA_TRY(expr)                        \
   do {                                           \
@@ -18,12 +19,6 @@
 namespace aq {
 
 void set_last_cuda_error(cudaError_t e, const char* what);
-
-// Device memory from a pool of the library's own, in stream order (aq_core.cu):
-// an allocation is there for work on st, and for other streams once they
-// wait for st.  pool_free(null) does nothing.
-cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st);
-void pool_free(void* p, cudaStream_t st);
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 

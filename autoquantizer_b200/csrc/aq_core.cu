@@ -5,7 +5,6 @@
 
 #include <algorithm>
 #include <mutex>
-#include <unordered_map>
 
 #include "aq_codec.cuh"
 #include "aq_common.cuh"
@@ -17,91 +16,6 @@ static thread_local char g_last_error[256] = "";
 
 void set_last_cuda_error(cudaError_t e, const char* what) {
   snprintf(g_last_error, sizeof(g_last_error), "%s: %s", what, cudaGetErrorString(e));
-}
-
-// ------------------------------------------------------------ memory pool
-//
-// Simulators, adjoints and the scratch of single calls take their memory
-// from one pool per device.  The pool keeps up to POOL_KEEP bytes that were
-// given back beyond what is in use (the release threshold counts both, so it
-// follows: with 1.4 GB in use and a threshold of 1 GiB, each call's scratch was
-// unmapped and mapped again; the driver's own default keeps none past the next
-// synchronization, and mapping memory anew took 0.1 to 10 ms an allocation,
-// more than the work of small calls), and gives back everything it can when
-// an allocation fails.  The driver's pool is safe for several threads and
-// streams: memory freed on one stream goes to another only after the free.
-constexpr uint64_t POOL_KEEP = uint64_t(1) << 30;
-constexpr int POOL_DEVICES = 64;
-
-static std::mutex g_pool_mu;
-static cudaMemPool_t g_pool[POOL_DEVICES];
-struct PoolBlock {
-  cudaMemPool_t pool;
-  size_t bytes;
-};
-static std::unordered_map<void*, PoolBlock> g_pool_live;
-static std::unordered_map<cudaMemPool_t, uint64_t> g_pool_used;
-
-// `by` more (or fewer) bytes in use in a pool; g_pool_mu held
-static void pool_count(cudaMemPool_t pool, int64_t by) {
-  uint64_t& used = g_pool_used[pool];
-  used += by;
-  uint64_t keep = used + POOL_KEEP;
-  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-}
-
-static cudaError_t pool_of(cudaMemPool_t* out) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= POOL_DEVICES) return cudaDeviceGetDefaultMemPool(out, dev);
-  std::lock_guard<std::mutex> g(g_pool_mu);
-  if (!g_pool[dev]) {
-    cudaMemPoolProps props;
-    memset(&props, 0, sizeof(props));
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t p;
-    if ((e = cudaMemPoolCreate(&p, &props)) != cudaSuccess) return e;
-    g_pool[dev] = p;
-  }
-  *out = g_pool[dev];
-  return cudaSuccess;
-}
-
-cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st) {
-  *p = nullptr;
-  cudaMemPool_t pool;
-  cudaError_t e = pool_of(&pool);
-  if (e != cudaSuccess) return e;
-  e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, st);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    cudaDeviceSynchronize();
-    cudaMemPoolTrimTo(pool, 0);
-    e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, st);
-    if (e != cudaSuccess) cudaGetLastError();
-  }
-  if (e == cudaSuccess) {
-    std::lock_guard<std::mutex> g(g_pool_mu);
-    g_pool_live[*p] = PoolBlock{pool, bytes};
-    pool_count(pool, (int64_t)bytes);
-  }
-  return e;
-}
-
-void pool_free(void* p, cudaStream_t st) {
-  if (!p) return;
-  {
-    std::lock_guard<std::mutex> g(g_pool_mu);
-    const auto it = g_pool_live.find(p);
-    if (it != g_pool_live.end()) {
-      pool_count(it->second.pool, -(int64_t)it->second.bytes);
-      g_pool_live.erase(it);
-    }
-  }
-  cudaFreeAsync(p, st);
 }
 
 // ----------------------------------------------------------- state error

@@ -603,6 +603,7 @@ struct aq_sim {
   aq_params P;
   aq_layout L;
   int W = 0, WS = 0, NS = 0, D = 0;
+  int device = 0;   // where its memory is
   int64_t n = 0;    // active records
   int64_t cap = 0;  // records the device buffers hold (n_particles at creation)
   uint64_t* words[2] = {nullptr, nullptr};
@@ -1410,7 +1411,7 @@ int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
     return AQ_E_LIMIT;  // the dense binning's cell keys are int32
   }
   s->stalled = stall_word();
-  if (!s->stalled) {
+  if (!s->stalled || cudaGetDevice(&s->device) != cudaSuccess) {
     free_sim(s);
     return AQ_E_NOMEM;
   }
@@ -1673,6 +1674,7 @@ int aq_sim_stream_chunks(const aq_sim* s, int64_t* h_chunk, int64_t* h_n_total) 
 
 int aq_sim_destroy(aq_sim* s) {
   if (!s) return AQ_E_ARG;
+  const OnDevice on(s->device);
   cudaDeviceSynchronize();
   free_sim(s);
   return AQ_OK;
