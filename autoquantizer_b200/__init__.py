@@ -14,5 +14,12 @@ def MPMSolver(*args, **kwargs):
     return _S(*args, **kwargs)
 
 
+def release_memory():
+    """Give the device memory that the library keeps for later calls (up to
+    1 GiB) back to the current device, e.g. before another allocator in the
+    process needs it (aq_memory_release).  Waits for the device."""
+    _lib.check(_lib.lib().aq_memory_release(), "aq_memory_release")
+
+
 __all__ = ["MPMConfig", "MPMSolver", "LagrangianCR", "LagrangianEB", "ScipySolver", "ScipySolverMemMode",
-           "quant", "solvers"]
+           "quant", "solvers", "release_memory"]

@@ -30,7 +30,7 @@ EXPORTS = [
     "aq_sim_field_stats", "aq_sim_set_collider", "aq_sim_collider_get", "aq_sim_collider_pose",
     "aq_sim_collider_velocity_mode", "aq_sim_sparse_blocks", "aq_sim_grid_mass", "aq_voxelize", "aq_adjoint_set_collider",
     "aq_sim_ranges_enable", "aq_sim_ranges_get", "aq_sim_status", "aq_sim_check", "aq_sim_wait_limit", "aq_sim_step_count", "aq_sim_set_step_count", "aq_sim_launches",
-    "aq_state_error", "aq_error_string", "aq_abi_version", "aq_sim_profile_enable", "aq_sim_profile_get",
+    "aq_state_error", "aq_memory_release", "aq_error_string", "aq_abi_version", "aq_sim_profile_enable", "aq_sim_profile_get",
     "aq_sim_kernel_is_jit", "aq_adjoint_create", "aq_adjoint_destroy", "aq_adjoint_forward", "aq_adjoint_backward",
     "aq_mlp_param_count", "aq_mlp_to_bf16", "aq_mlp_forward", "aq_mlp_backward", "aq_mlp_mse_grad", "aq_mlp_adam",
     "aq_state_error_noalloc", "aq_sim_create_streamed", "aq_sim_stream_set_words", "aq_sim_stream_get_words",
@@ -145,6 +145,7 @@ def lib():
         "aq_mlp_adam": ([vp, vp, vp, vp, vp, i64, C.c_float, C.c_float, C.c_float, C.c_float, i32, vp], C.c_int),
         "aq_state_error_noalloc": ([vp, i32, vp, i32, i64, i32, C.POINTER(C.c_double), C.POINTER(C.c_double), vp],
                                    C.c_int),
+        "aq_memory_release": ([], C.c_int),
         "aq_error_string": ([i32], C.c_char_p),
         "aq_abi_version": ([], i32),
     }

@@ -1416,6 +1416,7 @@ int aq_adjoint_destroy(aq_adjoint* a) {
   const OnDevice on(a->device);
   cudaDeviceSynchronize();
   free_ad(a);
+  cudaStreamSynchronize(0);  // what the pool does not keep goes back to the device now
   return AQ_OK;
 }
 

@@ -88,6 +88,11 @@ using namespace aq;
 
 extern "C" {
 
+int aq_memory_release(void) {
+  AQ_CUDA_TRY(pool_release());
+  return AQ_OK;
+}
+
 int32_t aq_abi_version(void) { return AQ_ABI_VERSION; }
 
 const char* aq_error_string(int32_t code) {

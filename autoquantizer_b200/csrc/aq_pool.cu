@@ -7,7 +7,7 @@
 // unmapped and mapped again; the driver's own default keeps none past the next
 // synchronization, and mapping memory anew took 0.1 to 10 ms an allocation,
 // more than the work of small calls), and gives back everything it can when
-// an allocation fails.  The driver's pool is safe for several threads and
+// an allocation fails or pool_release is called.  The driver's pool is safe for several threads and
 // streams: memory freed on one stream goes to another only after the free.
 #include "aq_pool.h"
 
@@ -103,6 +103,19 @@ cudaError_t pool_free(void* p, cudaStream_t st) {
     pool_count(b.pool, (int64_t)b.bytes);
   }
   return e;
+}
+
+cudaError_t pool_release() {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) return e;
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    if (dev >= 0 && dev < POOL_DEVICES) pool = g_pool[dev];
+  }
+  return pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
 }
 
 }  // namespace aq

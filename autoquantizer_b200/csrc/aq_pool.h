@@ -15,6 +15,10 @@ cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st);
 // does nothing.  After an error the memory still counts as in use.
 cudaError_t pool_free(void* p, cudaStream_t st);
 
+// What the current device's pool keeps beyond what is in use goes back to the
+// device.  Waits for the device.
+cudaError_t pool_release();
+
 // A device made current for a scope.
 class OnDevice {
   int was = -1;

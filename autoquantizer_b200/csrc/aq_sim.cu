@@ -1677,6 +1677,7 @@ int aq_sim_destroy(aq_sim* s) {
   const OnDevice on(s->device);
   cudaDeviceSynchronize();
   free_sim(s);
+  cudaStreamSynchronize(0);  // what the pool does not keep goes back to the device now
   return AQ_OK;
 }
 

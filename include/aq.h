@@ -442,6 +442,12 @@ int aq_mlp_mse_grad(const float* d_y, const float* d_target, const float* d_mask
 int aq_mlp_adam(float* d_params, uint16_t* d_params_bf16, float* d_m, float* d_v, const float* d_grad, int64_t n,
                 float lr, float beta1, float beta2, float eps, int32_t t, void* stream);
 
+/* Simulators, adjoints and the scratch of calls take device memory from a pool
+ * of the library's own, which keeps up to 1 GiB per device that was given back
+ * (set-up and small calls would spend most of their time mapping memory).
+ * This gives what the current device's pool keeps back to the device, for
+ * other allocators in the process; it waits for the device. */
+int aq_memory_release(void);
 const char* aq_error_string(int32_t code);
 int32_t aq_abi_version(void);
 #endif /* __CUDACC_RTC__ */

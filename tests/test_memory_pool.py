@@ -97,6 +97,11 @@ int main() {
   fake().failing_allocs = 2;
   CHECK(pool_alloc(&a, 64, nullptr) == cudaErrorMemoryAllocation && a == nullptr);
   CHECK(fake().pools[0]->threshold == keep);
+  // what is kept is given back on request, the current device's only
+  cudaSetDevice(1);
+  CHECK(pool_release() == cudaSuccess && fake().pools[1]->trims == 1 && fake().pools[0]->trims == 2);
+  cudaSetDevice(7);
+  CHECK(pool_release() == cudaSuccess);  // no pool there
   // threads
   std::vector<std::thread> ts;
   for (int t = 0; t < 4; ++t)
