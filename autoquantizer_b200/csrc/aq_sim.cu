@@ -1363,9 +1363,8 @@ static int store_values(aq_sim* s, const void* values, int32_t values_f64, int64
 
 using namespace aq;
 
-extern "C" {
-
-int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
+// streamed: without the third grid, which only chains of the in-core passes use
+static int sim_create(const aq_params* P, const aq_layout* L, bool streamed, aq_sim** out) {
   if (!P || !L || !out) return AQ_E_ARG;
   *out = nullptr;
   const int D = P->dim;
@@ -1481,7 +1480,7 @@ int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
     return AQ_E_LIMIT;
   }
   const size_t gbytes = rsz * 4 * s->ncell, before = total;
-  const bool third = !P->sparse && gbytes <= THIRD_GRID_MAX;
+  const bool third = !P->sparse && !streamed && gbytes <= THIRD_GRID_MAX;
   if (third) total += (gbytes + 255) & ~(size_t)255;  // the third grid, behind the others
   e = pool_alloc(&s->slab, total, 0);
   if (e == cudaSuccess && third) {
@@ -1548,6 +1547,10 @@ int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) {
   return AQ_OK;
 }
 
+extern "C" {
+
+int aq_sim_create(const aq_params* P, const aq_layout* L, aq_sim** out) { return sim_create(P, L, false, out); }
+
 int aq_sim_create_streamed(const aq_params* P, const aq_layout* L, int64_t chunk, aq_sim** out) {
   if (!P || !L || !out || chunk < 1) return AQ_E_ARG;
   *out = nullptr;
@@ -1558,7 +1561,7 @@ int aq_sim_create_streamed(const aq_params* P, const aq_layout* L, int64_t chunk
   aq_params Q = *P;
   Q.n_particles = chunk;  // the device buffers hold one chunk
   aq_sim* s = nullptr;
-  int rc = aq_sim_create(&Q, L, &s);
+  int rc = sim_create(&Q, L, true, &s);
   if (rc != AQ_OK) return rc;
   const int64_t nc = (n_total + chunk - 1) / chunk;
   const size_t wbytes = sizeof(uint64_t) * (size_t)(nc * grouped_words(chunk, s->W));

@@ -39,3 +39,23 @@ def test_memory_of_a_destroyed_simulator():
     assert before - free() < GB + 64 * MB
     aq.release_memory()
     assert before - free() < 64 * MB
+
+
+def test_streamed_simulator_holds_two_grids():
+    import torch
+
+    from autoquantizer_b200.streamed import StreamedSolver
+
+    cfg, vals = scenes.falling_block_3d(n=1000, n_grid=256)
+    s = MPMSolver(cfg)
+    s.set_particles(vals)
+    StreamedSolver(s, 1000).close()  # kernels compiled and loaded
+    torch.cuda.empty_cache()
+    aq.release_memory()
+    before = torch.cuda.mem_get_info()[0]
+    st = StreamedSolver(s, 1000)
+    held = before - torch.cuda.mem_get_info()[0]
+    st.close()
+    grid = 16 * 256 ** 3
+    cells = 2 * 4 * 256 ** 3  # per-cell counts and offsets of the binning
+    assert 2 * grid <= held < 2 * grid + cells + 64 * MB, held
