@@ -16,12 +16,11 @@ AQ_MAX_MATERIALS = 4
 
 AQ_FIXED, AQ_INT, AQ_FLOAT_EXP, AQ_SHARED_EXP, AQ_RAW_F32, AQ_RAW_F64 = range(6)
 AQ_MAT_FLUID, AQ_MAT_ELASTIC, AQ_MAT_COROTATED = range(3)
-AQ_ST_OUT_OF_DOMAIN, AQ_ST_NAN, AQ_ST_FALLBACK, AQ_ST_POOL_FULL, AQ_ST_STALLED = 0x1, 0x2, 0x4, 0x8, 0x10
+AQ_ST_OUT_OF_DOMAIN, AQ_ST_NAN, AQ_ST_FALLBACK, AQ_ST_POOL_FULL = 0x1, 0x2, 0x4, 0x8
 
 ERRORS = {0: "ok", -1: "bad argument", -2: "layout does not fit the simulator schema", -3: "CUDA error",
           -4: "device allocation failed", -5: "call not valid in the current state",
-          -6: "size above the documented maximum",
-          -7: "a substep launch gave up waiting for its own blocks: set the state anew"}
+          -6: "size above the documented maximum"}
 
 # every symbol include/aq.h declares (checked by the CPU test suite)
 EXPORTS = [
@@ -29,7 +28,7 @@ EXPORTS = [
     "aq_sim_get_state", "aq_sim_set_words", "aq_sim_get_words", "aq_sim_substeps", "aq_sim_loss",
     "aq_sim_field_stats", "aq_sim_set_collider", "aq_sim_collider_get", "aq_sim_collider_pose",
     "aq_sim_collider_velocity_mode", "aq_sim_sparse_blocks", "aq_sim_grid_mass", "aq_voxelize", "aq_adjoint_set_collider",
-    "aq_sim_ranges_enable", "aq_sim_ranges_get", "aq_sim_status", "aq_sim_check", "aq_sim_wait_limit", "aq_sim_step_count", "aq_sim_set_step_count", "aq_sim_launches",
+    "aq_sim_ranges_enable", "aq_sim_ranges_get", "aq_sim_status", "aq_sim_step_count", "aq_sim_set_step_count", "aq_sim_launches",
     "aq_state_error", "aq_memory_release", "aq_error_string", "aq_abi_version", "aq_sim_profile_enable", "aq_sim_profile_get",
     "aq_sim_kernel_is_jit", "aq_adjoint_create", "aq_adjoint_destroy", "aq_adjoint_forward", "aq_adjoint_backward",
     "aq_mlp_param_count", "aq_mlp_to_bf16", "aq_mlp_forward", "aq_mlp_backward", "aq_mlp_mse_grad", "aq_mlp_adam",
@@ -123,8 +122,6 @@ def lib():
         "aq_sim_ranges_enable": ([vp, i32, vp], C.c_int),
         "aq_sim_ranges_get": ([vp, C.POINTER(C.c_double), C.POINTER(C.c_double), vp], C.c_int),
         "aq_sim_status": ([vp, C.POINTER(C.c_uint32), C.POINTER(C.c_int64), i32, vp], C.c_int),
-        "aq_sim_check": ([vp], C.c_int),
-        "aq_sim_wait_limit": ([vp, i64], C.c_int),
         "aq_sim_step_count": ([vp, C.POINTER(C.c_int64)], C.c_int),
         "aq_sim_set_step_count": ([vp, i64], C.c_int),
         "aq_sim_launches": ([vp, C.POINTER(C.c_int64)], C.c_int),

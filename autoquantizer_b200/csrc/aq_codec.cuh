@@ -254,8 +254,7 @@ struct GRec {
 
 // Record r's W words into rec[0, W) / from rec: the pairs as 16-byte
 // vectors.  WC: the word count when it is a compile-time constant, else 0.
-// Loads go to L2: another CTA may have written the record earlier in the
-// same launch.
+// Loads go to L2 (a record is read once; and see kernel_begin on __ldg).
 template <int WC>
 __device__ __forceinline__ void load_grec(const uint64_t* words, int64_t r, int W, uint64_t* rec) {
   const int Wn = WC ? WC : W, W2 = Wn & ~1;

@@ -111,8 +111,6 @@ const char* aq_error_string(int32_t code) {
       return "call not valid in the current state";
     case AQ_E_LIMIT:
       return "size above the documented maximum";
-    case AQ_E_STALLED:
-      return "a substep launch gave up waiting for its own blocks: set the state anew";
     default:
       return "unknown error";
   }

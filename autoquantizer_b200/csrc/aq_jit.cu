@@ -49,8 +49,6 @@ struct Nvrtc {
 struct Driver {
   CUresult (*load)(CUmodule*, const void*) = nullptr;
   CUresult (*getfn)(CUfunction*, CUmodule, const char*) = nullptr;
-  CUresult (*launch_coop)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream,
-                          void**) = nullptr;
   CUresult (*launch_ex)(const CUlaunchConfig*, CUfunction, void**, void**) = nullptr;
   CUresult (*setattr)(CUfunction, CUfunction_attribute, int) = nullptr;
   CUresult (*occ)(int*, CUfunction, int, size_t) = nullptr;
@@ -95,7 +93,7 @@ void init_once() {
               sym(g_nv.h, "nvrtcGetLoweredName", g_nv.lowered) && sym(g_nv.h, "nvrtcDestroyProgram", g_nv.destroy);
   }
   g_dr.ok = drv("cuModuleLoadData", g_dr.load) && drv("cuModuleGetFunction", g_dr.getfn) &&
-            drv("cuLaunchKernelEx", g_dr.launch_ex) && drv("cuLaunchCooperativeKernel", g_dr.launch_coop) && drv("cuFuncSetAttribute", g_dr.setattr) &&
+            drv("cuLaunchKernelEx", g_dr.launch_ex) && drv("cuFuncSetAttribute", g_dr.setattr) &&
             drv("cuOccupancyMaxActiveBlocksPerMultiprocessor", g_dr.occ);
 }
 
@@ -154,8 +152,7 @@ bool jit_available() {
   return g_nv.ok && g_dr.ok;
 }
 
-void* jit_k_step(int D, bool HF, bool HM, bool f64, bool col, bool sparse, bool multi, const aq_layout& L,
-                 std::string* err) {
+void* jit_k_step(int D, bool HF, bool HM, bool f64, bool col, bool sparse, const aq_layout& L, std::string* err) {
   std::lock_guard<std::mutex> g(g_mu);
   init_once();
   if (!g_nv.ok || !g_dr.ok) {
@@ -163,10 +160,10 @@ void* jit_k_step(int D, bool HF, bool HM, bool f64, bool col, bool sparse, bool 
     return nullptr;
   }
   char name[160];
-  snprintf(name, sizeof name, "aq::k_step<%d, %s, %s, %s, aq::JitLayout, %s, %s, %s>", D, HF ? "true" : "false",
-           HM ? "true" : "false", f64 ? "double" : "float", col ? "true" : "false", sparse ? "true" : "false", multi ? "true" : "false");
+  snprintf(name, sizeof name, "aq::k_step<%d, %s, %s, %s, aq::JitLayout, %s, %s>", D, HF ? "true" : "false",
+           HM ? "true" : "false", f64 ? "double" : "float", col ? "true" : "false", sparse ? "true" : "false");
   std::string src = "#include \"aq_kernels.cuh\"\nnamespace aq {\n";
-  src += jit_layout_source(L, jit_min_blocks(L, D, multi));
+  src += jit_layout_source(L, jit_min_blocks(L, D));
   src += "}\n";
   // AQ_JIT_SOURCE_DIR (environment, kernel development): compile from the
   // aq_kernels.cuh found in this folder (and the headers it includes from
@@ -258,12 +255,6 @@ int jit_launch(void* fn, unsigned grid, unsigned block, size_t smem, cudaStream_
   c.attrs = &at;
   c.numAttrs = 1;
   return g_dr.launch_ex(&c, (CUfunction)fn, args, nullptr) == CUDA_SUCCESS ? AQ_OK : AQ_E_CUDA;
-}
-
-int jit_launch_cooperative(void* fn, unsigned grid, unsigned block, size_t smem, cudaStream_t st, void** args) {
-  return g_dr.launch_coop((CUfunction)fn, grid, 1, 1, block, 1, 1, (unsigned)smem, (CUstream)st, args) == CUDA_SUCCESS
-             ? AQ_OK
-             : AQ_E_CUDA;
 }
 
 }  // namespace aq

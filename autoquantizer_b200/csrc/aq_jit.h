@@ -12,9 +12,8 @@ namespace aq {
 
 bool jit_available();
 // Compile (or fetch from the in-process cache) k_step<D, HF, HM, R, JitLayout,
-// col, sparse, multi> for layout L; returns a CUfunction, or null with *err set.
-void* jit_k_step(int D, bool HF, bool HM, bool f64, bool col, bool sparse, bool multi, const aq_layout& L,
-                 std::string* err);
+// col, sparse> for layout L; returns a CUfunction, or null with *err set.
+void* jit_k_step(int D, bool HF, bool HM, bool f64, bool col, bool sparse, const aq_layout& L, std::string* err);
 std::string jit_layout_source(const aq_layout& L, int min_blocks);
 
 // Whether the layout-specialized k_step keeps a record's words in registers
@@ -29,26 +28,19 @@ inline bool jit_raw_record(const aq_layout& L) {
   return true;
 }
 inline bool jit_reg_record(const aq_layout& L) { return L.n_words <= kJitRegRecordMaxWords || jit_raw_record(L); }
-// CTAs per SM k_step's registers are budgeted for.  Several passes a launch
-// (MULTI) run one warp's work per scheduler or little more, so registers
-// count and warps do not: 128 a thread (2D, 65,536 quantized: 480 -> 424 us a
-// frame of 32 substeps against 80 registers; 3D, 20,000: 730 -> 695).  Else
-// short records are budgeted for 11 CTAs in 3D (254 us a substep of 2,097,152
-// quantized particles at rest, 261 with 12, 262 with 13: of the bench layout
-// ptxas still makes 80 registers, with fewer spills, and 12 CTAs fit) and 73 in 2D (14; 300,000: 936
-// -> 829 us against 12), long ones 113 (9; 262,144 to 1,200,000 FP32
-// particles: +1.5 to -4 % against 8).
-constexpr int kJitShortRecordMinBlocks = 704 / AQ_CH;
-inline int jit_min_blocks(const aq_layout& L, int D, bool multi) {
-  if (multi) return 512 / AQ_CH;
+// CTAs per SM k_step's registers are budgeted for: short records 11 CTAs in 3D
+// (254 us a substep of 2,097,152 quantized particles at rest, 261 with 12, 262
+// with 13: of the bench layout ptxas still makes 80 registers, with fewer
+// spills, and 12 CTAs fit) and 14 in 2D (73 registers; 300,000: 936 -> 829 us
+// against 12), long ones 9 (113; 262,144 to 1,200,000 FP32 particles: +1.5 to
+// -4 % against 8).
+inline int jit_min_blocks(const aq_layout& L, int D) {
   if (L.n_words > kJitRegRecordMaxWords) return 576 / AQ_CH;
-  return D == 2 ? 896 / AQ_CH : kJitShortRecordMinBlocks;
+  return D == 2 ? 896 / AQ_CH : 704 / AQ_CH;
 }
 int jit_set_smem(void* fn, int bytes);
 int jit_occupancy(void* fn, int block, size_t smem, int* out);
 // launched while the kernel before it in the stream ends (the kernel waits, kernel_begin)
 int jit_launch(void* fn, unsigned grid, unsigned block, size_t smem, cudaStream_t st, void** args);
-// the same with every CTA resident at once (kernels with a grid barrier)
-int jit_launch_cooperative(void* fn, unsigned grid, unsigned block, size_t smem, cudaStream_t st, void** args);
 
 }  // namespace aq

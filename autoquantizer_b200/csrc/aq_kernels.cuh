@@ -113,10 +113,6 @@ struct ColPose {
   int yshift;
 };
 
-// Passes one launch of k_step may make, at most: the default re-binning
-// interval's 16 substeps.
-constexpr int AQ_PASS_MAX = 17;
-
 template <class R>
 struct SimK {
   int res[3], nb[3];
@@ -134,7 +130,7 @@ struct SimK {
   const float* col_nrm;
   R col_omega;
   int col_node_cv;  // 1: collider velocity omega x r from the node itself (sdf_collision_no_arg)
-  ColPose<R> pose[AQ_PASS_MAX];  // per pass of the launch
+  ColPose<R> pose;
   // sparse grids (k_step's SP): grid block -> pool slot (-1: none), the
   // slots handed out so far, each slot's block, the pools' capacity
   int32_t* bptr;
@@ -143,48 +139,28 @@ struct SimK {
   int pool_cap;
 };
 
-// A chain of n_sub substeps is n_sub + 1 passes over the particles: pass 0
-// is P2G of the first substep, pass p in between G2P of substep p and P2G of
-// the next, pass n_sub the last G2P.  One launch makes the passes
-// [pass0, pass1), with a grid barrier between them (k_step's MULTI; all CTAs
-// resident), or the one pass pass0.  Pass p scatters into grid (rot + p) % 3,
-// gathers from (rot + p + 2) % 3 and, with `clear`, zeroes grid
-// (rot + p + 1) % 3 for the next pass; that one was last read by pass p - 1.
+// A chain of n substeps is n + 1 passes over the particles, a launch each:
+// P2G of the first substep, G2P of every substep with P2G of the next, the last
+// G2P.  With three grids a pass also zeroes the one that neither of its halves
+// uses, the next pass's P2G target (SimImpl::launch_chain).
 struct StepArgs {
   uint64_t* words;
   const int32_t* pid;
   const int4* items;
   const int32_t* n_items;
-  int32_t* sync;           // MULTI: [0] barrier arrivals, [32] barrier releases, [64 + k] items claimed in pass
-                           // pass0 + k; zeroed before the launch
-  int32_t* ctr;            // one pass: items claimed, zero at the launch
+  int32_t* ctr;            // items claimed, zero at the launch
   int32_t* ctr_next;       // the next launch's, zeroed by this one
-  void* grid[3];
-  const void* gin;         // pass0's G2P source, P2G target and the grid it clears
-  void* gout;
-  void* gnext;
-  uint64_t sk;             // pass0's dithering key
+  const void* gin;         // G2P source: the sums of the pass before
+  void* gout;              // P2G target, zero
+  void* gnext;             // zeroed by this pass, or null
+  uint64_t sk;             // dithering key of the substep whose G2P this is
   unsigned* status;
-  int32_t* stalled;        // host memory: set by a launch whose barrier ran out of time
-  long long wait_limit;    // cycles a CTA waits in the barrier, at most
   unsigned long long* fallbacks;
   double* rmax;
   double* rmin;
-  uint64_t seed;           // of the dithering generator
-  int64_t step0;           // index of the chain's first substep
   int64_t grid_nodes;      // nodes of a dense grid
-  int pass0, pass1, n_sub, rot, clear, ranges;
-  int do_g2p, do_p2g;      // pass0's halves
+  int do_g2p, do_p2g, ranges;
 };
-
-// Grid k of a pass: 0 its P2G target, 1 the next pass's, 2 its G2P source.
-__host__ __device__ __forceinline__ void* pass_grid(const StepArgs& A, int pass, int k) {
-  const int g = (A.rot + pass + k) % 3;
-  return g == 0 ? A.grid[0] : g == 1 ? A.grid[1] : A.grid[2];
-}
-
-// AQ_SYNC_WORDS: ints of StepArgs::sync
-constexpr int AQ_SYNC_WORDS = 64 + AQ_PASS_MAX;
 
 // Layout from the kernel parameter (nvcc build).
 struct RtLayout {
@@ -642,50 +618,12 @@ __device__ __forceinline__ void kernel_begin() {
   kernel_wait();
 }
 
-// Barrier of all CTAs of the launch (all of them resident: a cooperative
-// launch), the k-th of the launch (k >= 1).  sync[0] counts arrivals, the
-// last one of a round stores the round's number to sync[32], which the others
-// poll (in another cache line than the arrivals).  The fences order the
-// CTA's grid and record writes before it and its reads after it.  False when
-// the wait took longer than `limit` cycles (AQ_WAIT_LIMIT: some 9 s), which no
-// launch whose CTAs are resident comes near.
-constexpr long long AQ_WAIT_LIMIT = 1ll << 34;
-
-__device__ __forceinline__ bool grid_barrier(int32_t* sync, unsigned k, long long limit) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    __threadfence();
-    if ((unsigned)atomicAdd(sync, 1) + 1u == k * gridDim.x) {
-      __threadfence();
-      atomicExch(sync + 32, (int)k);
-    } else {
-      const long long t0 = clock64();
-      unsigned seen;
-      for (;;) {
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(sync + 32) : "memory");
-        if (seen >= k) break;
-        if (clock64() - t0 > limit) {
-          ok = 0;
-          break;
-        }
-        __nanosleep(32);
-      }
-    }
-    __threadfence();
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
-
 // ------------------------------------------------------------ the step
 
 // COL: compiled with the SDF collider (the library's own build always is;
 // the layout-specialized build only when a collider is set).  SP: sparse
 // grids (grid_in / grid_out are node pools reached through K.bptr).
-template <int D, bool HF, bool HM, class R, class LA, bool COL = true, bool SP = false, bool MULTI = false>
+template <int D, bool HF, bool HM, class R, class LA, bool COL = true, bool SP = false>
 __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __grid_constant__ aq_layout Lp,
                                                 const __grid_constant__ SimK<R> K,
                                                 const __grid_constant__ StepArgs A) {
@@ -705,12 +643,7 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
   uint64_t* srec = reinterpret_cast<uint64_t*>(ptile + NWARP * TNP);  // CH x WS: each thread's record (RtLayout)
   __shared__ R s_out[NWARP][OUTSIDE_WORDS];  // a particle outside its tile (gather_outside)
   __shared__ int sbox[6];  // tile-coordinate box of the item's P2G base cells (min[3], max[3])
-  // MULTI: this pass's G2P source, P2G target and dithering key (in shared
-  // memory: held in registers over the whole unit loop they spill)
-  __shared__ const void* s_gin;
-  __shared__ void* s_gout;
-  __shared__ uint64_t s_sk;
-  __shared__ int s_next;   // the CTA's next work item, claimed from A.item_ctr
+  __shared__ int s_next;   // the CTA's next work item, claimed from A.ctr
   __shared__ int sslot[SP ? 27 : 1];  // sparse grids: pool slots of the 3^D blocks around the item's block
   // range detection: the CTA's running max / min per slot (ord_key order)
   __shared__ unsigned long long s_rmax[AQ_MAX_SLOTS], s_rmin[AQ_MAX_SLOTS];
@@ -732,26 +665,18 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
   kernel_wait();
   const int nitems = *A.n_items;
 
-  for (int pass = A.pass0; pass < (MULTI ? A.pass1 : A.pass0 + 1); ++pass) {
-  const bool do_g2p = MULTI ? pass > 0 : A.do_g2p, do_p2g = MULTI ? pass < A.n_sub : A.do_p2g;
+  const bool do_g2p = A.do_g2p, do_p2g = A.do_p2g;
+  const R4* const gin = reinterpret_cast<const R4*>(A.gin);
+  R4* const gout = reinterpret_cast<R4*>(A.gout);
   if (tid == 0) {
     s_next = blockIdx.x;
-    if (MULTI) {
-      s_gout = pass_grid(A, pass, 0);
-      s_gin = pass_grid(A, pass, 2);
-      s_sk = step_key(A.seed, A.step0 + pass - 1);
-    } else if (blockIdx.x == 0) {
-      *A.ctr_next = 0;
-    }
+    if (blockIdx.x == 0) *A.ctr_next = 0;
   }
-  const ColPose<R>& pose = K.pose[MULTI ? pass - A.pass0 : 0];
-  if (A.clear && do_p2g) {  // the next pass's P2G target
+  if (A.gnext) {
     const int64_t nn = SP ? (int64_t)min(*(volatile int32_t*)K.n_alloc, K.pool_cap) * 64 : A.grid_nodes;
-    R4* const gnext = reinterpret_cast<R4*>(MULTI ? pass_grid(A, pass, 1) : A.gnext);
+    R4* const gnext = reinterpret_cast<R4*>(A.gnext);
     for (int64_t j = (int64_t)blockIdx.x * CH + tid; j < nn; j += (int64_t)gridDim.x * CH) gnext[j] = zero4;
   }
-#define AQ_GIN reinterpret_cast<const R4*>(MULTI ? s_gin : A.gin)
-#define AQ_GOUT reinterpret_cast<R4*>(MULTI ? s_gout : A.gout)
 
   // Work items are cell blocks or parts of them: a CTA's first is the one of
   // its own number, the others are claimed one at a time from a counter
@@ -824,15 +749,15 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
         if (ok) {
           if (SP) {
             const int sl = tile_slot<D>(sslot, ob0, ob1, ob2, g0, g1, g2);
-            if (sl >= 0) gv[q] = AQ_GIN[node_in_slot<D>(sl, g0, g1, g2)];
+            if (sl >= 0) gv[q] = gin[node_in_slot<D>(sl, g0, g1, g2)];
           } else {
-            gv[q] = AQ_GIN[cell_index<D>(K.res, g0, g1, g2)];
+            gv[q] = gin[cell_index<D>(K.res, g0, g1, g2)];
           }
         }
       }
 #pragma unroll
       for (int q = 0; q < NL; ++q) {
-        if (gi[q][0] >= 0) gv[q] = grid_op_node<D, R, COL>(K, pose, gv[q], gi[q][0], gi[q][1], gi[q][2]);
+        if (gi[q][0] >= 0) gv[q] = grid_op_node<D, R, COL>(K, K.pose, gv[q], gi[q][0], gi[q][1], gi[q][2]);
         if (jb + q * CH < TNP) gtile[jb + q * CH] = gv[q];
       }
       }
@@ -947,7 +872,7 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
             }
           }
           __syncwarp();
-          gather_outside<D, R, COL, SP>(K, pose, AQ_GIN, sc);
+          gather_outside<D, R, COL, SP>(K, K.pose, gin, sc);
           if (lane == __ffs(om) - 1) {
 #pragma unroll
             for (int d = 0; d < D; ++d) {
@@ -1005,7 +930,7 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
         for (int k = 0; k < D * D; ++k) vals[S::C + k] = nC[k];
         // bit_pack_assign of the new state; vals become the values a later
         // read of the record returns (input of the next P2G)
-        encode_record<NS, R>(L, vals, myrec, particle_key(MULTI ? s_sk : A.sk, pid), (const float*)0, (const double*)0);
+        encode_record<NS, R>(L, vals, myrec, particle_key(A.sk, pid), (const float*)0, (const double*)0);
         store_grec<LA::kWords>(A.words, rec, W, myrec);
         }
       }
@@ -1153,7 +1078,7 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
             }
           }
           __syncwarp();
-          fl |= scatter_outside<D, R, SP>(K, AQ_GOUT, sc);
+          fl |= scatter_outside<D, R, SP>(K, gout, sc);
         }
         __syncwarp();
       }
@@ -1190,27 +1115,19 @@ __global__ void __launch_bounds__(CH, AQ_STEP_MIN_BLOCKS(R, LA)) k_step(const __
           int sl = tile_slot<D>(sslot, ob0, ob1, ob2, g0, g1, g2);
           if (sl < 0) sl = claim_slot(K.bptr, K.n_alloc, K.pool_blk, K.pool_cap, block_of<D>(K.nb, g0, g1, g2));
           if (sl >= 0)
-            red_add_node(AQ_GOUT + node_in_slot<D>(sl, g0, g1, g2), sum.x, sum.y, sum.z, sum.w);
+            red_add_node(gout + node_in_slot<D>(sl, g0, g1, g2), sum.x, sum.y, sum.z, sum.w);
           else
             fl |= AQ_ST_POOL_FULL;
         } else {
-          red_add_node(AQ_GOUT + cell_index<D>(K.res, g0, g1, g2), sum.x, sum.y, sum.z, sum.w);
+          red_add_node(gout + cell_index<D>(K.res, g0, g1, g2), sum.x, sum.y, sum.z, sum.w);
         }
       }
     }
-    if (tid == 0) s_next = (int)gridDim.x + atomicAdd(MULTI ? A.sync + 64 + (pass - A.pass0) : A.ctr, 1);
+    if (tid == 0) s_next = (int)gridDim.x + atomicAdd(A.ctr, 1);
     __syncthreads();
   }
-#undef AQ_GIN
-#undef AQ_GOUT
-  if (MULTI && pass + 1 < A.pass1 && !grid_barrier(A.sync, (unsigned)(pass + 1 - A.pass0), A.wait_limit)) {
-    fl |= AQ_ST_STALLED;
-    break;
-  }
-  }  // passes
   kernel_let_next();
   if (fl) atomicOr(A.status, fl);
-  if (MULTI && (fl & AQ_ST_STALLED)) *reinterpret_cast<volatile int32_t*>(A.stalled) = 1;
   if (nfall) atomicAdd(A.fallbacks, (unsigned long long)nfall);
   if (A.ranges && tid < NS) {  // one merge per CTA and slot
     if (s_rmax[tid] != 0ull) atomic_max_d(A.rmax + tid, ord_val(s_rmax[tid]));

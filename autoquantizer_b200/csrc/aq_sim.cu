@@ -4,10 +4,8 @@
 //
 // Per substep: one pass of k_step (grid_op of the accumulated grid as each
 // tile is staged, G2P of substep k, P2G of substep k+1 into the next of three
-// grids, the third being cleared for the substep after).  In small scenes the
-// passes between two re-binnings are one cooperative launch with a grid
-// barrier between passes.  Every sort_interval substeps the records are
-// re-binned: k_bin (cell key and rank), an exclusive scan of the per-cell
+// grids, the third being cleared for the substep after).  Every sort_interval
+// substeps the records are re-binned: k_bin (cell key and rank), an exclusive scan of the per-cell
 // counts, k_scatter (records and ids into block-wide slot-major
 // order), k_items (the work items, the largest first; the scan counts them).
 #include <math.h>
@@ -555,37 +553,6 @@ __global__ void __launch_bounds__(256) k_loss(const __grid_constant__ aq_layout 
 
 // ------------------------------------------------------------------ host
 
-// One int of page-locked host memory per simulator, which a launch that gave
-// up waiting sets (StepArgs::stalled) and the host reads without a copy.
-// Handed out of pages of AQ_STALL_PAGE that are kept: mapping one takes longer
-// than all else in setting up a small simulator.
-constexpr int AQ_STALL_PAGE = 1024;
-static std::mutex g_stall_mu;
-static std::vector<int32_t*> g_stall_free;
-
-static int32_t* stall_word() {
-  std::lock_guard<std::mutex> g(g_stall_mu);
-  if (g_stall_free.empty()) {
-    int32_t* page = nullptr;
-    if (cudaHostAlloc((void**)&page, sizeof(int32_t) * AQ_STALL_PAGE, cudaHostAllocPortable | cudaHostAllocMapped) !=
-        cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    for (int k = AQ_STALL_PAGE - 1; k >= 0; --k) g_stall_free.push_back(page + k);
-  }
-  int32_t* w = g_stall_free.back();
-  g_stall_free.pop_back();
-  *w = 0;
-  return w;
-}
-
-static void stall_word_back(int32_t* w) {
-  if (!w) return;
-  std::lock_guard<std::mutex> g(g_stall_mu);
-  g_stall_free.push_back(w);
-}
-
 struct SimBase {
   virtual ~SimBase() {}
   virtual int substeps(int n, cudaStream_t st) = 0;
@@ -620,12 +587,10 @@ struct aq_sim {
   int32_t *keys = nullptr, *ranks = nullptr, *cell_count = nullptr, *cell_start = nullptr, *scan_sums = nullptr;
   int4* items = nullptr;
   int32_t* n_items = nullptr;  // [0] item count, then k_items' bucket sizes and cursors
-  int32_t* sync = nullptr;  // k_step's grid barrier and claim counters (StepArgs::sync), then ctr's two
-  int64_t step_launches = 0;  // launches without MULTI
+  int32_t* item_ctr = nullptr;  // [2] k_step's item claim counters
+  int64_t step_launches = 0;
   int64_t max_items = 0;
   unsigned* status = nullptr;
-  int32_t* stalled = nullptr;  // host memory (stall_word)
-  long long wait_limit = aq::AQ_WAIT_LIMIT;
   unsigned long long* fallbacks = nullptr;
   double *rmax = nullptr, *rmin = nullptr;
   double* dloss = nullptr;
@@ -690,8 +655,6 @@ struct aq_sim {
   int prof_on = 0;
   cudaEvent_t* prof_ev[2] = {nullptr, nullptr};  // [PROF_CAP * 2]
   int prof_n[2] = {0, 0};
-  int64_t prof_passes = 0;  // passes of the timed k_step launches
-  bool multi = false;  // jit_fn makes several passes in a cooperative launch (k_step's MULTI)
 };
 
 namespace aq {
@@ -934,89 +897,68 @@ struct SimImpl final : SimBase {
     if (do_p2g && clear && (rc_ = clear_grid(gout, st))) return rc_;
     StepArgs a;
     memset(&a, 0, sizeof(a));
-    a.pass0 = do_g2p ? 1 : 0;
-    a.pass1 = a.pass0 + 1;
-    a.n_sub = do_p2g ? 2 : 1;
-    a.grid[0] = do_g2p ? gin : gout;  // pass p scatters into grid p % 3 and gathers from the one before
-    a.grid[1] = gout;
+    a.do_g2p = do_g2p;
+    a.do_p2g = do_p2g;
+    a.gin = gin;
+    a.gout = gout;
     return launch(a, st);
   }
 
-  // Passes [pass0, pass1) of a chain of n_sub substeps on the three grids.
-  int launch_chain(int pass0, int pass1, int n_sub, cudaStream_t st) {
+  // Pass p of a chain of n substeps on the three grids: scatters into grid
+  // (rot + p) % 3, gathers from (rot + p + 2) % 3 and zeroes (rot + p + 1) % 3
+  // for the pass after; that one was last read by the pass before.
+  int launch_chain(int p, int n, cudaStream_t st) {
+    void* const* g = s->grid;
     StepArgs a;
     memset(&a, 0, sizeof(a));
-    a.pass0 = pass0;
-    a.pass1 = pass1;
-    a.n_sub = n_sub;
-    a.rot = s->rot;
-    a.clear = 1;
-    for (int k = 0; k < 3; ++k) a.grid[k] = s->grid[k];
+    a.do_g2p = p > 0;
+    a.do_p2g = p < n;
+    a.gin = g[(s->rot + p + 2) % 3];
+    a.gout = g[(s->rot + p) % 3];
+    if (a.do_p2g) a.gnext = g[(s->rot + p + 1) % 3];
     return launch(a, st);
   }
 
-  // The arguments every launch has; the launch itself.  a's chain starts at
-  // the simulator's current substep.
+  // The arguments every launch has; the launch itself.  G2P is that of the
+  // simulator's current substep.
   int launch(StepArgs& a, cudaStream_t st) {
     aq_sim* S_ = s;
     a.words = S_->words[S_->cur];
     a.pid = S_->pid[S_->cur];
     a.items = S_->items;
     a.n_items = S_->n_items;
-    a.sync = S_->sync;
     a.status = S_->status;
-    a.stalled = S_->stalled;
-    a.wait_limit = S_->wait_limit;
     a.fallbacks = S_->fallbacks;
     a.rmax = S_->rmax;
     a.rmin = S_->rmin;
-    a.seed = S_->P.seed;
-    a.step0 = S_->step;
+    a.sk = step_key(S_->P.seed, S_->step);
     a.grid_nodes = S_->ncell;
     a.ranges = S_->ranges_on;
     K.bptr = S_->bptr;
     K.n_alloc = S_->n_alloc;
     K.pool_blk = S_->pool_blk;
     K.pool_cap = S_->pool_cap;
-    if (K.col_on) {  // step_collider (mpm_solver.py:1542-1547) after every substep
-      double theta = S_->col_theta, height = S_->col_height;
-      for (int p = 0; p < a.pass1; ++p) {
-        if (p > 1) {
-          theta += S_->col_omega * S_->P.dt;
-          height += S_->col_rate * S_->P.dt;
-        }
-        if (p < a.pass0) continue;
-        K.pose[p - a.pass0].c = (R)cos(theta);
-        K.pose[p - a.pass0].s = (R)sin(theta);
-        K.pose[p - a.pass0].yshift = (int)(height / S_->P.dx + 0.5);
-      }
+    if (K.col_on) {
+      K.pose.c = (R)cos(S_->col_theta);
+      K.pose.s = (R)sin(S_->col_theta);
+      K.pose.yshift = (int)(S_->col_height / S_->P.dx + 0.5);
     }
-    const int passes = a.pass1 - a.pass0;
-    a.gin = pass_grid(a, a.pass0, 2);
-    a.gout = pass_grid(a, a.pass0, 0);
-    a.gnext = pass_grid(a, a.pass0, 1);
-    a.sk = step_key(a.seed, a.step0 + a.pass0 - 1);
-    a.do_g2p = a.pass0 > 0;
-    a.do_p2g = a.pass0 < a.n_sub;
     // CTAs: one per work item, and with few items on a large grid enough for
     // the clear (16 nodes a thread; 256^3 nodes, 16 substeps of one particle:
     // 65 ms on the two CTAs of its items, 0.92 with these)
     int64_t busy = items_bound();
-    if (a.clear && !S_->P.sparse) busy = std::max(busy, (S_->ncell + 16 * CH - 1) / (16 * CH));
+    if (a.gnext && !S_->P.sparse) busy = std::max(busy, (S_->ncell + 16 * CH - 1) / (16 * CH));
     const int ctas = (int)std::min<int64_t>(S_->step_grid, busy);
-    if (S_->multi) AQ_CUDA_TRY(cudaMemsetAsync(S_->sync, 0, sizeof(int32_t) * AQ_SYNC_WORDS, st));
-    // two claim counters alternate between launches without MULTI; each launch
-    // zeroes the one the next launch uses (both start at zero)
-    a.ctr = S_->sync + AQ_SYNC_WORDS + (S_->step_launches & 1);
-    a.ctr_next = S_->sync + AQ_SYNC_WORDS + ((S_->step_launches + 1) & 1);
-    if (!S_->multi) ++S_->step_launches;
+    // two claim counters alternate between launches; each launch zeroes the
+    // one the next launch uses (both start at zero)
+    a.ctr = S_->item_ctr + (S_->step_launches & 1);
+    a.ctr_next = S_->item_ctr + ((S_->step_launches + 1) & 1);
+    ++S_->step_launches;
     const bool prof = S_->prof_on && S_->prof_n[0] < aq_sim::PROF_CAP;
     if (prof) AQ_CUDA_TRY(cudaEventRecord(S_->prof_ev[0][2 * S_->prof_n[0]], st));
     void* args[] = {(void*)&S_->L, (void*)&K, (void*)&a};
     if (S_->jit_fn) {
-      const int rc = passes > 1 ? jit_launch_cooperative(S_->jit_fn, ctas, CH, S_->step_smem, st, args)
-                                : jit_launch(S_->jit_fn, ctas, CH, S_->step_smem, st, args);
-      if (rc != AQ_OK) {
+      if (jit_launch(S_->jit_fn, ctas, CH, S_->step_smem, st, args) != AQ_OK) {
         set_last_cuda_error(cudaErrorLaunchFailure, "cuLaunchKernel(k_step)");
         return AQ_E_CUDA;
       }
@@ -1026,10 +968,7 @@ struct SimImpl final : SimBase {
       const PdlConfig c(ctas, CH, S_->step_smem, st);
       AQ_CUDA_TRY(cudaLaunchKernelExC(&c.c, f, args));
     }
-    if (prof) {
-      AQ_CUDA_TRY(cudaEventRecord(S_->prof_ev[0][2 * S_->prof_n[0]++ + 1], st));
-      S_->prof_passes += passes;
-    }
+    if (prof) AQ_CUDA_TRY(cudaEventRecord(S_->prof_ev[0][2 * S_->prof_n[0]++ + 1], st));
     S_->launches += 1;
     return AQ_OK;
   }
@@ -1167,7 +1106,7 @@ struct SimImpl final : SimBase {
     if (S_->grid[2])
       AQ_CUDA_TRY(cudaMemsetAsync(S_->grid[S_->rot], 0,
                                   sizeof(R4) * (S_->P.sparse ? (size_t)S_->pool_cap * 64 : (size_t)S_->ncell), st));
-    AQ_CUDA_TRY(cudaMemsetAsync(S_->sync + AQ_SYNC_WORDS, 0, 2 * sizeof(int32_t), st));
+    AQ_CUDA_TRY(cudaMemsetAsync(S_->item_ctr, 0, 2 * sizeof(int32_t), st));
     return AQ_OK;
   }
 
@@ -1192,12 +1131,12 @@ struct SimImpl final : SimBase {
       // m + 1 passes: P2G of the first substep, G2P of each fused with P2G
       // of the next, G2P of the last (grid_op applied as tiles are staged)
       if (S_->grid[2]) {
-        const int per = S_->multi ? AQ_PASS_MAX : 1;
-        for (int p = 0; p <= m; p += per)
-          if ((rc = launch_chain(p, std::min(p + per, m + 1), m, st))) return rc;
+        for (int p = 0; p <= m; ++p) {
+          if ((rc = launch_chain(p, m, st))) return rc;
+          if (p) advance();
+        }
         S_->last_grid = (S_->rot + m + 2) % 3;
         S_->rot = (S_->rot + m) % 3;
-        for (int k = 0; k < m; ++k) advance();
       } else {
         int a = 0;
         if ((rc = launch_step(0, 1, nullptr, S_->grid[a], st))) return rc;
@@ -1243,19 +1182,11 @@ struct SimImpl final : SimBase {
 // select the library's own k_step, and size its persistent grid.
 template <int D, bool HF, bool HM, class R>
 static int setup_step_kernel(aq_sim* s, size_t smem_jit, size_t smem_aot, bool col) {
-  int occ = 0, dev = 0, coop = 0;
+  int occ = 0;
   s->jit_fn = nullptr;
-  AQ_CUDA_TRY(cudaGetDevice(&dev));
-  AQ_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
   if (s->P.jit) {
     const size_t smem = smem_jit;
-    // Several passes a launch where a CTA's share of the records is one
-    // 64-record item or less: there the launches and their gaps weigh (2D,
-    // 8,192 particles: 13 % of a substep; 65,536: 11 %; 3D, 60,000: 8 %),
-    // while with more units per warp the pass loop's registers cost what it
-    // saves (262,144: +-3 %, 2,097,152: 3 % slower).
-    s->multi = coop && s->cap <= (int64_t)64 * kJitShortRecordMinBlocks * num_sms();
-    s->jit_fn = jit_k_step(D, HF, HM, sizeof(R) == 8, col, s->P.sparse != 0, s->multi, s->L, &s->jit_error);
+    s->jit_fn = jit_k_step(D, HF, HM, sizeof(R) == 8, col, s->P.sparse != 0, s->L, &s->jit_error);
     if (s->jit_fn && (jit_set_smem(s->jit_fn, (int)smem) != AQ_OK || jit_occupancy(s->jit_fn, CH, smem, &occ) != AQ_OK)) {
       s->jit_fn = nullptr;
       s->jit_error = "cuFuncSetAttribute/occupancy failed";
@@ -1263,7 +1194,6 @@ static int setup_step_kernel(aq_sim* s, size_t smem_jit, size_t smem_aot, bool c
     s->step_smem = smem;
   }
   if (!s->jit_fn) {
-    s->multi = false;
     const size_t smem = smem_aot;
     s->step_smem = smem;
     if (s->P.sparse) {
@@ -1318,7 +1248,6 @@ static void free_sim(aq_sim* s) {
     pool_free(s->cub_tmp, 0);
   }
   pool_free(s->slab, 0);
-  stall_word_back(s->stalled);
   if (s->h_words) cudaFreeHost(s->h_words);
   if (s->words_dl) cudaFree(s->words_dl);
   if (s->words_up[1]) cudaFree(s->words_up[1]);
@@ -1329,24 +1258,6 @@ static void free_sim(aq_sim* s) {
   if (s->up_st) cudaStreamDestroy(s->up_st);
   if (s->down_st) cudaStreamDestroy(s->down_st);
   delete s;
-}
-
-static int sim_check(const aq_sim* s) {
-  return *reinterpret_cast<const volatile int32_t*>(s->stalled) ? AQ_E_STALLED : AQ_OK;
-}
-
-// The state is set anew: after a launch that gave up, its status flag goes and
-// the next chain clears its grids.
-static int sim_recover(aq_sim* s) {
-  if (sim_check(s) == AQ_OK) return AQ_OK;
-  unsigned f = 0;
-  AQ_CUDA_TRY(cudaDeviceSynchronize());
-  AQ_CUDA_TRY(cudaMemcpy(&f, s->status, sizeof(f), cudaMemcpyDeviceToHost));
-  f &= ~AQ_ST_STALLED;
-  AQ_CUDA_TRY(cudaMemcpy(s->status, &f, sizeof(f), cudaMemcpyHostToDevice));
-  *s->stalled = 0;
-  s->stale = true;
-  return AQ_OK;
 }
 
 // Encode `count` particles from values into the current records at position
@@ -1409,8 +1320,7 @@ static int sim_create(const aq_params* P, const aq_layout* L, bool streamed, aq_
     delete s;
     return AQ_E_LIMIT;  // the dense binning's cell keys are int32
   }
-  s->stalled = stall_word();
-  if (!s->stalled || cudaGetDevice(&s->device) != cudaSuccess) {
+  if (cudaGetDevice(&s->device) != cudaSuccess) {
     free_sim(s);
     return AQ_E_NOMEM;
   }
@@ -1468,7 +1378,7 @@ static int sim_create(const aq_params* P, const aq_layout* L, bool streamed, aq_
   }
   alloc((void**)&s->items, sizeof(int4) * s->max_items);
   if (P->sparse) alloc((void**)&s->n_items, sizeof(int32_t) * (1 + 2 * IB));
-  alloc((void**)&s->sync, sizeof(int32_t) * (AQ_SYNC_WORDS + 2));
+  alloc((void**)&s->item_ctr, 2 * sizeof(int32_t));
   alloc((void**)&s->status, sizeof(unsigned));
   alloc((void**)&s->fallbacks, sizeof(unsigned long long));
   alloc((void**)&s->rmax, sizeof(double) * AQ_MAX_SLOTS);
@@ -1520,7 +1430,7 @@ static int sim_create(const aq_params* P, const aq_layout* L, bool streamed, aq_
   if (e == cudaSuccess) e = cudaMemset(s->words[0], 0, sizeof(uint64_t) * (grouped_words(n, s->W) + 2));
   if (e == cudaSuccess) e = cudaMemset(s->status, 0, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(s->fallbacks, 0, sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMemset(s->sync, 0, sizeof(int32_t) * (AQ_SYNC_WORDS + 2));
+  if (e == cudaSuccess) e = cudaMemset(s->item_ctr, 0, 2 * sizeof(int32_t));
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "cudaMemset");
     free_sim(s);
@@ -1653,7 +1563,6 @@ int aq_sim_append(aq_sim* s, const void* values, int32_t values_f64, int64_t cou
   cudaStream_t st = as_stream(stream);
   const int64_t base = s->n;
   int rc;
-  if ((rc = sim_check(s))) return rc;
   if ((rc = store_values(s, values, values_f64, base, count, st))) return rc;
   s->n = base + count;
   s->sorted = false;
@@ -1689,7 +1598,6 @@ int aq_sim_set_state(aq_sim* s, const void* values, int32_t values_f64, void* st
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
   int rc;
-  if ((rc = sim_recover(s))) return rc;
   if ((rc = store_values(s, values, values_f64, 0, s->n, st))) return rc;
   s->sorted = false;
   s->launches += 1;
@@ -1700,8 +1608,6 @@ int aq_sim_get_state(aq_sim* s, void* values, int32_t values_f64, void* stream) 
   if (!s || !values) return AQ_E_ARG;
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
-  const int rc = sim_check(s);
-  if (rc != AQ_OK) return rc;
   AQ_CUDA_TRY(rec_fetch(s->L, s->words[s->cur], s->pid[s->cur], values, values_f64 != 0, s->n, st));
   s->launches += 1;
   return AQ_OK;
@@ -1778,15 +1684,13 @@ int aq_sim_field_stats(aq_sim* s, const void* ref, int32_t ref_f64, double* h_ou
   s->launches += 1;
   AQ_CUDA_TRY(cudaMemcpyAsync(h_out, s->dstats, sizeof(double) * 5 * s->NS, cudaMemcpyDeviceToHost, st));
   AQ_CUDA_TRY(cudaStreamSynchronize(st));
-  return sim_check(s);
+  return AQ_OK;
 }
 
 int aq_sim_set_words(aq_sim* s, const uint64_t* words, void* stream) {
   if (!s || !words) return AQ_E_ARG;
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
-  const int rc = sim_recover(s);
-  if (rc != AQ_OK) return rc;
   k_iota<<<grid_for(s->n, 256), 256, 0, st>>>(s->pid[s->cur], s->n);
   AQ_CUDA_TRY(cudaGetLastError());
   AQ_CUDA_TRY(rec_group(words, s->words[s->cur], s->n, s->W, st));
@@ -1799,8 +1703,6 @@ int aq_sim_get_words(aq_sim* s, uint64_t* words, void* stream) {
   if (!s || !words) return AQ_E_ARG;
   if (s->chunk) return AQ_E_STATE;  // streamed: the state is in host memory
   cudaStream_t st = as_stream(stream);
-  const int rc = sim_check(s);
-  if (rc != AQ_OK) return rc;
   AQ_CUDA_TRY(rec_ungroup(s->words[s->cur], s->pid[s->cur], words, s->n, s->W, 0, st));
   s->launches += 1;
   return AQ_OK;
@@ -1809,15 +1711,11 @@ int aq_sim_get_words(aq_sim* s, uint64_t* words, void* stream) {
 int aq_sim_substeps(aq_sim* s, int32_t n, void* stream) {
   if (!s || n < 0) return AQ_E_ARG;
   if (n == 0) return AQ_OK;
-  const int rc = sim_check(s);
-  if (rc != AQ_OK) return rc;
   return s->impl->substeps(n, as_stream(stream));
 }
 
 int aq_sim_grid_mass(aq_sim* s, float* d_out, void* stream) {
   if (!s || !d_out) return AQ_E_ARG;
-  const int rc = sim_check(s);
-  if (rc != AQ_OK) return rc;
   cudaStream_t st = as_stream(stream);
   const unsigned nb = (unsigned)std::min<int64_t>(grid_for(s->ncell, 256), (int64_t)num_sms() * 8);
   if (s->P.sparse) {
@@ -1850,8 +1748,7 @@ int aq_sim_grid_mass(aq_sim* s, float* d_out, void* stream) {
 int aq_sim_loss(aq_sim* s, int32_t kind, double* h_out, void* stream) {
   if (!s || !h_out || kind != 0) return AQ_E_ARG;
   s->launches += 1;
-  const int rc = s->impl->loss(h_out, as_stream(stream));
-  return rc != AQ_OK ? rc : sim_check(s);
+  return s->impl->loss(h_out, as_stream(stream));
 }
 
 int aq_sim_ranges_enable(aq_sim* s, int32_t on, void* stream) {
@@ -1877,7 +1774,7 @@ int aq_sim_ranges_get(aq_sim* s, double* h_max, double* h_min, void* stream) {
   AQ_CUDA_TRY(cudaMemcpyAsync(h_max, s->rmax, sizeof(double) * s->NS, cudaMemcpyDeviceToHost, st));
   AQ_CUDA_TRY(cudaMemcpyAsync(h_min, s->rmin, sizeof(double) * s->NS, cudaMemcpyDeviceToHost, st));
   AQ_CUDA_TRY(cudaStreamSynchronize(st));
-  return sim_check(s);
+  return AQ_OK;
 }
 
 int aq_sim_status(aq_sim* s, uint32_t* h_flags, int64_t* h_fallbacks, int32_t clear, void* stream) {
@@ -1895,17 +1792,6 @@ int aq_sim_status(aq_sim* s, uint32_t* h_flags, int64_t* h_fallbacks, int32_t cl
   if (h_flags) *h_flags = f;
   if (h_fallbacks) *h_fallbacks = (int64_t)fb;
   return AQ_OK;
-}
-
-int aq_sim_wait_limit(aq_sim* s, int64_t cycles) {
-  if (!s || cycles < 1) return AQ_E_ARG;
-  s->wait_limit = cycles;
-  return AQ_OK;
-}
-
-int aq_sim_check(const aq_sim* s) {
-  if (!s) return AQ_E_ARG;
-  return sim_check(s);
 }
 
 int aq_sim_step_count(const aq_sim* s, int64_t* h_out) {
@@ -1943,7 +1829,6 @@ int aq_sim_profile_enable(aq_sim* s, int32_t on) {
       }
       s->prof_n[k] = 0;
     }
-    s->prof_passes = 0;
   }
   s->prof_on = on ? 1 : 0;
   return AQ_OK;
@@ -1961,8 +1846,7 @@ int aq_sim_profile_get(aq_sim* s, int32_t which, double* h_total_ms, int64_t* h_
   }
   s->prof_n[which] = 0;
   *h_total_ms = tot;
-  *h_launches = which == 0 ? s->prof_passes : n;
-  if (which == 0) s->prof_passes = 0;
+  *h_launches = n;
   return AQ_OK;
 }
 

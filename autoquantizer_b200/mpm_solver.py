@@ -537,14 +537,8 @@ class MPMSolver:
 
     def state_values(self, f64=True):
         """Decoded state, particle order, (n x n_slots) numpy array."""
-        v = self.state_tensor(f64).cpu().numpy()
-        self._check_stalled()
-        return v
-
-    def _check_stalled(self):
-        """After the host has waited for the substeps: raise if one of their
-        launches gave up (aq_sim_check)."""
-        _lib.check(_lib.lib().aq_sim_check(self._sim), "aq_sim_check")
+        t = self.state_tensor(f64)
+        return t.cpu().numpy()
 
     def state_tensor(self, f64=True):
         import torch
@@ -563,9 +557,7 @@ class MPMSolver:
         out = torch.empty((self.current_idx, self.layout().n_words), dtype=torch.int64, device="cuda")
         _lib.check(_lib.lib().aq_sim_get_words(self._sim, C.c_void_p(out.data_ptr()), _lib.stream_ptr()),
                    "aq_sim_get_words")
-        words = out.cpu().numpy().view(np.uint64)
-        self._check_stalled()
-        return words
+        return out.cpu().numpy().view(np.uint64)
 
     def set_words(self, words):
         import torch

@@ -46,14 +46,12 @@ extern "C" {
 #define AQ_E_NOMEM (-4)    /* device allocation failed */
 #define AQ_E_STATE (-5)    /* call not valid in the current state */
 #define AQ_E_LIMIT (-6)    /* size above a documented maximum */
-#define AQ_E_STALLED (-7)  /* a substep launch gave up waiting for its own blocks: set the state anew */
 
 /* device status flags (aq_sim_status) */
 #define AQ_ST_OUT_OF_DOMAIN 0x1u  /* a particle stencil left the grid; base clamped */
 #define AQ_ST_NAN 0x2u            /* a NaN position was met; base clamped */
 #define AQ_ST_FALLBACK 0x4u       /* a particle left its shared-memory tile (informational) */
 #define AQ_ST_POOL_FULL 0x8u      /* sparse grid: no free node block; contributions to it were dropped */
-#define AQ_ST_STALLED 0x10u       /* a substep launch gave up waiting for its own blocks: the state is not valid */
 
 /* scalar kinds: quantized types of the reference
  *   AQ_FIXED      ti.quant.fixed(frac=bits, signed, range, offset)
@@ -315,16 +313,6 @@ int aq_sim_ranges_get(aq_sim* sim, double* h_max, double* h_min, void* stream);
  * stream.  clear != 0 resets them. */
 int aq_sim_status(aq_sim* sim, uint32_t* h_flags, int64_t* h_fallbacks,
                   int32_t clear, void* stream);
-/* In small scenes one launch makes several passes over the particles, with a
- * barrier between them.  A launch whose blocks waited longer than this many
- * SM clock cycles for one another (0 < cycles; default 2^34, some 9 s, which
- * no launch comes near) gives up: AQ_ST_STALLED is set, and from then on
- * substeps, append and every call that reads the state return AQ_E_STALLED
- * until aq_sim_set_state or aq_sim_set_words sets it anew.
- * aq_sim_check returns AQ_E_STALLED once a launch that the host has waited
- * for gave up, AQ_OK else; it does not synchronize. */
-int aq_sim_wait_limit(aq_sim* sim, int64_t cycles);
-int aq_sim_check(const aq_sim* sim);
 int aq_sim_step_count(const aq_sim* sim, int64_t* h_out);
 /* Set the substep counter (the dithering generator's step index), e.g. when
  * resuming from saved records so that the continuation draws the same
@@ -338,12 +326,10 @@ int aq_sim_kernel_is_jit(const aq_sim* sim, int32_t* h_out);
 int aq_sim_launches(const aq_sim* sim, int64_t* h_out);
 
 /* Kernel timing with CUDA events recorded around each launch of the fused
- * substep kernel (k_step) and of the grid kernel (k_grid) on the stream they
- * run on.  No reference counterpart (the reference profiles through CUPTI,
+ * substep kernel (k_step) and each grid clear on the stream they run on.  No reference counterpart (the reference profiles through CUPTI,
  * taichi_submission/taichi/program/kernel_profiler.h:46).  which: 0 = k_step,
- * counted in passes over the particles (one launch may make several), 1 = the
- * grid clears that are launches of their own.  profile_get synchronizes and
- * resets the accumulators. */
+ * 1 = the grid clears that are launches of their own.  profile_get synchronizes
+ * and resets the accumulators. */
 int aq_sim_profile_enable(aq_sim* sim, int32_t on);
 int aq_sim_profile_get(aq_sim* sim, int32_t which, double* h_total_ms, int64_t* h_launches);
 
