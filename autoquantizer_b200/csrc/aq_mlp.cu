@@ -605,7 +605,7 @@ int aq_mlp_forward(int32_t in, int32_t h, int32_t out, const float* d_params, co
 
 int aq_mlp_backward(int32_t in, int32_t h, int32_t out, const uint16_t* d_params_bf16, const float* d_x, int32_t B,
                     const float* d_act, const float* d_dy, float* d_grad, void* stream) {
-  if (!d_params_bf16 || !d_x || !d_act || !d_dy || !d_grad || B < 1) return AQ_E_ARG;
+  if (!d_params_bf16 || !d_x || !d_act || !d_dy || !d_grad || B < 1 || in < 1 || h < 1 || out < 1) return AQ_E_ARG;
   cudaStream_t st = as_stream(stream);
   const MlpOffsets o = offsets(in, h, out);
   const __nv_bfloat16* wb = (const __nv_bfloat16*)d_params_bf16;
