@@ -48,7 +48,7 @@ namespace aq {
 
 template <class R>
 struct AdK {
-  int res[3], D, NS, HF, mat;
+  int res[3], mat;
   R inv_dx, dx, dt, p_mass, kst, four_inv_dx2, grav, mu, lam;
   int wlo[3], whi[3];  // walls: node indices below wlo / above whi
   // rotating SDF collider (3D; col_on = 0: none), the fields collider_at
@@ -231,7 +231,7 @@ __device__ __forceinline__ void ad_sigma_bwd(const AdK<R>& K, const R* s, const 
 // ------------------------------------------------------------- layout
 //
 // States and their adjoints inside the library: the particles in the order
-// of ad_sort_key, in groups of 32 that hold slot s of all 32 side by side, so
+// of k_ad_keys, in groups of 32 that hold slot s of all 32 side by side, so
 // that a warp's loads and stores of a slot are one coalesced access.
 
 __host__ __device__ __forceinline__ int64_t ad_padded(int64_t n) { return (n + 31) & ~int64_t(31); }
@@ -484,7 +484,7 @@ struct AdSrc {
 // Every sum over a particle's nodes is of terms of these offsets, node by
 // node.  Taking fx out of the sums (sum w g off - fx sum w g, and m v - A fx +
 // A off) is a third fewer operations (3D falling block, 262,144 particles,
-// FP32, 32 substeps forward and back: 6.5 ms against 7.3), but the difference
+// FP32, 32 substeps forward and back: 6.5 ms against 7.4), but the difference
 // of two larger sums: the FP32 error of the adjoint of C was 1.3 to 2.3 times
 // this form's, that of the new C up to 1.6 times (2D and 3D fluid).
 template <int D, class R>
@@ -1123,9 +1123,6 @@ struct AdImpl final : AdBase {
       K.wlo[d] = wall_lo(P.lb[d]);
       K.whi[d] = wall_hi(P.ub[d]);
     }
-    K.D = D;
-    K.NS = adj->NS;
-    K.HF = HF;
     K.mat = P.mat[0].kind;
     K.inv_dx = (R)(1.0 / P.dx);
     K.dx = (R)P.dx;
@@ -1213,7 +1210,7 @@ struct AdImpl final : AdBase {
   }
 };
 
-// Sort the particles (ad_sort order): a->perm[sorted position] = caller's index.
+// Sort the particles (k_ad_keys's order): a->perm[sorted position] = caller's index.
 static int ad_make_perm(aq_adjoint* a, const void* d_s0, cudaStream_t st) {
   const int bs = a->D == 3 ? 4 : 8;
   int64_t nblk = 1;

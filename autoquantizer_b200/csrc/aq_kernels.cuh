@@ -17,22 +17,24 @@
 //              (grec_word, aq_codec.cuh): a warp's record loads and stores
 //              are coalesced 16-byte vectors.  A particle-id array moves
 //              with the records.
-//   grids    : two dense grids of R4 nodes (m, m v), row-major: one holds
-//              the P2G sums of substep k (grid_op is applied as tiles are
-//              staged from it), the other receives the P2G of substep k+1
-//              (cleared by the host before the launch).
-//   binning  : per-cell counts/offsets, per-particle key and rank, and one
-//              work item per occupied block (block, first record, count).
+//   grids    : dense grids of R4 nodes (m, m v), row-major: one holds the P2G
+//              sums of substep k (grid_op is applied as tiles are staged from
+//              it), the next receives the P2G of substep k+1, the third is
+//              cleared by the launch for the substep after (two where a third
+//              does not fit, the target cleared by a memset).
+//   binning  : per-cell counts/offsets, per-particle key and rank, and the
+//              work items (block, first record, count): an occupied block's
+//              records or, in small scenes, equal parts of them.
 //
 // k_step, persistent CTAs of CH = 64 threads (two warps) claiming work items
-// (whole cell blocks, the fullest first) from a counter:
+// (the largest first) from a counter:
 //   1. stage the block's grid tile (7^3 nodes in 3D: the block, the cell
 //      below it and the stencil) in shared memory, applying grid_op (and
 //      the SDF collider when compiled in) to every node (G2P source);
 //   2. the warps take the block's records 32 at a time (units), without
 //      CTA barriers between units; per unit each lane loads its record into
-//      registers (layout-specialized build, short records) or its shared
-//      slot, and
+//      registers (layout-specialized build, short or unquantized records) or
+//      its shared slot, and
 //      a. G2P of substep k: gather 3^d nodes (z-separable sums), new v, C,
 //         x, F|J; bit_pack_assign into the record, which also yields the
 //         values a later decode returns; record written back to HBM;
@@ -77,8 +79,9 @@ struct Geo {
   static constexpr int BS = D == 3 ? 4 : 8;          // block edge (cells)
   // tile edge: base cells of a block's particles span the block and the
   // cell below it, plus the 3-node stencil; 2D keeps one cell of slack for
-  // drift between re-binnings (3D particles that drift out take the global
-  // fallback path: a 7-node tile leaves room in L1 for the 4 CTAs per SM)
+  // drift between re-binnings (3D particles that drift out are done on the
+  // global grid, gather_outside and scatter_outside: with a 7-node tile a CTA
+  // takes 17.5 KB and registers set how many fit)
   static constexpr int T = D == 3 ? BS + 3 : BS + 4;
   // stride of the slowest tile axis, padded to 4 mod 8 nodes so that
   // neighbouring x planes fall in different 16-byte bank groups

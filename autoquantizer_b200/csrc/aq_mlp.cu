@@ -262,7 +262,9 @@ static MlpOffsets offsets(int in, int h, int out) {
 //   k_mlp_dz        the same for the hidden layers' output gradients
 //   k_mlp_dw        all weight and bias gradients, a warp per 16 x 32 tile
 // Every product is the same m16n8k16 as k_gemm_bf16's, in the same order of k,
-// so the results are the same bits.  A weight fragment is used once per CTA,
+// so outputs, hidden gradients and, up to DW_ROWS rows, weight gradients are
+// those of the layer-by-layer kernels; bias gradients (four strided sums) and
+// longer batches (a sum per segment) are added up in another FP32 order.  A weight fragment is used once per CTA,
 // so it goes from L2 to registers directly.
 // Rule (mlp_fused): in and h multiples of 64 (whole chunks of four k-steps)
 // and at most 512 (16 rows of two layers fit 48 KB), out at most 128, weights

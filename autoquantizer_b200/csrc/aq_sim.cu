@@ -738,9 +738,10 @@ struct SimImpl final : SimBase {
   int item_max() const { return (int)std::max<int64_t>(64, (s->n / s->step_grid + 63) / 64 * 64); }
 
   // Small parts for the end of the launch (item_part) where a CTA has little
-  // more than one item's worth: 262,144 to 550,000 particles 3 to 8 % faster;
-  // with several items a CTA the extra tiles cost more (800,000: 2 % slower,
-  // 2,097,152: 5 %).
+  // more than one item's worth: 3D, 262,144 to 550,000 particles 3 to 8 %
+  // faster; with several items a CTA the extra tiles cost more (800,000: 2 %
+  // slower, 2,097,152: 5 %).  2D, where the line lies at 829,000: 400,000 3 %
+  // slower, 550,000 to 820,000 1 to 7 % faster (FP64 2 % slower to 20 % faster).
   int item_tail() const { return s->n < (int64_t)400 * s->step_grid ? 128 : 0; }
 
   // Work items there can be, at most: a launch needs no more CTAs.
@@ -1333,8 +1334,8 @@ static int sim_create(const aq_params* P, const aq_layout* L, bool streamed, aq_
   const int64_t n = s->n;
   const int nt = (int)((s->nkeys + SCAN_TILE - 1) / SCAN_TILE);
   cudaError_t e = cudaSuccess;
-  // every buffer is carved from one device allocation (one cudaMalloc per
-  // simulator, given back at destroy), each on a 256-byte boundary
+  // every buffer is carved from one allocation of the pool, given back at
+  // destroy, each on a 256-byte boundary
   struct Part {
     void** p;
     size_t off;
