@@ -258,8 +258,8 @@ __device__ __forceinline__ void ad_load(const R* st, int64_t p, R (&s)[NS]) {
 // and to the grid.  No two warps share a tile, so there is no CTA barrier.
 // Particle by particle with scalar global atomics, from rows of 96 bytes and
 // with the grid's operation in kernels of its own, a substep of the 3D
-// falling block (262,144 particles, FP32) took 127 us forward (now 49) and
-// 287 us backward, recomputed sums and squares included (now 124).
+// falling block (262,144 particles, FP32) took 127 us forward (now 46) and
+// 287 us backward, recomputed sums and squares included (now 144).
 //
 // Half a block's cells (4 x 2 x 4, and 4 x 8 in 2D) reach 6 x 4 x 6 = 144
 // nodes (6 x 10 = 60); AdTile leaves room for a cell of drift on every side,
