@@ -1,6 +1,8 @@
 """What a destroyed simulator held goes back to the device: all but 1 GiB at
 once, and that too after release_memory.  64 MB are left for the pool's own
 granularity and for what other code of the process maps meanwhile."""
+import gc
+
 import pytest
 
 import autoquantizer_b200 as aq
@@ -29,6 +31,7 @@ def test_memory_of_a_destroyed_simulator():
         return s
 
     solver()._drop_sim()  # kernels compiled and loaded
+    gc.collect()  # nothing of earlier tests is freed meanwhile
     torch.cuda.empty_cache()
     aq.release_memory()
     before = free()
@@ -50,6 +53,7 @@ def test_streamed_simulator_holds_two_grids():
     s = MPMSolver(cfg)
     s.set_particles(vals)
     StreamedSolver(s, 1000).close()  # kernels compiled and loaded
+    gc.collect()  # nothing of earlier tests is freed meanwhile
     torch.cuda.empty_cache()
     aq.release_memory()
     before = torch.cuda.mem_get_info()[0]
